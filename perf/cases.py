@@ -206,8 +206,8 @@ def run(state):
     if isinstance(state, _Snapshot):
         s = state
         E.force_snapshot_noalloc(s.spec, s.r.data_ptr(), s.q.data_ptr(), s.L,
-                                 s.wall.data_ptr() if s.wall is not None else 0, s.f.data_ptr(), s.n.data_ptr(), s.out.data_ptr(),
-                                 torch.cuda.current_stream().cuda_stream)
+                                 s.wall.data_ptr() if s.wall is not None else 0, s.f.data_ptr(), s.n.data_ptr(),
+                                 s.out.data_ptr(), torch.cuda.current_stream().cuda_stream)
         return {"force": s.f, "torque": s.n, "sums": s.out.float()}   # FP32 pair sums
     kept = np.float64 if state.precision == "fp64" else np.float32
     if state.kind == "relax":
