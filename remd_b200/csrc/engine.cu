@@ -38,7 +38,7 @@ using namespace remd;
     }                                                                              \
   } while (0)
 
-constexpr int kMaxChains = 4;   // independent chains of the interval graph
+constexpr int kMaxChains = 8;   // independent chains of the interval graph
 
 struct remd_engine_s {
   int device = 0;
@@ -57,8 +57,13 @@ struct remd_engine_s {
   std::vector<int> order2;         // the same per chain: chain k's tiles [chain_tile[k], chain_tile[k+1])
   int nchain = 1;                  // independent chains of the interval graph
   int chain_tile[kMaxChains + 1] = {};
-  int chain_rep[kMaxChains + 1] = {};   // chain k's replicas [chain_rep[k], chain_rep[k+1])
+  std::vector<int> reps2;          // replicas by chain: chain k's are reps2[chain_rep[k] .. chain_rep[k+1])
+  int chain_rep[kMaxChains + 1] = {};
+  int* d_reps2 = nullptr;
   int* d_order2 = nullptr;
+  std::vector<PairBlk> pblk, pblk2;   // FP32 form: list and pair blocks in the order of `order`, `order2`
+  int chain_pblk[kMaxChains + 1] = {};
+  PairBlk* d_pblk2 = nullptr;
   std::vector<double> curT, curP;
   std::vector<double> wall_h;
   DevPtrs d{};
@@ -191,7 +196,7 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
   const int T = h->tile;
   h->tiles.clear();
   long long pack_words = 0, nbr_words = 0;
-  int nwarps = 0;
+  int nwarps = 0, npart2 = 0;
   for (int r = 0; r < h->nrep; r++) {
     RepConst& c = h->rc[r];
     c.tile_off = (int)h->tiles.size();
@@ -199,11 +204,18 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     c.warp_off = nwarps;
     c.nwarp = (c.nmol + 31) / 32;
     nwarps += c.nwarp;
+    c.part2_off = npart2;
+    c.npart2 = (c.nmol + kPart2Mol - 1) / kPart2Mol;
+    npart2 += c.npart2;
     for (int t = 0; t < c.ntile; t++) {
       Tile tt;
       tt.rep = r;
       tt.start = t * T;
       tt.count = std::min(T, c.nmol - t * T);
+      tt.mol_off = c.mol_off;
+      tt.part2_off = c.part2_off;
+      tt.npart2 = c.npart2;
+      tt.tile_off = c.tile_off;
       tt.pad = 0;
       h->tiles.push_back(tt);
     }
@@ -211,7 +223,9 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     c.pack_off = pack_words;
     pack_words += (long long)c.nmol * c.pack_stride;
     c.nbr_off = nbr_words;
-    nbr_words += (long long)c.ntile * c.nbr_cap * T;
+    // FP32 form: one row per molecule; FP64 form: column-major inside a tile
+    c.nbr_stride = (c.nbr_cap + 7) / 8 * 8;
+    nbr_words += (h->prec == kF32) ? (long long)c.nmol * c.nbr_stride : (long long)c.ntile * c.nbr_cap * T;
   }
   // force blocks in decreasing order of estimated pair work (longest first, so
   // the costliest tiles do not form the tail of the launch): molecules x
@@ -227,37 +241,95 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     h->order.resize(h->tiles.size());
     for (size_t t = 0; t < h->order.size(); t++) h->order[t] = (int)t;
     std::stable_sort(h->order.begin(), h->order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-    // groups of whole replicas of about equal cost (boundaries at the replica
-    // boundaries nearest k/K of the total) for the independent chains of the
-    // interval graph
-    const int K = std::min(kMaxChains, h->nrep);
-    std::vector<double> before(h->nrep + 1, 0.0);   // cost of replicas [0, r)
+    // groups of whole replicas for the independent chains of the interval graph:
+    // each of one water model where there are no more models than chains (the
+    // pair kernel compiled for one model needs fewer registers and instructions
+    // than the one for all), of about equal cost within a model
+    // Eight chains while a quarter of the batch is no more than one wave of pair
+    // blocks (about 2400 blocks in all), else four: 8 replicas of 4096 molecules run
+    // 785 us a 10-step interval on four and 730 us on eight; 256 replicas, 111 432
+    // molecules, 3680 us on four and 3718 us on eight (twice the graph's nodes).
+    const int K = std::min(npart2 <= 2400 ? kMaxChains : 4, h->nrep);
+    std::vector<double> rcost(h->nrep, 0.0);
+    std::map<int, double> mcost;   // cost per model
+    const bool by_model = h->prec == kF32;
     for (int r = 0; r < h->nrep; r++) {
-      double w = 0.0;
-      for (int t = h->rc[r].tile_off; t < h->rc[r].tile_off + h->rc[r].ntile; t++) w += cost[t];
-      before[r + 1] = before[r] + w;
+      for (int t = h->rc[r].tile_off; t < h->rc[r].tile_off + h->rc[r].ntile; t++) rcost[r] += cost[t];
+      mcost[by_model ? h->rc[r].nsite : 0] += rcost[r];
     }
-    std::vector<int> cut(1, 0);   // first replica of each chain
-    for (int k = 1; k < K; k++) {
-      const double goal = before[h->nrep] * k / K;
-      int best = cut.back() + 1;
-      for (int r = cut.back() + 1; r <= h->nrep - (K - k); r++)
-        if (std::fabs(before[r] - goal) < std::fabs(before[best] - goal)) best = r;
-      cut.push_back(best);
+    std::map<int, int> mchains, mreps;   // chains and replicas per model
+    for (int r = 0; r < h->nrep; r++) mreps[by_model ? h->rc[r].nsite : 0]++;
+    if ((int)mcost.size() > K) {
+      double all = 0.0;
+      for (auto& m : mcost) all += m.second;
+      mcost = {{-1, all}};
+      mreps = {{-1, h->nrep}};
     }
-    h->nchain = K;
-    for (int k = 0; k < K; k++) {
-      h->chain_tile[k] = h->rc[cut[k]].tile_off;
-      h->chain_rep[k] = cut[k];
+    for (auto& m : mcost) mchains[m.first] = 1;
+    for (int left = K - (int)mcost.size(); left > 0; left--) {   // to the model whose chains are costliest
+      int best = -2;
+      for (auto& m : mcost)
+        if (mchains[m.first] < mreps[m.first] &&
+            (best == -2 || m.second / mchains[m.first] > mcost[best] / mchains[best]))
+          best = m.first;
+      if (best == -2) break;
+      mchains[best]++;
     }
-    h->chain_tile[K] = (int)h->tiles.size();
-    h->chain_rep[K] = h->nrep;
+    h->reps2.clear();
     h->order2.clear();
-    for (int k = 0; k < K; k++)
+    h->nchain = 0;
+    h->chain_tile[0] = h->chain_rep[0] = 0;
+    std::vector<int> chain_of(h->nrep, 0);
+    for (auto& m : mcost) {
+      // the model's replicas in order, cut where the cost passes k / chains of its total
+      double run = 0.0;
+      int k = 0, used = 0, in_chain = 0, seen = 0;
+      for (int r = 0; r < h->nrep; r++) {
+        if (m.first != -1 && m.first != 0 && h->rc[r].nsite != m.first) continue;
+        const int left_reps = mreps[m.first] - seen, left_chains = mchains[m.first] - k;
+        if (in_chain > 0 && k + 1 < mchains[m.first] &&
+            (run + 0.5 * rcost[r] > m.second * (k + 1) / mchains[m.first] || left_reps < left_chains)) {
+          k++;
+          in_chain = 0;
+        }
+        chain_of[r] = h->nchain + k;
+        run += rcost[r];
+        in_chain++;
+        seen++;
+        used = k + 1;
+      }
+      h->nchain += used;
+    }
+    for (int k = 0; k < h->nchain; k++) {
+      for (int r = 0; r < h->nrep; r++)
+        if (chain_of[r] == k) h->reps2.push_back(r);
       for (int t : h->order)
-        if (t >= h->chain_tile[k] && t < h->chain_tile[k + 1]) h->order2.push_back(t);
+        if (chain_of[h->tiles[t].rep] == k) h->order2.push_back(t);
+      h->chain_rep[k + 1] = (int)h->reps2.size();
+      h->chain_tile[k + 1] = (int)h->order2.size();
+    }
+    auto blocks = [&](const std::vector<int>& order, std::vector<PairBlk>& out) {
+      out.clear();
+      for (int t : order)
+        for (int k = 0; k < h->tiles[t].count; k += kPart2Mol)
+          out.push_back(pair_blk(h->rc[h->tiles[t].rep], h->tiles[t].rep, h->tiles[t].start + k, T));
+    };
+    blocks(h->order, h->pblk);
+    blocks(h->order2, h->pblk2);
+    h->chain_pblk[0] = 0;
+    for (int k = 0; k < h->nchain; k++) {
+      int n = 0;
+      for (int r = h->chain_rep[k]; r < h->chain_rep[k + 1]; r++) n += h->rc[h->reps2[r]].npart2;
+      h->chain_pblk[k + 1] = h->chain_pblk[k] + n;
+    }
   }
   const size_t N = h->N, nt = h->tiles.size(), nr = h->nrep;
+  const size_t nf = (h->prec == kF32) ? 1 : 0;
+  if (nf) {   // 16-byte pieces of every molecule, as many as the largest record has
+    int stride = 0;
+    for (const RepConst& c : h->rc) stride = std::max(stride, c.pack_stride);
+    pack_words = (long long)N * stride;
+  }
   const size_t elem = (h->prec == kF32) ? 4 : 8;
   const size_t sizes[] = {
       nr * sizeof(RepConst),           // 0 rc
@@ -266,10 +338,10 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
       (size_t)pack_words * elem,       // 8 pack
       N * sizeof(int4),                // 9 ref_com
       nt * 3 * 8,                      // 10 Lbuild
-      (size_t)nbr_words * 2,           // 11 nbr
+      (size_t)(nbr_words + kListPad) * 2,   // 11 nbr
       N * 4,                           // 12 nbr_cnt
       std::max<size_t>(h->wall_h.size(), 2) * 8,   // 13 wall
-      (size_t)nwarps * sizeof(Part1), (size_t)nwarps * sizeof(Part2),   // 14, 15 (per 32 molecules)
+      (size_t)nwarps * sizeof(Part1), (size_t)npart2 * sizeof(Part2),   // 14, 15
       nr * kNumAvg * 8,                // 16 avg
       nr * 4, 64,                      // 17 status, 18 err
       nr * 8, nr * 8,                  // 19 T, 20 P
@@ -279,16 +351,17 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
       (size_t)std::max(nr / 2, (size_t)1) * 8,   // 27 u
       (size_t)h->nens * 8,             // 28 per-ensemble exchange step counter
       (size_t)h->nens * 8,             // 29 per-ensemble exchange seed
-      (h->prec == kF32) ? (size_t)nbr_words * 2 : 0,   // 30 nbt (FP32 per-step lists)
-      nt * 4,                          // 31 order
-      (h->prec == kF32) ? N * 4 : 0,   // 32 nt_cnt (FP32 per-step list counts)
-      N * sizeof(int4),                // 33 com (FP32 current fixed-point centres)
-      nt * 4,                          // 34 order per chain (multi-chain interval graph)
-      nr * sizeof(CellGrid),           // 35 cell grid + rebuild decision per replica
-      nr * (size_t)(kMaxCells + 1) * 4,   // 36 cell offsets per replica
-      N * sizeof(int4),                // 37 centres sorted by cell
-      nr * sizeof(int2),               // 38 carried replicas' sources (serving batch changes)
-      (size_t)h->nens * 4, (size_t)h->nens * 4,   // 39 carried ensembles' sources, 40 replicas per ensemble
+      nt * 4,                          // 30 order
+      nf ? 0 : N * sizeof(int4),       // 31 com (FP64 form; FP32: the records' first pieces)
+      nt * 4,                          // 32 order per chain (multi-chain interval graph)
+      nr * sizeof(CellGrid),           // 33 cell grid + rebuild decision per replica
+      nr * (size_t)(kMaxCells + 1) * 4,   // 34 cell offsets per replica
+      N * sizeof(int4),                // 35 centres sorted by cell
+      nr * sizeof(int2),               // 36 carried replicas' sources (serving batch changes)
+      (size_t)h->nens * 4, (size_t)h->nens * 4,   // 37 carried ensembles' sources, 38 replicas per ensemble
+      nf * nr * sizeof(PairConst), nf * npart2 * sizeof(PairBlk), nf * npart2 * sizeof(PairBlk),   // 39 pair constants, 40 pair blocks, 41 per chain
+      nf * nbr_words * 2, nf * N * 4, nf * N * 32,   // 42 nbt (per-step lists), 43 their counts, 44 wall terms
+      nr * 4,                          // 45 replicas per chain
   };
   offs.clear();
   total = 0;
@@ -302,6 +375,17 @@ static void free_pool(remd_engine_s* h) {
   if (h->mempool) cudaFreeAsync(h->pool, h->stream);
   else cudaFree(h->pool);
   h->pool = nullptr;
+}
+
+// DevPtrs::model_l of a launch over n replicas (reps == NULL: the first n).
+static int common_model(const remd_engine_s* h, const int* reps, int n) {
+  int m = pair_model(h->rc[reps ? reps[0] : 0]);
+  for (int k = 1; k < n; k++) {
+    const int x = pair_model(h->rc[reps ? reps[k] : k]);
+    if (x % kStdCharges != m % kStdCharges) m = m / kStdCharges * kStdCharges;   // sites differ
+    if (x < kStdCharges) m %= kStdCharges;
+  }
+  return m;
 }
 
 static remd_status allocate(remd_engine_s* h) {
@@ -355,20 +439,26 @@ static remd_status allocate(remd_engine_s* h) {
   h->d_u = reinterpret_cast<double*>(b + offs[27]);
   h->d_step = reinterpret_cast<long long*>(b + offs[28]);
   h->d_seed = reinterpret_cast<unsigned long long*>(b + offs[29]);
-  d.nbt = reinterpret_cast<uint16_t*>(b + offs[30]);
-  d.order = reinterpret_cast<int*>(b + offs[31]);
-  d.nt_cnt = reinterpret_cast<int*>(b + offs[32]);
-  d.com = reinterpret_cast<int4*>(b + offs[33]);
-  d.tile0 = 0;
-  h->d_order2 = reinterpret_cast<int*>(b + offs[34]);
-  d.cgrid = reinterpret_cast<CellGrid*>(b + offs[35]);
-  d.cell_start = reinterpret_cast<int*>(b + offs[36]);
-  d.cell_com = reinterpret_cast<int4*>(b + offs[37]);
-  h->d_carry_src = reinterpret_cast<int2*>(b + offs[38]);
-  h->d_carry_ens = reinterpret_cast<int*>(b + offs[39]);
-  h->d_ens_nrep = reinterpret_cast<int*>(b + offs[40]);
-  d.rep0 = 0;
+  d.order = reinterpret_cast<int*>(b + offs[30]);
+  d.com = reinterpret_cast<int4*>(h->prec == kF32 ? d.pack : b + offs[31]);
+  h->d_order2 = reinterpret_cast<int*>(b + offs[32]);
+  d.cgrid = reinterpret_cast<CellGrid*>(b + offs[33]);
+  d.cell_start = reinterpret_cast<int*>(b + offs[34]);
+  d.cell_com = reinterpret_cast<int4*>(b + offs[35]);
+  h->d_carry_src = reinterpret_cast<int2*>(b + offs[36]);
+  h->d_carry_ens = reinterpret_cast<int*>(b + offs[37]);
+  h->d_ens_nrep = reinterpret_cast<int*>(b + offs[38]);
+  d.pc = reinterpret_cast<PairConst*>(b + offs[39]);
+  d.pblk = reinterpret_cast<PairBlk*>(b + offs[40]);
+  d.npblk = (int)h->pblk.size();
+  h->d_pblk2 = reinterpret_cast<PairBlk*>(b + offs[41]);
+  d.nbt = reinterpret_cast<uint16_t*>(b + offs[42]);
+  d.nt_cnt = reinterpret_cast<int*>(b + offs[43]);
+  d.wallf = reinterpret_cast<double*>(b + offs[44]);
+  h->d_reps2 = reinterpret_cast<int*>(b + offs[45]);
+  d.reps = nullptr;
   d.nrep_l = h->nrep;
+  d.model_l = common_model(h, nullptr, h->nrep);
   {
     int nmax = 1;
     for (const RepConst& c : h->rc) nmax = std::max(nmax, c.nmol);
@@ -380,6 +470,14 @@ static remd_status allocate(remd_engine_s* h) {
   CK(cudaMemcpyAsync((void*)d.tiles, h->tiles.data(), h->tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync((void*)d.order, h->order.data(), h->order.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->d_order2, h->order2.data(), h->order2.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->d_reps2, h->reps2.data(), h->reps2.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  std::vector<PairConst> pc;
+  if (h->prec == kF32) {
+    for (const RepConst& c : h->rc) pc.push_back(pair_const(c));
+    CK(cudaMemcpyAsync((void*)d.pc, pc.data(), pc.size() * sizeof(PairConst), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync((void*)d.pblk, h->pblk.data(), h->pblk.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->d_pblk2, h->pblk2.data(), h->pblk2.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
+  }
   if (!h->wall_h.empty())
     CK(cudaMemcpyAsync((void*)d.wall, h->wall_h.data(), h->wall_h.size() * 8, cudaMemcpyHostToDevice, h->stream));
   // later set-up copies use the default stream, which does not order with this
@@ -451,6 +549,11 @@ static void launch_step_integrate(remd_engine_s* h, int s) {
 
 static remd_status build_graph(remd_engine_s* h) {
   cudaGraph_t g;
+  if (!h->vscale)   // the chains' streams, when first needed
+    for (int k = 0; k < h->nchain - 1; k++) {
+      if (!h->stream2[k]) CK(cudaStreamCreateWithFlags(&h->stream2[k], cudaStreamNonBlocking));
+      if (!h->ev_join[k]) CK(cudaEventCreateWithFlags(&h->ev_join[k], cudaEventDisableTiming));
+    }
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   launch_replica_start(h->d, h->X, h->stream);
   if (h->nchain > 1 && !h->vscale) {
@@ -463,9 +566,11 @@ static remd_status build_graph(remd_engine_s* h) {
       dg[k] = h->d;
       dg[k].ntiles = h->chain_tile[k + 1] - h->chain_tile[k];
       dg[k].order = h->d_order2 + h->chain_tile[k];
-      dg[k].tile0 = h->chain_tile[k];
-      dg[k].rep0 = h->chain_rep[k];
+      dg[k].reps = h->d_reps2 + h->chain_rep[k];
       dg[k].nrep_l = h->chain_rep[k + 1] - h->chain_rep[k];
+      dg[k].model_l = common_model(h, &h->reps2[h->chain_rep[k]], dg[k].nrep_l);
+      dg[k].pblk = h->d_pblk2 + h->chain_pblk[k];
+      dg[k].npblk = h->chain_pblk[k + 1] - h->chain_pblk[k];
     }
     cudaEventRecord(h->ev_fork, h->stream);
     for (int k = 1; k < h->nchain; k++) cudaStreamWaitEvent(h->stream2[k - 1], h->ev_fork, 0);
@@ -529,7 +634,7 @@ static remd_status build_graph(remd_engine_s* h) {
 
 static long long host_pairs(remd_engine_s* h) {
   const RepConst& last = h->rc.back();
-  std::vector<Part2> p2((size_t)last.warp_off + last.nwarp);
+  std::vector<Part2> p2((size_t)last.part2_off + last.npart2);
   if (cudaMemcpy(p2.data(), h->d.part2, p2.size() * sizeof(Part2), cudaMemcpyDeviceToHost) != cudaSuccess)
     return -1;
   long long s = 0;
@@ -780,6 +885,10 @@ static remd_status create_impl(const remd_system_desc* systems, int nens, const 
       c.W = ri.W > 0.0 ? ri.W : 1.0;
       c.mass = ri.mass[0];
       for (int x = 0; x < 3; x++) c.I[x] = ri.inertia[x];
+      c.hQ = c.dthalf / (2.0 * c.Q);
+      c.iW = 1.0 / c.W;
+      c.im = 1.0 / c.mass;
+      for (int x = 0; x < 3; x++) c.iI[x] = 1.0 / c.I[x];
       const double wl = s.wall_length * 1e-10 / unit_length();
       c.wall_dr = (s.confined == 2) ? 0.5 * (wl / (double)s.nfwall) : wl / (double)std::max(s.nfwall, 1);
       c.wall_length_param = s.wall_length;
@@ -794,6 +903,7 @@ static remd_status create_impl(const remd_system_desc* systems, int nens, const 
       }
       for (int k = 0; k < s.nsite; k++)
         for (int l = 0; l < s.nsite; l++) c.qq[k][l] = qr[k] * qr[l];
+      for (int k = 0; k < s.nsite; k++) c.qr[k] = qr[k];
       c.site_reach = 0.0;
       for (int k = 0; k < s.nsite; k++)
         c.site_reach = std::max(c.site_reach, std::sqrt(c.body[k][0] * c.body[k][0] + c.body[k][1] * c.body[k][1] +
@@ -859,13 +969,6 @@ static remd_status create_impl(const remd_system_desc* systems, int nens, const 
       delete h;
       return REMD_ERR_CUDA;
     }
-    for (int k = 0; k < kMaxChains - 1; k++)
-      if (cudaStreamCreateWithFlags(&h->stream2[k], cudaStreamNonBlocking) != cudaSuccess ||
-          cudaEventCreateWithFlags(&h->ev_join[k], cudaEventDisableTiming) != cudaSuccess) {
-        set_error("cannot create the interval graph's streams");
-        undo_carry(h, cy);
-        return REMD_ERR_CUDA;
-      }
   }
   remd_status st = allocate(h);
   if (st != REMD_OK) { undo_carry(h, cy); return st; }
@@ -1160,8 +1263,8 @@ remd_status remd_get_state(remd_handle h, int rep, remd_state_view* o) {
   o->s = st.s; o->Ps = st.Ps; o->Q = c.Q; o->W = c.W;
   for (int x = 0; x < 3; x++) { o->Pv[x] = st.Pv[x]; o->L[x] = st.L[x]; }
   o->T = st.T; o->P = st.P; o->H0 = st.H0;
-  std::vector<Part2> p2(c.nwarp);
-  CK(cudaMemcpy(p2.data(), h->d.part2 + c.warp_off, c.nwarp * sizeof(Part2), cudaMemcpyDeviceToHost));
+  std::vector<Part2> p2(c.npart2);
+  CK(cudaMemcpy(p2.data(), h->d.part2 + c.part2_off, c.npart2 * sizeof(Part2), cudaMemcpyDeviceToHost));
   double lj = 0, cl = 0, w = 0, v[3] = {0, 0, 0};
   for (auto& p : p2) { lj += p.lj; cl += p.clmb; w += p.wall; for (int x = 0; x < 3; x++) v[x] += p.vir[x]; }
   o->lj = lj * 0.5; o->clmb = cl * 0.5; o->wall = w;
@@ -1204,8 +1307,8 @@ long long remd_replica_pair_count(remd_handle h, int rep) {
   if (!h || rep < 0 || rep >= h->nrep) return -1;
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return -1;
   const RepConst& c = h->rc[rep];
-  std::vector<Part2> p2(c.nwarp);
-  if (cudaMemcpy(p2.data(), h->d.part2 + c.warp_off, c.nwarp * sizeof(Part2), cudaMemcpyDeviceToHost) != cudaSuccess)
+  std::vector<Part2> p2(c.npart2);
+  if (cudaMemcpy(p2.data(), h->d.part2 + c.part2_off, c.npart2 * sizeof(Part2), cudaMemcpyDeviceToHost) != cudaSuccess)
     return -1;
   long long s = 0;
   for (auto& p : p2) s += p.npairs;

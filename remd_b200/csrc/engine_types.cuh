@@ -23,6 +23,7 @@ namespace remd {
 
 constexpr int kMaxSites = 5;
 constexpr int kNumAvg = 19;
+constexpr int kPart2Mol = 16;                   // molecules of a force partial sum (Part2)
 constexpr double kFix = 4294967296.0;          // 2^32: fixed-point box fraction
 constexpr double kFixInv = 1.0 / 4294967296.0;
 
@@ -30,30 +31,65 @@ constexpr double kFixInv = 1.0 / 4294967296.0;
 struct RepConst {
   int nmol, mol_off;       // molecules; first global index
   int tile_off, ntile;     // force/integrate tiles [tile_off, tile_off+ntile)
-  int warp_off, nwarp;     // 32-molecule partial-sum units [warp_off, warp_off+nwarp)
+  int warp_off, nwarp;     // 32-molecule partial-sum units [warp_off, warp_off+nwarp) of Part1
+  int part2_off, npart2;   // kPart2Mol-molecule units [part2_off, part2_off+npart2) of Part2
   int nsite, c0;           // sites; first charged site (charged sites are [c0, nsite))
   int confined, tconstant, pconstant;
   int nfwall, wall_off;    // wall table entries and offset into the table array
   int nbr_cap;             // neighbour list capacity per molecule
+  int nbr_stride;          // FP32 form: words of a molecule's list (nbr_cap rounded up to 8)
   int ens;                 // ensemble index
   int pack_stride;         // words (FP32) or doubles (FP64) per pack record
-  long long pack_off;      // first record word/double of this replica
-  long long nbr_off;       // first neighbour word of tile_off
+  long long pack_off;      // FP64 form: first record double of this replica
+  long long nbr_off;       // first neighbour word of the replica
   double dt, dthalf;
   double rc, rs, coef_sw;  // switching: coef_sw = 1/(rs-rc)^5
   double skin;
   double Q, W;
   double mass, I[3];
+  double hQ, iW, im, iI[3];   // (dt/2) / (2 Q), 1/W, 1/mass, 1/I
   double wall_dr;          // table spacing: wall_length/nfwall (tube) or half of it (slit)
   double wall_length_param;   // A, as read from .inp
   double bottom_area;      // GetBottomArea (tube)
   double slit_width;       // wall length in reduced units (slit volume)
   double body[kMaxSites][3];
-  double qq[kMaxSites][kMaxSites];
+  double qr[kMaxSites], qq[kMaxSites][kMaxSites];   // site charges and their products
   double sgm2, eps;        // O-O Lennard-Jones: ((s+s)/2)^2 and sqrt(e e)
   double site_reach;       // max |site - centre of mass| (A): per-site images matter
                            // once L_d < 2 (rc + 2 site_reach)
 };
+
+// The constants of the FP32 pair step, loaded whole into shared memory by each block.
+struct PairConst {
+  int nmol, mol_off, nsite, part2_off;
+  int nbr_stride, nbr_cap, confined, pad0;
+  long long nbr_off;
+  float rc, rs, rc2, coef;     // switching: coef = 1/(rs-rc)^5
+  float sgm2q, eps4, reach;    // sigma^2 / 4, 4 epsilon, site_reach
+  float uu;                    // square of the unit charge (that of the second charged site)
+  float q[kMaxSites];          // site charges in units of it
+  float pad1;
+  double body[kMaxSites][3];
+};
+// A list or pair block of the FP32 form: kPart2Mol molecules of a replica, with
+// what their first loads need.
+struct alignas(16) PairBlk {
+  int rep, li0;                // replica, first local molecule
+  int nmol, mol_off;
+  long long nbr_off;
+  int nbr_stride;
+  int16_t confined, tile;      // tile: molecules of a tile
+};
+__host__ __device__ inline PairBlk pair_blk(const RepConst& c, int rep, int li0, int tile) {
+  PairBlk b;
+  b.rep = rep; b.li0 = li0; b.nmol = c.nmol; b.mol_off = c.mol_off;
+  b.nbr_off = c.nbr_off; b.nbr_stride = c.nbr_stride; b.confined = (int16_t)c.confined; b.tile = (int16_t)tile;
+  return b;
+}
+constexpr int kListPad = 128;  // FP32 form: list entries read past a list's end (masked), the array's padding
+
+// Added to DevPtrs::model_l: the charge ratios are those of charge_ratio (kernels.cu).
+constexpr int kStdCharges = 8;
 
 // Per-replica scalars (two copies, ping-pong).
 struct RepState {
@@ -69,15 +105,16 @@ struct Part1 {
   double pad[3];
 };
 
-// Force-kernel partials of 32 molecules (raw ordered-pair sums; consumers halve lj/clmb/vir).
+// Force-kernel partials of kPart2Mol molecules (raw ordered-pair sums; consumers halve lj/clmb/vir).
 struct Part2 {
   double lj, clmb, wall, vir[3];
   long long npairs;        // ordered pairs within rc
   double pad;
 };
 
-struct Tile {
-  int rep, start, count, pad;   // replica, first local molecule, molecules in tile
+struct alignas(16) Tile {
+  int rep, start, count, mol_off;   // replica, first local molecule, molecules in tile; as RepConst:
+  int part2_off, npart2, tile_off, pad;
 };
 
 // Cell lists of a replica (rebuilt with its neighbour lists): the periodic box
@@ -96,15 +133,16 @@ struct DevPtrs {
   int ntiles, nrep;
   const RepConst* rc;
   const Tile* tiles;
-  const int* order;              // force-launch block -> tile, costliest first (NULL: identity)
+  const int* order;              // block -> tile of a launch, costliest first (NULL: identity)
   double *r, *v, *q, *p, *f, *n; // SoA, component-major, stride N
-  void* pack;                    // FP32 words or FP64 doubles
+  void* pack;                    // FP32: 16-byte pieces, piece m of molecule g at m N + g; FP64: doubles, by molecule
   int4* ref_com;                 // fixed-point com at the last list build
-  int4* com;                     // FP32 form: current fixed-point com (written with the pack)
+  int4* com;                     // current fixed-point com (FP32 form: the records' first 16 bytes)
   double* Lbuild;                // per tile, 3 doubles (NaN = list invalid)
   uint16_t* nbr;                 // neighbour lists (rcut + skin)
   uint16_t* nbt;                 // FP32 form: per-step lists of the pairs within rcut (same layout)
   int* nt_cnt;                   // FP32 form: per molecule, nfar | nnear << 16 in nbt
+  double* wallf;                 // FP32 form: per molecule, wall force and energy (confined replicas)
   int* nbr_cnt;                  // per molecule
   const double* wall;            // {f, U} pairs
   Part1* part1;
@@ -118,8 +156,12 @@ struct DevPtrs {
   const double* newT;            // conditions for the next interval (per replica)
   const double* newP;
   const int* changed;            // 1 = apply the exchange tail at the interval start
-  int tile0;                     // first tile of a launch over a tile range (order == NULL)
-  int rep0, nrep_l;              // replicas [rep0, rep0 + nrep_l) of a launch (per-replica kernels)
+  const PairConst* pc;           // FP32 form, per replica
+  const PairBlk* pblk;           // FP32 form: list and pair blocks, costliest first
+  int npblk;                     // pair blocks of a launch
+  int model_l;                   // sites of every replica of a launch (0 when they differ) + kStdCharges
+  const int* reps;               // replicas of a launch of the replica head (NULL: all)
+  int nrep_l;                    // their number
   int bm_win;                    // words per row of the list-rebuild bitmap (kernels.cu)
 };
 

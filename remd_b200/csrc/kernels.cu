@@ -18,11 +18,38 @@ namespace remd {
 constexpr int kRepThreads = 256;   // threads of the per-replica kernels
 constexpr int kBitmapMaxWords = 64; // list-rebuild bitmap window: 2048 molecules per pass
 constexpr int kCellMinPrune = 4;    // cut a replica into cells when they prune at least 4x
-constexpr int kListLanes = 4;       // lanes per molecule in the FP32 list kernel (adjacent in a warp)
+constexpr int kGroup = 8;           // FP32 form: lanes per molecule in the list and pair kernels
+constexpr int kWarpMol = 32 / kGroup;   // molecules of a warp there
+constexpr int kPairWarps = kPart2Mol / kWarpMol;   // warps of a list or pair block (kPart2Mol molecules)
+constexpr int kSegPairs = 32 * kGroup;  // pairs of a molecule per FP32 partial sum (32 per lane)
 
 int pack_stride(int nsite, int prec) {
   if (prec == kF32) return ((3 + 3 * nsite) + 3) / 4 * 4;   // words, 16-B multiple
   return ((3 + 3 * nsite) + 1) / 2 * 2;                      // doubles, 16-B multiple
+}
+
+PairConst pair_const(const RepConst& c) {
+  PairConst p{};
+  p.nmol = c.nmol; p.mol_off = c.mol_off; p.nsite = c.nsite; p.part2_off = c.part2_off;
+  p.nbr_stride = c.nbr_stride; p.nbr_cap = c.nbr_cap; p.confined = c.confined;
+  p.nbr_off = c.nbr_off;
+  p.rc = (float)c.rc; p.rs = (float)c.rs; p.rc2 = (float)(c.rc * c.rc); p.coef = (float)c.coef_sw;
+  p.sgm2q = (float)(0.25 * c.sgm2); p.eps4 = (float)(4.0 * c.eps); p.reach = (float)c.site_reach;
+  const double unit = c.qr[c.c0 + 1];
+  p.uu = (float)(unit * unit);
+  for (int k = c.c0; k < c.nsite; k++) p.q[k] = (float)(c.qr[k] / unit);
+  for (int k = 0; k < kMaxSites; k++)
+    for (int x = 0; x < 3; x++) p.body[k][x] = c.body[k][x];
+  return p;
+}
+
+int pair_model(const RepConst& c) {
+  const PairConst p = pair_const(c);
+  const float* q = p.q;
+  const bool std_q = c.nsite == 3   ? (q[0] == -2.f && q[1] == 1.f && q[2] == 1.f)
+                     : c.nsite == 4 ? (q[1] == 1.f && q[2] == 1.f && q[3] == -2.f)
+                                    : (q[1] == 1.f && q[2] == 1.f && q[3] == -1.f && q[4] == -1.f);
+  return c.nsite + (std_q ? kStdCharges : 0);
 }
 
 // ------------------------------------------------------------------ reductions
@@ -81,9 +108,9 @@ __device__ inline double warp_max(double v) {
 struct P2Sum {
   double lj, clmb, wall, vir[3];
 };
-__device__ inline P2Sum reduce_part2(const DevPtrs& d, const RepConst& c) {
+__device__ inline P2Sum reduce_part2(const DevPtrs& d, int part2_off, int npart2) {
   double v[6] = {0, 0, 0, 0, 0, 0};
-  for (int t = c.warp_off + (threadIdx.x & 31); t < c.warp_off + c.nwarp; t += 32) {
+  for (int t = part2_off + (threadIdx.x & 31); t < part2_off + npart2; t += 32) {
     const Part2 p = d.part2[t];
     v[0] += p.lj; v[1] += p.clmb; v[2] += p.wall;
     v[3] += p.vir[0]; v[4] += p.vir[1]; v[5] += p.vir[2];
@@ -120,35 +147,55 @@ __device__ inline int fix_coord(double r) {
   return (int)(unsigned int)(long long)llrint((r - 0.5) * kFix);
 }
 
-__device__ inline void write_pack(const DevPtrs& d, const RepConst& c, int prec, int li,
-                                  const double* r, const double* q) {
-  const int ns = c.nsite;
+// Rotation matrix (body to space) of a quaternion, the map of body_to_space.
+struct Rot {
+  double m[3][3];
+  __device__ __forceinline__ explicit Rot(const double* a) {
+    const double a0 = a[0] * a[0], a1 = a[1] * a[1], a2 = a[2] * a[2], a3 = a[3] * a[3];
+    const double a01 = a[0] * a[1], a02 = a[0] * a[2], a03 = a[0] * a[3];
+    const double a12 = a[1] * a[2], a13 = a[1] * a[3], a23 = a[2] * a[3];
+    m[0][0] = a0 + a1 - a2 - a3; m[0][1] = 2. * (a12 - a03); m[0][2] = 2. * (a13 + a02);
+    m[1][0] = 2. * (a12 + a03); m[1][1] = a0 - a1 + a2 - a3; m[1][2] = 2. * (a23 - a01);
+    m[2][0] = 2. * (a13 - a02); m[2][1] = 2. * (a23 + a01); m[2][2] = a0 - a1 - a2 + a3;
+  }
+  __device__ __forceinline__ double at(int x, const double* b) const {
+    return m[x][0] * b[0] + m[x][1] * b[1] + m[x][2] * b[2];
+  }
+};
+
+template <int S>
+__device__ __forceinline__ void write_pack_f32(const DevPtrs& d, const RepConst& c, int g, const int* fx,
+                                               const double* q) {
+  constexpr int NV = ((3 + 3 * S) + 3) / 4;
+  uint32_t buf[4 * NV];
+  for (int k = 3 + 3 * S; k < 4 * NV; k++) buf[k] = 0u;
+  for (int x = 0; x < 3; x++) buf[x] = (uint32_t)fx[x];
+  const Rot R(q);
+#pragma unroll
+  for (int k = 0; k < S; k++)
+    for (int x = 0; x < 3; x++) buf[3 + 3 * k + x] = __float_as_uint((float)R.at(x, c.body[k]));
+  uint4* w4 = reinterpret_cast<uint4*>(d.pack) + g;
+#pragma unroll
+  for (int k = 0; k < NV; k++)
+    w4[(long long)k * d.N] = make_uint4(buf[4 * k], buf[4 * k + 1], buf[4 * k + 2], buf[4 * k + 3]);
+}
+
+// The force record of molecule li at (r, q); fx: its fixed-point centre.
+__device__ inline void write_pack(const DevPtrs& d, const RepConst& c, int prec, int li, const double* r,
+                                  const double* q, const int* fx) {
+  const int ns = c.nsite, g = c.mol_off + li;
   if (prec == kF32) {
-    uint32_t* w = reinterpret_cast<uint32_t*>(d.pack) + c.pack_off + (long long)li * c.pack_stride;
-    uint32_t buf[20];
-    for (int k = 0; k < 20; k++) buf[k] = 0u;
-    buf[0] = (uint32_t)fix_coord(r[0]);
-    buf[1] = (uint32_t)fix_coord(r[1]);
-    buf[2] = (uint32_t)fix_coord(r[2]);
-    for (int k = 0; k < ns; k++) {
-      double o[3];
-      body_to_space(q, c.body[k], o);
-      for (int x = 0; x < 3; x++) buf[3 + 3 * k + x] = __float_as_uint((float)o[x]);
-    }
-    uint4* w4 = reinterpret_cast<uint4*>(w);
-    for (int k = 0; k < c.pack_stride / 4; k++)
-      w4[k] = make_uint4(buf[4 * k], buf[4 * k + 1], buf[4 * k + 2], buf[4 * k + 3]);
-    d.com[c.mol_off + li] = make_int4((int)buf[0], (int)buf[1], (int)buf[2], 0);
+    if (ns == 3) write_pack_f32<3>(d, c, g, fx, q);
+    else if (ns == 4) write_pack_f32<4>(d, c, g, fx, q);
+    else write_pack_f32<5>(d, c, g, fx, q);
   } else {
     double* w = reinterpret_cast<double*>(d.pack) + c.pack_off + (long long)li * c.pack_stride;
     w[0] = r[0]; w[1] = r[1]; w[2] = r[2];
-    for (int k = 0; k < ns; k++) {
-      double o[3];
-      body_to_space(q, c.body[k], o);
-      for (int x = 0; x < 3; x++) w[3 + 3 * k + x] = o[x];
-    }
+    const Rot R(q);
+    for (int k = 0; k < ns; k++)
+      for (int x = 0; x < 3; x++) w[3 + 3 * k + x] = R.at(x, c.body[k]);
     // fixed-point centre: the cell of the molecule at the next list build
-    d.com[c.mol_off + li] = make_int4(fix_coord(r[0]), fix_coord(r[1]), fix_coord(r[2]), 0);
+    d.com[g] = make_int4(fx[0], fx[1], fx[2], 0);
   }
 }
 
@@ -162,7 +209,8 @@ __global__ void k_pack(DevPtrs d, int prec) {
     double r[3], q[4];
     for (int x = 0; x < 3; x++) r[x] = d.r[x * d.N + g];
     for (int x = 0; x < 4; x++) q[x] = d.q[x * d.N + g];
-    write_pack(d, c, prec, li, r, q);
+    const int fx[3] = {fix_coord(r[0]), fix_coord(r[1]), fix_coord(r[2])};
+    write_pack(d, c, prec, li, r, q, fx);
   }
   if (i == 0) {
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
@@ -174,89 +222,114 @@ __global__ void k_pack(DevPtrs d, int prec) {
 struct StepCoef {
   double coef_v_a[3], coef_p_a;   // end-of-previous-step kick
   double coef_v_c[3], coef_p_c;   // this step's kick
-  double coef_xi, cxi1, coef_r[3];
+  double coef_xi, coef_r[3];
   double Lb[3];
 };
 
-template <bool MID>
-__global__ void __launch_bounds__(128, 7) k_integrate(DevPtrs d, const RepState* __restrict__ X,
-                                                   RepState* __restrict__ Y, int prec) {
+// One MD step's integration.  It is bound by latency, not by throughput (a block's
+// FP64 scalar chain, then each molecule's): what a block needs -- the replica's
+// constants and scalars, the force partials -- is requested at once from the tile's
+// descriptor.  CHAIN: one more warp runs the scalar chain while the molecules' warps
+// load their state, into registers; for grids that leave room for the extra warp
+// (launch_integrate_prec).
+template <bool MID, bool CHAIN>
+__global__ void __launch_bounds__(CHAIN ? 160 : 128, CHAIN ? 3 : 7)
+    k_integrate(DevPtrs d, const RepState* __restrict__ X, RepState* __restrict__ Y, int prec) {
   step_kernel_entry();
   __shared__ StepCoef sc;
-  const int tix = d.tile0 + blockIdx.x;   // this launch's tile range
+  __shared__ std::conditional_t<CHAIN, RepConst, int> own;   // the constants, in shared memory
+  const int tix = d.order ? d.order[blockIdx.x] : (int)blockIdx.x;
   const Tile t = d.tiles[tix];
-  const RepConst& c = d.rc[t.rep];
+  const int B = blockDim.x, N = d.N;
+  const int lead = CHAIN ? B - 32 : 0;                 // first thread of the chain's warp
+  const int i = threadIdx.x;
+  const bool active = i < t.count;
+  const bool chain = i >= lead && i < lead + 32;
+  const int g = t.mol_off + t.start + min(i, t.count - 1);
+  if constexpr (CHAIN) {
+    const uint32_t* cs = reinterpret_cast<const uint32_t*>(d.rc + t.rep);
+    for (int k = i; k < (int)(sizeof(RepConst) / 4); k += B) reinterpret_cast<uint32_t*>(&own)[k] = cs[k];
+  }
+  const RepConst& c = *(CHAIN ? reinterpret_cast<const RepConst*>(&own) : d.rc + t.rep);
+  RepState st;
+  if (i == lead) {
+    st = X[t.rep];
+    for (int x = 0; x < 3; x++) sc.Lb[x] = d.Lbuild[3 * tix + x];
+  }
+  double r[3], v[3], q[4], p[4], f[3], n[4];
+  int4 ref;
+  auto load_state = [&]() {
+    for (int x = 0; x < 3; x++) { r[x] = d.r[x * N + g]; v[x] = d.v[x * N + g]; f[x] = d.f[x * N + g]; }
+    for (int x = 0; x < 4; x++) { q[x] = d.q[x * N + g]; p[x] = d.p[x * N + g]; n[x] = d.n[x * N + g]; }
+    ref = d.ref_com[g];
+  };
   P2Sum e;
-  if (threadIdx.x < 32) e = reduce_part2(d, c);
-  if (threadIdx.x == 0) {
-    RepState st = X[t.rep];
+  if (chain) e = reduce_part2(d, t.part2_off, t.npart2);
+  if (CHAIN && !chain) load_state();
+  if (CHAIN) __syncthreads();
+  if (i == lead) {
     const double pot = e.lj + e.clmb + e.wall;
+    const D5Terms f5 = d5_terms(c, st, pot, e.vir);   // L does not change before the second D5
     if (MID) {   // D5 (scalar) + D6 closing the previous step
-      for (int x = 0; x < 3; x++) sc.coef_v_a[x] = st.L[x] * st.s * c.dthalf;
+      for (int x = 0; x < 3; x++) sc.coef_v_a[x] = st.L[x] * st.s * c.dthalf * c.im;
       sc.coef_p_a = 2.0 * st.s * c.dthalf;
-      d5_scalar(c, st, pot, e.vir);
+      d5_apply(st, f5);
       d6(c, st);
     }
     d6(c, st);   // D6 opening this step
-    for (int x = 0; x < 3; x++) sc.coef_v_c[x] = st.L[x] * st.s * c.dthalf;
+    for (int x = 0; x < 3; x++) sc.coef_v_c[x] = st.L[x] * st.s * c.dthalf * c.im;
     sc.coef_p_c = 2.0 * st.s * c.dthalf;
-    d5_scalar(c, st, pot, e.vir);
+    d5_apply(st, f5);
+    const double si = 1.0 / st.s;   // D4 leaves s
+    sc.coef_xi = 0.25 * si;
     d4(c, st);
-    sc.coef_xi = 0.25 / st.s;
-    const double si = 1.0 / st.s;
-    sc.cxi1 = 0.25 * si;
     for (int x = 0; x < 3; x++) {
       const double Li = 1.0 / st.L[x];
       sc.coef_r[x] = Li * Li * si * c.dt;
     }
-    for (int x = 0; x < 3; x++) sc.Lb[x] = d.Lbuild[3 * tix + x];
-    if (tix == c.tile_off) Y[t.rep] = st;
+    if (tix == t.tile_off) Y[t.rep] = st;
   }
   __syncthreads();
-  const int i = threadIdx.x;
+  if (CHAIN && chain) return;
+  if (!CHAIN) load_state();
   double acc[4] = {0, 0, 0, 0};
   double disp = 0.0;
-  if (i < t.count) {
+  if (active) {
     const int li = t.start + i;
-    const int g = c.mol_off + li;
-    const int N = d.N;
-    double r[3], v[3], q[4], p[4], f[3], n[4];
-    for (int x = 0; x < 3; x++) { r[x] = d.r[x * N + g]; v[x] = d.v[x * N + g]; f[x] = d.f[x * N + g]; }
-    for (int x = 0; x < 4; x++) { q[x] = d.q[x * N + g]; p[x] = d.p[x * N + g]; n[x] = d.n[x * N + g]; }
-    const double m = c.mass;
-    if (MID) kick(v, p, q, f, n, sc.coef_v_a, sc.coef_p_a, m);
-    kick(v, p, q, f, n, sc.coef_v_c, sc.coef_p_c, m);
+    if (MID) kick(v, p, q, f, n, sc.coef_v_a, sc.coef_p_a);
+    kick(v, p, q, f, n, sc.coef_v_c, sc.coef_p_c);
     const bool T1 = (c.tconstant == 1);
     double sPs = 0.0;
-    double xi = rotate(q, p, 3, c.I[2], sc.coef_xi, c.dthalf);
+    double xi = rotate(q, p, 3, c.iI[2], sc.coef_xi, c.dthalf);
     if (T1) sPs += 0.5 * xi * xi * c.I[2];
-    xi = rotate(q, p, 2, c.I[1], sc.coef_xi, c.dthalf);
+    xi = rotate(q, p, 2, c.iI[1], sc.coef_xi, c.dthalf);
     if (T1) sPs += 0.5 * xi * xi * c.I[1];
+    int fx[3];
     for (int x = 0; x < 3; x++) {
       r[x] += v[x] * sc.coef_r[x];
       if (r[x] < 0.0) r[x] += 1.0;
       if (r[x] >= 1.0) r[x] -= 1.0;
+      fx[x] = fix_coord(r[x]);
+      d.r[x * N + g] = r[x];
+      d.v[x * N + g] = v[x];
     }
-    xi = rotate(q, p, 1, c.I[0], sc.cxi1, c.dt);
+    xi = rotate(q, p, 1, c.iI[0], sc.coef_xi, c.dt);
     if (c.pconstant > 0 || T1)
-      for (int x = 0; x < 3; x++) acc[x] = 2.0 * m * v[x] * v[x];
+      for (int x = 0; x < 3; x++) acc[x] = 2.0 * c.mass * v[x] * v[x];
     if (T1) sPs += xi * xi * c.I[0];
-    xi = rotate(q, p, 2, c.I[1], sc.coef_xi, c.dthalf);
-    if (T1) sPs += 0.5 * xi * xi * c.I[1];
-    xi = rotate(q, p, 3, c.I[2], sc.coef_xi, c.dthalf);
-    if (T1) sPs += 0.5 * xi * xi * c.I[2];
-    acc[3] = sPs;
-    for (int x = 0; x < 3; x++) { d.r[x * N + g] = r[x]; d.v[x * N + g] = v[x]; }
-    for (int x = 0; x < 4; x++) { d.q[x * N + g] = q[x]; d.p[x * N + g] = p[x]; }
-    write_pack(d, c, prec, li, r, q);
     // displacement since the last neighbour-list build, in the build box
-    const int4 ref = d.ref_com[g];
-    const int fx = fix_coord(r[0]), fy = fix_coord(r[1]), fz = fix_coord(r[2]);
-    const double dx = (double)wrap_diff(fx, ref.x) * kFixInv * sc.Lb[0];
-    const double dy = (double)wrap_diff(fy, ref.y) * kFixInv * sc.Lb[1];
-    const double dz = (double)wrap_diff(fz, ref.z) * kFixInv * sc.Lb[2];
+    const double dx = (double)wrap_diff(fx[0], ref.x) * kFixInv * sc.Lb[0];
+    const double dy = (double)wrap_diff(fx[1], ref.y) * kFixInv * sc.Lb[1];
+    const double dz = (double)wrap_diff(fx[2], ref.z) * kFixInv * sc.Lb[2];
     disp = sqrt(dx * dx + dy * dy + dz * dz);
     if (!(disp == disp)) disp = 1e30;   // NaN box: force a rebuild
+    xi = rotate(q, p, 2, c.iI[1], sc.coef_xi, c.dthalf);
+    if (T1) sPs += 0.5 * xi * xi * c.I[1];
+    xi = rotate(q, p, 3, c.iI[2], sc.coef_xi, c.dthalf);
+    if (T1) sPs += 0.5 * xi * xi * c.I[2];
+    acc[3] = sPs;
+    for (int x = 0; x < 4; x++) { d.q[x * N + g] = q[x]; d.p[x * N + g] = p[x]; }
+    write_pack(d, c, prec, li, r, q, fx);
   }
   warp_sum<4>(acc);
   disp = warp_max(disp);
@@ -316,11 +389,6 @@ __device__ inline CellGrid cell_grid(const RepConst& c, const double* L) {
   return g;
 }
 
-// The kListLanes bits of a warp ballot that belong to this lane's molecule.
-__device__ __forceinline__ unsigned group_bits(unsigned ballot, int lane) {
-  return (ballot >> (lane & ~(kListLanes - 1))) & ((1u << kListLanes) - 1u);
-}
-
 __device__ inline int cell_of(const int4 x, const CellGrid& g) {
   return (cell_coord(x.z, g.nz) * g.ny + cell_coord(x.y, g.ny)) * g.nx + cell_coord(x.x, g.nx);
 }
@@ -346,37 +414,56 @@ __global__ void __launch_bounds__(kRepThreads) k_replica_head(DevPtrs d, const R
   __shared__ int cnt[kMaxCells];
   __shared__ int wsum[kRepThreads / 32];
   __shared__ CellGrid grid;
-  const int rep = d.rep0 + blockIdx.x;
-  const RepConst& c = d.rc[rep];
+  const int rep = d.reps ? d.reps[blockIdx.x] : (int)blockIdx.x;
+  __shared__ RepConst c;
+  __shared__ RepState st0;
+  __shared__ double Lb[3];
+  {
+    const int tid = threadIdx.x;
+    const uint32_t* cs = reinterpret_cast<const uint32_t*>(d.rc + rep);
+    for (int k = tid; k < (int)(sizeof(RepConst) / 4); k += kRepThreads) reinterpret_cast<uint32_t*>(&c)[k] = cs[k];
+    const uint32_t* ys = reinterpret_cast<const uint32_t*>(Yin + rep);
+    if (tid >= 64 && tid < 64 + (int)(sizeof(RepState) / 4)) reinterpret_cast<uint32_t*>(&st0)[tid - 64] = ys[tid - 64];
+    // every tile of a replica holds the same build box
+    if (tid >= 128 && tid < 131) Lb[tid - 128] = d.Lbuild[3 * d.rc[rep].tile_off + tid - 128];
+  }
+  double v[4] = {0, 0, 0, 0}, disp = 0.0;
+  if (!FORCE_ONLY && threadIdx.x < 32) {
+    const int w0 = d.rc[rep].warp_off, w1 = w0 + d.rc[rep].nwarp;
+    for (int k = w0 + threadIdx.x; k < w1; k += 32) {
+      const Part1 p = d.part1[k];
+      v[0] += p.sum_Pv[0]; v[1] += p.sum_Pv[1]; v[2] += p.sum_Pv[2];
+      v[3] += p.sum_Ps;
+      disp = fmax(disp, p.disp);
+    }
+  }
+  __syncthreads();
   if (threadIdx.x < 32) {
-    double v[4] = {0, 0, 0, 0}, disp = 0.0;
+    const double log_s = log(st0.s);   // on every lane, ahead of the sums' exchange
     if (!FORCE_ONLY) {
-      for (int k = c.warp_off + threadIdx.x; k < c.warp_off + c.nwarp; k += 32) {
-        const Part1 p = d.part1[k];
-        v[0] += p.sum_Pv[0]; v[1] += p.sum_Pv[1]; v[2] += p.sum_Pv[2];
-        v[3] += p.sum_Ps;
-        disp = fmax(disp, p.disp);
-      }
       warp_sum<4>(v);
       disp = warp_max(disp);
     }
-    if (threadIdx.x == 0) {
-      RepState st = Yin[rep];
-      int rb = 1;
-      if (!FORCE_ONLY) {
-        double sPv[3] = {v[0], v[1], v[2]};
-        pspv(c, st, sPv, v[3]);
-        d4(c, st);
-        const int tix = c.tile_off;   // every tile of a replica holds the same build box
-        const double lb0 = d.Lbuild[3 * tix], lb1 = d.Lbuild[3 * tix + 1], lb2 = d.Lbuild[3 * tix + 2];
-        rb = !(lb0 == lb0);
-        if (!rb) {
-          const double lam = fmax(fmax(lb0 / st.L[0], lb1 / st.L[1]), lb2 / st.L[2]);
-          rb = (2.0 * disp + c.rc * (lam - 1.0) > c.skin);
-        }
+    RepState st = st0;
+    int rb = 1;
+    if (!FORCE_ONLY) {   // every lane runs the chain (the same bits); lane 0 stores
+      pspv(c, st, v, v[3], log_s);
+      d4(c, st);
+      rb = !(Lb[0] == Lb[0]);
+      if (!rb) {
+        // lam = max_x Lbuild_x / L_x, one dimension per lane
+        const int x = min((int)threadIdx.x, 2);
+        double lam = Lb[x] / st.L[x];
+        lam = fmax(fmax(__shfl_sync(0xffffffffu, lam, 0), __shfl_sync(0xffffffffu, lam, 1)),
+                   __shfl_sync(0xffffffffu, lam, 2));
+        rb = (2.0 * disp + c.rc * (lam - 1.0) > c.skin);
       }
+    }
+    if (threadIdx.x == 0) {
       Xout[rep] = st;   // FORCE_ONLY launches pass Xout == Yin: unchanged there
-      CellGrid g = cell_grid(c, st.L);
+      CellGrid g;
+      g.nx = g.ny = g.nz = 1;
+      if (rb) g = cell_grid(c, st.L);
       g.rebuild = rb;
       grid = g;
       d.cgrid[rep] = g;
@@ -427,7 +514,7 @@ __global__ void __launch_bounds__(kRepThreads) k_replica_head(DevPtrs d, const R
 
 // Neighbour-list rebuild for the molecules of this tile, one lane per molecule
 // (build_lists, the FP64 form; the FP32 form's build_lists_f32 below gives the
-// same lists with four lanes per molecule).  The list of molecule i holds, in
+// same lists with eight lanes per molecule).  The list of molecule i holds, in
 // ascending j, every j that passes the list test (below):
 //  * a replica not cut into cells (CellGrid 1 x 1 x 1): every molecule of the
 //    replica is tested, 128 candidates at a time from shared memory (all lanes
@@ -565,61 +652,69 @@ __device__ void build_lists(const DevPtrs& d, const RepConst& c, const Tile& t, 
   }
 }
 
-// FP32 skin-list build for the list kernel, kListLanes lanes per molecule
-// (molecule slot threadIdx.x / kListLanes, lane sub = threadIdx.x % kListLanes).
-// The lists are entry for entry those that build_lists gives with one lane per
-// molecule (the FP64 form still builds its lists that way):
-//  * all-molecule scan: lane sub tests candidates sub, sub + 4, ... of each
-//    128-molecule chunk staged in shared memory, and a ballot places the kept
-//    ones in ascending j;
-//  * cell lists: the lanes split each neighbouring cell's molecules and set
-//    the molecule's bitmap row with shared-memory atomics; the row is then
-//    emitted in ascending j, lane sub taking words sub, sub + 4, ..., placed by
-//    a prefix of their popcounts over the group.
-// Returns the list length (equal on the group's lanes); lane 0 stores it.
-__device__ int build_lists_f32(const DevPtrs& d, const RepConst& c, const Tile& t, const double* L,
-                               uint16_t* nb, int T, uint32_t* bm, int win) {
-  __shared__ int4 cand[128];
-  const int i = threadIdx.x / kListLanes, sub = threadIdx.x % kListLanes, lane = threadIdx.x & 31;
-  const unsigned below = (1u << sub) - 1u;
-  const bool valid = i < t.count;
-  const int li = t.start + i;
+// FP32 skin-list build, kGroup lanes per molecule: a warp builds the lists of
+// kWarpMol consecutive molecules from li0 on, row-major (molecule li's list at
+// d.nbr + nbr_off + li * nbr_stride).  The lists are entry for entry those that
+// build_lists gives with one lane per molecule (the FP64 form still builds its
+// lists that way):
+//  * all-molecule scan: a lane loads one candidate and tests it against the
+//    warp's molecules, so that one load serves kWarpMol tests and 32 candidates
+//    advance per round; a ballot per molecule places the kept ones in
+//    ascending j;
+//  * cell lists: the molecule's kGroup lanes split each neighbouring cell's
+//    molecules and set its bitmap row with shared-memory atomics; the row is
+//    then emitted in ascending j, lane sub taking words sub, sub + kGroup, ...,
+//    placed by a prefix of their popcounts over the group.
+__device__ void build_lists_f32(const DevPtrs& d, const RepConst& c, int rep, int li0, const double* L,
+                                uint32_t* bm, int win) {
+  const int lane = threadIdx.x & 31, grp = lane / kGroup, sub = lane % kGroup;
   const float lsc0 = (float)(L[0] * (1.0 / 65536.0)), lsc1 = (float)(L[1] * (1.0 / 65536.0)),
               lsc2 = (float)(L[2] * (1.0 / 65536.0));
   const double rw = list_test_radius(c, L);
   const float rl2f = (float)(rw * rw);
   const int4* com = d.com + c.mol_off;
-  const int4 me = valid ? com[li] : make_int4(0, 0, 0, 0);
-  const CellGrid g = d.cgrid[t.rep];
-  int cnt = 0;
+  uint16_t* nb0 = d.nbr + c.nbr_off + (long long)li0 * c.nbr_stride;
+  const int nmol = c.nmol, cap = c.nbr_cap;
+  const CellGrid g = d.cgrid[rep];
+  int cnt = 0;   // entries of molecule li0 + grp
   if (g.nx * g.ny * g.nz == 1) {
-    for (int base = 0; base < c.nmol; base += 128) {   // uniform over the block
-      __syncthreads();
-      for (int k = threadIdx.x; k < 128 && base + k < c.nmol; k += blockDim.x) cand[k] = com[base + k];
-      __syncthreads();
-      const int nk = min(128, c.nmol - base);
-      for (int k0 = 0; k0 < nk; k0 += kListLanes) {
-        const int k = k0 + sub, j = base + k;
-        const bool in = valid && k < nk && j != li &&
-                        list_test<kF32>(me, cand[k], lsc0, lsc1, lsc2, rl2f, 0.0, 0.0, 0.0, nullptr, L, 0.0);
-        const unsigned gb = group_bits(__ballot_sync(0xffffffffu, in), lane);
-        if (in) {
-          const int pos = cnt + __popc(gb & below);
-          if (pos < c.nbr_cap) nb[(long long)pos * T] = (uint16_t)j;
-        }
-        cnt += __popc(gb);
+    int4 me[kWarpMol];
+    int n[kWarpMol];
+#pragma unroll
+    for (int m = 0; m < kWarpMol; m++) {
+      me[m] = com[min(li0 + m, nmol - 1)];
+      n[m] = 0;
+    }
+    const unsigned below = (1u << lane) - 1u;
+    for (int base = 0; base < nmol; base += 32) {
+      const int j = base + lane;
+      const int4 cj = com[min(j, nmol - 1)];
+#pragma unroll
+      for (int m = 0; m < kWarpMol; m++) {
+        const bool in = j < nmol && j != li0 + m &&
+                        list_test<kF32>(me[m], cj, lsc0, lsc1, lsc2, rl2f, 0.0, 0.0, 0.0, nullptr, L, 0.0);
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        const int pos = n[m] + __popc(b & below);
+        if (in && pos < cap && li0 + m < nmol) nb0[(long long)m * c.nbr_stride + pos] = (uint16_t)j;
+        n[m] += __popc(b);
       }
     }
+#pragma unroll
+    for (int m = 0; m < kWarpMol; m++) cnt = (grp == m) ? n[m] : cnt;
   } else {
-    uint32_t* row = bm + i * (win | 1);   // odd row length: the molecules' words fall in distinct banks
-    const int W = (c.nmol + 31) >> 5;
+    const int li = li0 + grp;
+    const bool valid = li < nmol;
+    const int4 me = com[min(li, nmol - 1)];
+    uint16_t* nb = nb0 + (long long)grp * c.nbr_stride;
+    uint32_t* row = bm + (threadIdx.x / kGroup) * (win | 1);   // odd row length: the molecules' words in distinct banks
+    const int W = (nmol + 31) >> 5;
     const int cx = cell_coord(me.x, g.nx), cy = cell_coord(me.y, g.ny), cz = cell_coord(me.z, g.nz);
     const int ox = (g.nx == 1) ? 0 : 1, oy = (g.ny == 1) ? 0 : 1, oz = (g.nz == 1) ? 0 : 1;
-    const int* cs = d.cell_start + (long long)t.rep * (kMaxCells + 1);
+    const int* cs = d.cell_start + (long long)rep * (kMaxCells + 1);
     const int4* cm = d.cell_com + c.mol_off;
-    for (int w0 = 0; w0 < W; w0 += win) {   // uniform over the block
+    for (int w0 = 0; w0 < W; w0 += win) {   // uniform over the warp
       const int nw = min(win, W - w0);
-      for (int w = sub; w < nw; w += kListLanes) row[w] = 0u;
+      for (int w = sub; w < nw; w += kGroup) row[w] = 0u;
       __syncwarp();
       const int jlo = 32 * w0, jhi = 32 * (w0 + nw);
       if (valid) {
@@ -637,7 +732,7 @@ __device__ int build_lists_f32(const DevPtrs& d, const RepConst& c, const Tile& 
               xc -= (xc >= g.nx) ? g.nx : 0;
               const int cell = (zc * g.ny + yc) * g.nx + xc;
               const int e = cs[cell + 1];
-              for (int k = cs[cell] + sub; k < e; k += kListLanes) {
+              for (int k = cs[cell] + sub; k < e; k += kGroup) {
                 const int4 cj = cm[k];
                 const int j = cj.w;
                 if (j < jlo || j >= jhi || j == li) continue;
@@ -649,13 +744,13 @@ __device__ int build_lists_f32(const DevPtrs& d, const RepConst& c, const Tile& 
         }
       }
       __syncwarp();
-      for (int w = 0; w < nw; w += kListLanes) {   // uniform over the block
+      for (int w = 0; w < nw; w += kGroup) {   // uniform over the warp
         const uint32_t word = (w + sub < nw) ? row[w + sub] : 0u;
         const int n = __popc(word);
         int incl = n;   // inclusive prefix of n over the group's lanes
 #pragma unroll
-        for (int o = 1; o < kListLanes; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, incl, o, kListLanes);
+        for (int o = 1; o < kGroup; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o, kGroup);
           if (sub >= o) incl += y;
         }
         int pos = cnt + incl - n;
@@ -663,23 +758,22 @@ __device__ int build_lists_f32(const DevPtrs& d, const RepConst& c, const Tile& 
         while (bits) {
           const int j = jlo + 32 * (w + sub) + (__ffs(bits) - 1);
           bits &= bits - 1u;
-          if (pos < c.nbr_cap) nb[(long long)pos * T] = (uint16_t)j;
+          if (pos < cap && valid) nb[pos] = (uint16_t)j;
           pos++;
         }
-        cnt += __shfl_sync(0xffffffffu, incl, kListLanes - 1, kListLanes);
+        cnt += __shfl_sync(0xffffffffu, incl, kGroup - 1, kGroup);
       }
       __syncwarp();   // the row is cleared again for the next window
     }
   }
-  if (cnt > c.nbr_cap) {
-    if (valid && sub == 0) {
+  if (sub == 0 && li0 + grp < nmol) {
+    if (cnt > cap) {
       atomicOr(d.err, kErrNbrOverflow);
-      atomicMax(&d.status[t.rep], 8);
+      atomicMax(&d.status[rep], 8);
+      cnt = cap;
     }
-    cnt = c.nbr_cap;
+    d.nbr_cnt[c.mol_off + li0 + grp] = cnt;
   }
-  if (valid && sub == 0) d.nbr_cnt[c.mol_off + li] = cnt;
-  return cnt;
 }
 
 // Accumulators of one molecule i.
@@ -689,337 +783,6 @@ struct IAcc {
   double vir[3], lj, clmb;
   long long npair;
 };
-
-// FP32 pair loop over i's neighbour list, in two passes run by two kernels.
-// Pass 1 (k_force_lists) scans the (rcut + skin) list and writes the neighbours
-// within rcut, in the list's ascending-j order, to i's column of the per-step
-// list `nbt` (same layout and capacity as the skin list; it cannot overflow).  Under the
-// per-site minimum image (SIMG, below) it splits them: pairs whose COM vector
-// keeps every site-pair component clear of +-L/2 ("far", from the front of the
-// column) need no per-site image at all; the others ("near", from the back)
-// get the per-site image.  Pass 2 computes exactly those pairs, so the lanes of
-// a warp stay converged (no cutoff branch) and differ only in their counts
-// (k_force_pairs).  Pass 1 runs in its own light kernel, whose occupancy hides
-// the latency of its gathered loads; pass 2 is register-heavy.
-// Pair math in FP32 (rsqrt on the SFU plus one Newton step); partial sums in
-// FP32 over 32 pairs, then FP64 accumulation into this thread's slots of `acc`
-// (shared memory, field f at acc[f * blockDim.x + threadIdx.x]: 3S site-force
-// components, 3 switching-correction, 3 virial, LJ, Coulomb).  The pairs within
-// rcut, their far/near class and order, and their grouping by 32 depend only
-// on the positions, not on when the skin list was built.  The next
-// neighbour's index is read one pair ahead of its use.
-// SIMG: apply the minimum image to every site pair as the reference does
-// (src/force_calculator.cxx:737-741).  It changes the result only when a box
-// length is below 2 (rc + 2 site_reach); the caller enables it just then.
-struct F32Const {
-  float qq[kMaxSites][kMaxSites];
-  float Ls[3], Lf[3], hL[3];
-  double L[3];
-};
-
-// Per-site minimum image (SIMG) flips a site-pair vector by a box length where
-// one of its components crosses +-L/2, so the FP32 and FP64 forms must take the
-// same image there.  A site pair with a component within kImageTol of L/2
-// (FP32 rounding of the site vector is below ~4e-6 A) is left out of the pair
-// loop (its vector is set far away, so its terms vanish) and added afterwards
-// by site_pair_exact: the image is decided with the FP64 form's arithmetic
-// (pair_loop_f64: COM vector from the FP64 box fractions, site offsets R(q) b
-// in FP64), then the terms are evaluated as in the loop.  Up to kMaxDefer such
-// site pairs per molecule and step are deferred; further ones (never seen in
-// practice) keep the FP32 image.
-constexpr float kImageTol = 2e-5f;
-constexpr int kMaxDefer = 2;
-
-template <int S, int C0>
-__device__ __noinline__ void site_pair_exact(const DevPtrs& d, const RepConst& c, const F32Const& k32, int li,
-                                             int code, double* acc) {
-  const int j = code >> 8, kk = (code >> 4) & 15, l = code & 15;
-  const int T = blockDim.x, tid = threadIdx.x;
-  const int N = d.N, gi = c.mol_off + li, gj = c.mol_off + j;
-  const double* L = k32.L;
-  // COM vector and switch exactly as the FP32 loop forms them
-  const uint32_t* base = reinterpret_cast<const uint32_t*>(d.pack) + c.pack_off;
-  const int stride = c.pack_stride;
-  const int* wi = reinterpret_cast<const int*>(base + (long long)li * stride);
-  const int* wj = reinterpret_cast<const int*>(base + (long long)j * stride);
-  const float dx = (float)wrap_diff(wi[0], wj[0]) * k32.Ls[0];
-  const float dy = (float)wrap_diff(wi[1], wj[1]) * k32.Ls[1];
-  const float dz = (float)wrap_diff(wi[2], wj[2]) * k32.Ls[2];
-  const float r2 = dx * dx + dy * dy + dz * dz;
-  const float rinv = rsqrtf(r2);
-  const float r = r2 * rinv;
-  const float rc = (float)c.rc, rs = (float)c.rs, coef = (float)c.coef_sw;
-  float sw = 1.f, dsw = 0.f;
-  if (r > rs) {
-    const float r01c = r - rc, r01l = r - rs;
-    sw = coef * r01c * r01c * r01c * (10.f * r01l * r01l - 5.f * r01l * r01c + r01c * r01c);
-    dsw = coef * 30.f * r01c * r01c * r01l * r01l;
-  }
-  // the site vector with the FP64 form's image
-  double qi[4], qj[4], si[3], sj[3];
-  for (int x = 0; x < 4; x++) { qi[x] = d.q[x * N + gi]; qj[x] = d.q[x * N + gj]; }
-  body_to_space(qi, c.body[kk], si);
-  body_to_space(qj, c.body[l], sj);
-  float v[3];
-  for (int x = 0; x < 3; x++) {
-    double gr = (d.r[x * N + gi] - d.r[x * N + gj]) * L[x];
-    if (gr >= 0.5 * L[x]) gr -= L[x];
-    if (gr < -0.5 * L[x]) gr += L[x];
-    double rv = gr + si[x] - sj[x];
-    if (rv >= 0.5 * L[x]) rv -= L[x];
-    if (rv < -0.5 * L[x]) rv += L[x];
-    v[x] = (float)rv;
-  }
-  const float rr = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-  float ri = rsqrtf(rr);
-  ri = ri * fmaf(-0.5f * rr * ri, ri, 1.5f);
-  const float ri2 = ri * ri;
-  float ftmp = 0.f, elj = 0.f, ecl = 0.f;
-  if (kk == 0 && l == 0) {
-    float s6 = (float)c.sgm2 * ri2;
-    s6 = s6 * s6 * s6;
-    elj = (float)(4.0 * c.eps) * s6 * (s6 - 1.f);
-    ftmp += (float)(48.0 * c.eps) * s6 * (s6 - 0.5f) * ri2;
-  }
-  if (kk >= C0 && l >= C0) {
-    ecl = k32.qq[kk][l] * ri;
-    ftmp += ecl * ri2;
-  }
-  ftmp *= sw;
-  const float t[3] = {v[0] * ftmp, v[1] * ftmp, v[2] * ftmp};
-  const float g = dsw * rinv * (elj + ecl);
-  const float cv[3] = {-dx * g, -dy * g, -dz * g};
-  const float dv[3] = {dx, dy, dz};
-  for (int x = 0; x < 3; x++) {
-    acc[(3 * kk + x) * T + tid] += (double)t[x];
-    acc[(3 * S + x) * T + tid] += (double)cv[x];
-    acc[(3 * S + 3 + x) * T + tid] += (double)((t[x] + cv[x]) * dv[x]);
-  }
-  acc[(3 * S + 6) * T + tid] += (double)(sw * elj);
-  acc[(3 * S + 7) * T + tid] += (double)(sw * ecl);
-}
-
-// Pass 1 for molecule li of tile t, run by its kListLanes lanes (sub = 0..3):
-// the neighbours of its (rcut + skin) list that are within rcut, in ascending
-// j, into its column of `nt` -- far pairs from the front, near pairs (SIMG
-// only) from the back.  Lane sub tests list entries sub, sub + 4, ...; a round
-// of the group covers four consecutive entries, and the kept ones are placed by
-// a ballot in list order, so the lists equal those of one lane walking the
-// list in turn.  Four rounds per batch, so that their record loads are in
-// flight together.  Lane 0 stores nfar | nnear << 16 in d.nt_cnt.  Every lane
-// of the warp runs the warp's longest list (ballots need the whole warp).
-template <bool SIMG>
-__device__ void tight_lists_f32(const DevPtrs& d, const RepConst& c, int li, bool valid, int sub,
-                                const double* L, const uint16_t* nb, uint16_t* nt, int cnt, int T) {
-  const int4* base = d.com + c.mol_off;   // compact centres: 16 B per molecule, L1-resident
-  const float Ls0 = (float)(L[0] * kFixInv), Ls1 = (float)(L[1] * kFixInv), Ls2 = (float)(L[2] * kFixInv);
-  const float rc2 = (float)(c.rc * c.rc);
-  const int4 ui = valid ? __ldg(base + li) : make_int4(0, 0, 0, 0);
-  const int xi = ui.x, yi = ui.y, zi = ui.z;
-  // far bound: |d_x| below it keeps every site-pair component below L/2 - kImageTol
-  float bnd0 = 0.f, bnd1 = 0.f, bnd2 = 0.f;
-  if (SIMG) {
-    const float m = 2.f * (float)c.site_reach + kImageTol + 1e-3f;
-    bnd0 = 0.5f * (float)L[0] - m; bnd1 = 0.5f * (float)L[1] - m; bnd2 = 0.5f * (float)L[2] - m;
-  }
-  const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << sub) - 1u;
-  const int back = c.nbr_cap - 1;
-  int nfar = 0, nnear = 0;
-  const int rounds = __reduce_max_sync(0xffffffffu, (cnt + kListLanes - 1) / kListLanes);
-  constexpr int B = 4;
-  for (int r0 = 0; r0 < rounds; r0 += B) {
-    int j[B];
-    int4 u[B];
-#pragma unroll
-    for (int m = 0; m < B; m++) {
-      const int k = (r0 + m) * kListLanes + sub;
-      j[m] = (k < cnt) ? (int)nb[(long long)k * T] : -1;
-    }
-#pragma unroll
-    for (int m = 0; m < B; m++) u[m] = (j[m] >= 0) ? __ldg(base + j[m]) : ui;
-#pragma unroll
-    for (int m = 0; m < B; m++) {
-      const float dx = (float)wrap_diff(xi, u[m].x) * Ls0, dy = (float)wrap_diff(yi, u[m].y) * Ls1,
-                  dz = (float)wrap_diff(zi, u[m].z) * Ls2;
-      const bool in = j[m] >= 0 && dx * dx + dy * dy + dz * dz <= rc2;
-      const bool near = SIMG && in && (fabsf(dx) >= bnd0 || fabsf(dy) >= bnd1 || fabsf(dz) >= bnd2);
-      const unsigned gf = group_bits(__ballot_sync(0xffffffffu, in && !near), lane);
-      if (in && !near) nt[(long long)(nfar + __popc(gf & below)) * T] = (uint16_t)j[m];
-      nfar += __popc(gf);
-      if (SIMG) {
-        const unsigned gn = group_bits(__ballot_sync(0xffffffffu, near), lane);
-        if (near) nt[(long long)(back - nnear - __popc(gn & below)) * T] = (uint16_t)j[m];
-        nnear += __popc(gn);
-      }
-    }
-  }
-  if (valid && sub == 0) d.nt_cnt[c.mol_off + li] = nfar | (nnear << 16);
-}
-
-template <int S, int C0, bool SIMG>
-__device__ void pair_loop_f32(const DevPtrs& d, const RepConst& c, const F32Const& k32, int li,
-                              const uint16_t* nt, int lstride, int nfar, int nnear, int p0, int p1,
-                              double* acc) {
-  constexpr int STRIDE = ((3 + 3 * S) + 3) / 4 * 4;
-  constexpr int NV = STRIDE / 4;
-  const int T = blockDim.x, tid = threadIdx.x;   // accumulator slots
-  const uint4* base = reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(d.pack) + c.pack_off);
-  const float Ls0 = k32.Ls[0], Ls1 = k32.Ls[1], Ls2 = k32.Ls[2];
-  int xi, yi, zi;
-  float si[S][3];
-  {
-    uint32_t wi[STRIDE];
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-      const uint4 u = __ldg(base + (long long)li * NV + k);
-      wi[4 * k] = u.x; wi[4 * k + 1] = u.y; wi[4 * k + 2] = u.z; wi[4 * k + 3] = u.w;
-    }
-    xi = (int)wi[0]; yi = (int)wi[1]; zi = (int)wi[2];
-#pragma unroll
-    for (int k = 0; k < S; k++)
-#pragma unroll
-      for (int x = 0; x < 3; x++) si[k][x] = __uint_as_float(wi[3 + 3 * k + x]);
-  }
-  const int back = c.nbr_cap - 1;
-  const float rc = (float)c.rc, rs = (float)c.rs;
-  const float coef = (float)c.coef_sw;
-  const float sgm2 = (float)c.sgm2, eps4 = (float)(4.0 * c.eps), eps48 = (float)(48.0 * c.eps);
-
-  float fs[S][3], fc[3], fv[3], flj, fcl;
-  auto zero = [&]() {
-#pragma unroll
-    for (int k = 0; k < S; k++) fs[k][0] = fs[k][1] = fs[k][2] = 0.f;
-    fc[0] = fc[1] = fc[2] = 0.f;
-    fv[0] = fv[1] = fv[2] = 0.f;
-    flj = fcl = 0.f;
-  };
-  auto flush = [&]() {
-#pragma unroll
-    for (int k = 0; k < S; k++)
-#pragma unroll
-      for (int x = 0; x < 3; x++) acc[(3 * k + x) * T + tid] += (double)fs[k][x];
-#pragma unroll
-    for (int x = 0; x < 3; x++) {
-      acc[(3 * S + x) * T + tid] += (double)fc[x];
-      acc[(3 * S + 3 + x) * T + tid] += (double)fv[x];
-    }
-    acc[(3 * S + 6) * T + tid] += (double)flj;
-    acc[(3 * S + 7) * T + tid] += (double)fcl;
-  };
-  zero();
-  int done = 0;                       // pairs accumulated (partial sums close every 32)
-  int ndef = 0, def0 = 0, def1 = 0;   // deferred site pairs (near pass only)
-
-  // pass 2: `n` pairs of the list starting at column slot `pos0`, stepping `dir`;
-  // IMG: per-site minimum image with exact ties (near pairs)
-  auto run = [&](auto img, int n, int pos0, int dir) {
-    constexpr bool IMG = decltype(img)::value;
-    const float hL0 = k32.hL[0], hL1 = k32.hL[1], hL2 = k32.hL[2];
-    const float Lf0 = k32.Lf[0], Lf1 = k32.Lf[1], Lf2 = k32.Lf[2];
-    // the next neighbour's index one pair ahead; the record at the top of the
-    // iteration (a record held in registers one pair ahead was 5 % slower)
-    int jnext = (n > 0) ? nt[(long long)pos0 * lstride] : 0;
-    for (int k = 0; k < n; k++) {
-      const int jcur = jnext;
-      if (k + 1 < n) jnext = nt[(long long)(pos0 + dir * (k + 1)) * lstride];
-      uint32_t wj[STRIDE];
-#pragma unroll
-      for (int m = 0; m < NV; m++) {
-        const uint4 u = __ldg(base + (long long)jcur * NV + m);
-        wj[4 * m] = u.x; wj[4 * m + 1] = u.y; wj[4 * m + 2] = u.z; wj[4 * m + 3] = u.w;
-      }
-      const float dx = (float)wrap_diff(xi, (int)wj[0]) * Ls0;
-      const float dy = (float)wrap_diff(yi, (int)wj[1]) * Ls1;
-      const float dz = (float)wrap_diff(zi, (int)wj[2]) * Ls2;
-      const float r2 = dx * dx + dy * dy + dz * dz;
-      const float rinv = rsqrtf(r2);
-      const float r = r2 * rinv;
-      float sw = 1.f, dsw = 0.f;
-      if (r > rs) {
-        const float r01c = r - rc, r01l = r - rs;
-        sw = coef * r01c * r01c * r01c * (10.f * r01l * r01l - 5.f * r01l * r01c + r01c * r01c);
-        dsw = coef * 30.f * r01c * r01c * r01l * r01l;
-      }
-      float elj = 0.f, ecl = 0.f;
-      float fpx = 0.f, fpy = 0.f, fpz = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < S; kk++) {
-        if (kk != 0 && kk < C0) continue;
-        const float ax = dx + si[kk][0], ay = dy + si[kk][1], az = dz + si[kk][2];
-        float tx = 0.f, ty = 0.f, tz = 0.f;
-#pragma unroll
-        for (int l = 0; l < S; l++) {
-          const bool lj_pair = (kk == 0 && l == 0);
-          const bool cl_pair = (kk >= C0 && l >= C0);
-          if (!lj_pair && !cl_pair) continue;
-          float x = ax - __uint_as_float(wj[3 + 3 * l]);
-          float y = ay - __uint_as_float(wj[3 + 3 * l + 1]);
-          float z = az - __uint_as_float(wj[3 + 3 * l + 2]);
-          if (IMG) {
-            if ((fabsf(fabsf(x) - hL0) < kImageTol || fabsf(fabsf(y) - hL1) < kImageTol ||
-                 fabsf(fabsf(z) - hL2) < kImageTol) && ndef < kMaxDefer) {
-              const int code = (jcur << 8) | (kk << 4) | l;
-              if (ndef == 0) def0 = code; else def1 = code;
-              ndef++;
-              x = y = z = 1e18f;   // this site pair's terms vanish here; added exactly below
-            }
-            if (x >= hL0) x -= Lf0;
-            if (x < -hL0) x += Lf0;
-            if (y >= hL1) y -= Lf1;
-            if (y < -hL1) y += Lf1;
-            if (z >= hL2) z -= Lf2;
-            if (z < -hL2) z += Lf2;
-          }
-          const float rr = x * x + y * y + z * z;
-          float ri = rsqrtf(rr);
-          ri = ri * fmaf(-0.5f * rr * ri, ri, 1.5f);   // one Newton step: ~0.5 ulp
-          const float ri2 = ri * ri;
-          float ftmp = 0.f;
-          if (lj_pair) {
-            float s6 = sgm2 * ri2;
-            s6 = s6 * s6 * s6;
-            elj += eps4 * s6 * (s6 - 1.f);
-            ftmp += eps48 * s6 * (s6 - 0.5f) * ri2;
-          }
-          if (cl_pair) {
-            const float e = k32.qq[kk][l] * ri;
-            ecl += e;
-            ftmp += e * ri2;
-          }
-          tx += x * ftmp; ty += y * ftmp; tz += z * ftmp;
-        }
-        // the switch multiplies the site forces once per site (FFMA into the sums)
-        fs[kk][0] = fmaf(sw, tx, fs[kk][0]);
-        fs[kk][1] = fmaf(sw, ty, fs[kk][1]);
-        fs[kk][2] = fmaf(sw, tz, fs[kk][2]);
-        fpx += tx; fpy += ty; fpz += tz;
-      }
-      const float e = elj + ecl;
-      const float g = dsw * rinv * e;
-      const float cx = -dx * g, cy = -dy * g, cz = -dz * g;
-      fc[0] += cx; fc[1] += cy; fc[2] += cz;
-      fv[0] += fmaf(fpx, sw, cx) * dx;
-      fv[1] += fmaf(fpy, sw, cy) * dy;
-      fv[2] += fmaf(fpz, sw, cz) * dz;
-      flj += sw * elj;
-      fcl += sw * ecl;
-      if ((++done & 31) == 0) { flush(); zero(); }
-    }
-  };
-  // positions [p0, p1) of the sequence far pairs (rows 0..) then near pairs (rows back, back-1, ..)
-  const int f1 = min(p1, nfar);
-  run(std::false_type{}, max(f1 - p0, 0), p0, 1);
-  if (SIMG) {
-    const int q0 = max(p0, nfar);
-    run(std::true_type{}, max(p1 - q0, 0), back - (q0 - nfar), -1);
-  }
-  flush();
-  if (SIMG && ndef > 0) {
-    site_pair_exact<S, C0>(d, c, k32, li, def0, acc);
-    if (ndef > 1) site_pair_exact<S, C0>(d, c, k32, li, def1, acc);
-  }
-}
 
 template <int S, int C0, bool SIMG>
 __device__ void pair_loop_f64(const DevPtrs& d, const RepConst& c, const Tile& t, const double* L,
@@ -1099,7 +862,37 @@ __device__ void pair_loop_f64(const DevPtrs& d, const RepConst& c, const Tile& t
   }
 }
 
-// Wall on the oxygen site and A2M for molecule g (FP64): writes d.f, d.n.
+// Wall on the oxygen site of a molecule at (r, q): adds the force to f and
+// returns the energy (ForceCalculator::Confined, src/force_calculator.cxx:1527-1566;
+// slit: src/remdgpu.cu:1708-1720).
+__device__ __forceinline__ double wall_site(const DevPtrs& d, const RepConst& c, const double* q, const double* r,
+                                            const double* L, double* f) {
+  double o[3];
+  body_to_space(q, c.body[0], o);
+  const double2* fw = reinterpret_cast<const double2*>(d.wall) + c.wall_off;
+  const double dr = c.wall_dr;
+  if (c.confined == 1) {
+    const double x = r[0] * L[0] + o[0] - L[0] * 0.5;
+    const double y = r[1] * L[1] + o[1] - L[1] * 0.5;
+    const double r01 = sqrt(x * x + y * y);
+    int idx = (r01 >= 0.0) ? (int)fmin(r01 / dr, (double)(c.nfwall - 2)) : 0;   // NaN -> 0
+    const double2 w0 = fw[idx], w1 = fw[idx + 1];
+    const double fr = (w1.x - w0.x) / dr * (r01 - dr * idx) + w0.x;
+    f[0] += fr * x;
+    f[1] += fr * y;
+    return (w1.y - w0.y) / dr * (r01 - dr * idx) + w0.y;
+  }
+  const double z = r[2] * L[2] + o[2] - 0.5 * L[2];
+  const double za = fabs(z);
+  const double dir = (za != 0.0) ? z / za : 1.0;
+  int idx = (za >= 0.0) ? (int)fmin(za / dr, (double)(c.nfwall - 2)) : 0;       // NaN -> 0
+  const double2 w0 = fw[idx], w1 = fw[idx + 1];
+  const double fz = (w1.x - w0.x) / dr * (za - dr * idx) + w0.x;
+  f[2] += fz * dir;
+  return (w1.y - w0.y) / dr * (za - dr * idx) + w0.y;
+}
+
+// Wall and A2M for molecule g (FP64 form): writes d.f, d.n.
 template <int S>
 __device__ void finish_molecule(const DevPtrs& d, const RepConst& c, int g, const double* L, IAcc& a,
                                 double& wall_e) {
@@ -1107,36 +900,7 @@ __device__ void finish_molecule(const DevPtrs& d, const RepConst& c, int g, cons
   double q[4], r[3];
   for (int x = 0; x < 4; x++) q[x] = d.q[x * N + g];
   for (int x = 0; x < 3; x++) r[x] = d.r[x * N + g];
-  // wall on the oxygen site (ForceCalculator::Confined, src/force_calculator.cxx:1527-1566;
-  // slit: src/remdgpu.cu:1708-1720)
-  if (c.confined > 0) {
-    double o[3];
-    body_to_space(q, c.body[0], o);
-    const double2* fw = reinterpret_cast<const double2*>(d.wall) + c.wall_off;
-    const double dr = c.wall_dr;
-    if (c.confined == 1) {
-      const double x = r[0] * L[0] + o[0] - L[0] * 0.5;
-      const double y = r[1] * L[1] + o[1] - L[1] * 0.5;
-      const double r01 = sqrt(x * x + y * y);
-      int idx = (r01 >= 0.0) ? (int)fmin(r01 / dr, (double)(c.nfwall - 2)) : 0;   // NaN -> 0
-      const double2 w0 = fw[idx], w1 = fw[idx + 1];
-      const double f = (w1.x - w0.x) / dr * (r01 - dr * idx) + w0.x;
-      const double e = (w1.y - w0.y) / dr * (r01 - dr * idx) + w0.y;
-      a.fs[0][0] += f * x;
-      a.fs[0][1] += f * y;
-      wall_e = e;
-    } else {
-      const double z = r[2] * L[2] + o[2] - 0.5 * L[2];
-      const double za = fabs(z);
-      const double dir = (za != 0.0) ? z / za : 1.0;
-      int idx = (za >= 0.0) ? (int)fmin(za / dr, (double)(c.nfwall - 2)) : 0;     // NaN -> 0
-      const double2 w0 = fw[idx], w1 = fw[idx + 1];
-      const double f = (w1.x - w0.x) / dr * (za - dr * idx) + w0.x;
-      const double e = (w1.y - w0.y) / dr * (za - dr * idx) + w0.y;
-      a.fs[0][2] += f * dir;
-      wall_e = e;
-    }
-  }
+  if (c.confined > 0) wall_e = wall_site(d, c, q, r, L, a.fs[0]);
   // A2M: molecular force and body torque (src/molecules.cxx:447-475)
   double F[3] = {a.fc[0], a.fc[1], a.fc[2]};
   double nq[4] = {0, 0, 0, 0};
@@ -1155,19 +919,22 @@ __device__ void finish_molecule(const DevPtrs& d, const RepConst& c, int g, cons
   for (int x = 0; x < 4; x++) d.n[x * N + g] = nq[x];
 }
 
-// Force partials of the tile's 32-molecule units (one fixed shuffle tree per warp).
+// Force partials of the tile's units of kPart2Mol molecules (a fixed shuffle tree
+// over kPart2Mol lanes; FP64 form, one lane per molecule).
 __device__ inline void write_part2(const DevPtrs& d, const RepConst& c, const Tile& t, const IAcc& a,
                                    double wall_e) {
-  double s6[7] = {a.lj, a.clmb, wall_e, a.vir[0], a.vir[1], a.vir[2], (double)a.npair};
-  warp_sum<7>(s6);
-  const int w = (t.start + threadIdx.x) >> 5;   // 32-molecule unit of the replica
-  if ((threadIdx.x & 31) == 0 && w < c.nwarp) {
+  double s7[7] = {a.lj, a.clmb, wall_e, a.vir[0], a.vir[1], a.vir[2], (double)a.npair};
+#pragma unroll
+  for (int k = 0; k < 7; k++)
+    for (int o = kPart2Mol / 2; o > 0; o >>= 1) s7[k] += __shfl_xor_sync(0xffffffffu, s7[k], o);
+  const int w = (t.start + threadIdx.x) / kPart2Mol;
+  if (threadIdx.x % kPart2Mol == 0 && w < c.npart2) {
     Part2 p;
-    p.lj = s6[0]; p.clmb = s6[1]; p.wall = s6[2];
-    p.vir[0] = s6[3]; p.vir[1] = s6[4]; p.vir[2] = s6[5];
-    p.npairs = (long long)llrint(s6[6]);
+    p.lj = s7[0]; p.clmb = s7[1]; p.wall = s7[2];
+    p.vir[0] = s7[3]; p.vir[1] = s7[4]; p.vir[2] = s7[5];
+    p.npairs = (long long)llrint(s7[6]);
     p.pad = 0.0;
-    d.part2[c.warp_off + w] = p;
+    d.part2[c.part2_off + w] = p;
   }
 }
 
@@ -1221,71 +988,376 @@ __device__ void force_tile_f64(const DevPtrs& d, const RepConst& c, const Tile& 
   write_part2(d, c, t, a, wall_e);
 }
 
-// FP32 form, pass 2 + wall + A2M (the per-step list comes from k_force_lists).
-// Two threads per molecule: thread (i, ch) computes positions [ch n/2, (ch+1) n/2)
-// of i's n pairs, so a launch has twice the work units (a shorter tail); the
-// two FP64 partials are added in chunk order.  The split is by list position
-// and the list holds exactly the pairs within rcut in ascending j, so results
-// depend neither on the tile size nor on the list history.
-constexpr int kPairChunks = 2;
+// ------------------------------------------------------------------ FP32 pair step
+// The pair step of the FP32 form, in two kernels, kGroup = 8 lanes per molecule
+// (four molecules per warp):
+//  * k_force_lists writes the molecule's per-step list: the neighbours within rcut,
+//    in the (rcut + skin) list's ascending-j order (and the wall term of a confined
+//    molecule).  Under the per-site minimum image "far" pairs, whose COM vector
+//    keeps every site-pair component clear of +-L/2, fill the list from the front,
+//    the others ("near") from the back;
+//  * k_force_pairs computes exactly those pairs, lane sub entries sub, sub + 8, ...
+//    (first the near, then the far ones), with no cutoff branch.  A lane's sums are
+//    FP32 in registers over at most 32 + 1 pairs; then the group's lanes are added
+//    in FP64 by a fixed exchange tree that leaves three of the molecule's 24 sums
+//    with each lane, and finish_group forms force and torque (A2M).
+// Which pairs a lane sums, and in what order, depends on the positions only:
+// not on the skin list's age, the tile, the batch or the launch.
+struct F32Const {
+  float Ls[3], Lf[3], hL[3];
+  double L[3];
+};
 
-template <int S, int C0>
-__device__ void force_tile_f32(const DevPtrs& d, const RepConst& c, const Tile& t, int tix, const double* L,
-                               int tile_size) {
-  __shared__ F32Const k32;
-  extern __shared__ double acc[];   // (3S + 8) x blockDim.x FP64 accumulators
-  const int B = blockDim.x;
-  const int i = threadIdx.x % tile_size, ch = threadIdx.x / tile_size;
-  const int li = t.start + i;
-  const int g = c.mol_off + li;
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < kMaxSites; k++)
-      for (int l = 0; l < kMaxSites; l++) k32.qq[k][l] = (float)c.qq[k][l];
-    for (int x = 0; x < 3; x++) {
-      k32.Ls[x] = (float)(L[x] * kFixInv);
-      k32.Lf[x] = (float)L[x];
-      k32.hL[x] = 0.5f * (float)L[x];
-      k32.L[x] = L[x];
-    }
+// Per-site minimum image (SIMG) flips a site-pair vector by a box length where
+// one of its components crosses +-L/2, so the FP32 and FP64 forms must take the
+// same image there.  For a site pair with a component within kImageTol of L/2
+// (FP32 rounding of the site vector is below ~4e-6 A) the vector is formed anew
+// with the FP64 form's arithmetic (pair_loop_f64: COM vector from the FP64 box
+// fractions, site offsets R(q) b in FP64, the image decided on their sum).
+constexpr float kImageTol = 2e-5f;
+
+__device__ __noinline__ float3 site_vector_exact(const DevPtrs& d, const PairConst& c, const double* L, int li,
+                                                 int j, int kk, int l) {
+  const int N = d.N, gi = c.mol_off + li, gj = c.mol_off + j;
+  double qi[4], qj[4], si[3], sj[3];
+  for (int x = 0; x < 4; x++) { qi[x] = d.q[x * N + gi]; qj[x] = d.q[x * N + gj]; }
+  body_to_space(qi, c.body[kk], si);
+  body_to_space(qj, c.body[l], sj);
+  float v[3];
+  for (int x = 0; x < 3; x++) {
+    double gr = (d.r[x * N + gi] - d.r[x * N + gj]) * L[x];
+    if (gr >= 0.5 * L[x]) gr -= L[x];
+    if (gr < -0.5 * L[x]) gr += L[x];
+    double rv = gr + si[x] - sj[x];
+    if (rv >= 0.5 * L[x]) rv -= L[x];
+    if (rv < -0.5 * L[x]) rv += L[x];
+    v[x] = (float)rv;
   }
-  for (int f = 0; f < 3 * S + 8; f++) acc[f * B + threadIdx.x] = 0.0;
-  __syncthreads();
-  int npairs = 0;
-  if (i < t.count) {
-    const uint16_t* nt = d.nbt + c.nbr_off + (long long)(tix - c.tile_off) * c.nbr_cap * tile_size + i;
-    const int nc = d.nt_cnt[g];
-    const int nfar = nc & 0xffff, nnear = nc >> 16;
-    npairs = nfar + nnear;
-    const int p0 = (npairs * ch) / kPairChunks, p1 = (npairs * (ch + 1)) / kPairChunks;
-    if (site_image_needed(c, L))
-      pair_loop_f32<S, C0, true>(d, c, k32, li, nt, tile_size, nfar, nnear, p0, p1, acc);
-    else
-      pair_loop_f32<S, C0, false>(d, c, k32, li, nt, tile_size, nfar, nnear, p0, p1, acc);
-  }
-  __syncthreads();
-  if (ch != 0) return;   // chunk-0 threads (whole warps) finish the molecules
-  IAcc a;
-  zero_acc(a);
-  double wall_e = 0.0;
-  if (i < t.count) {
-    auto sum = [&](int f) {
-      double v = 0.0;
-      for (int k = 0; k < kPairChunks; k++) v += acc[f * B + i + k * tile_size];
-      return v;
-    };
+  return make_float3(v[0], v[1], v[2]);
+}
+
+// Whether the per-site minimum image can change a pair of this box.
+__device__ __forceinline__ bool site_image_f32(const PairConst& c, float L0, float L1, float L2) {
+  const float reach = 2.f * (c.rc + 2.f * c.reach);
+  return L0 < reach || L1 < reach || L2 < reach;
+}
+
+// FP32 sums of one lane over its pairs of a segment.
+template <int S>
+struct F32Sums {
+  float fs[S][3], fc[3], fv[3], lj, cl;
+  __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int k = 0; k < S; k++)
-      for (int x = 0; x < 3; x++) a.fs[k][x] = sum(3 * k + x);
-    for (int x = 0; x < 3; x++) {
-      a.fc[x] = sum(3 * S + x);
-      a.vir[x] = sum(3 * S + 3 + x);
-    }
-    a.lj = sum(3 * S + 6);
-    a.clmb = sum(3 * S + 7);
-    a.npair = npairs;
-    finish_molecule<S>(d, c, g, L, a, wall_e);
+    for (int k = 0; k < S; k++) fs[k][0] = fs[k][1] = fs[k][2] = 0.f;
+    fc[0] = fc[1] = fc[2] = 0.f;
+    fv[0] = fv[1] = fv[2] = 0.f;
+    lj = cl = 0.f;
   }
-  write_part2(d, c, t, a, wall_e);
+  // the 24 sums by slot: slots 0..4 the sites' forces, 5 the switching correction,
+  // 6 the virial, 7 {LJ, Coulomb, -}
+  __device__ __forceinline__ float at(int slot, int x) const {
+    if (slot < S) return fs[slot][x];
+    if (slot == 5) return fc[x];
+    if (slot == 6) return fv[x];
+    if (slot == 7) return x == 0 ? lj : x == 1 ? cl : 0.f;
+    return 0.f;
+  }
+};
+
+// 2 / sqrt(x): the SFU's reciprocal square root y and one Newton step,
+// y (3 - x y^2), without the division by two (~0.5 ulp; three operations).
+__device__ __forceinline__ float two_rsqrt(float x) {
+  const float y = rsqrtf(x);
+  return y * fmaf(-(x * y), y, 3.f);
+}
+
+// Site charge in units of the second charged site's (the hydrogens of the water
+// models).  STD: the ratios of TIP3P {-2, 1, 1}, TIP4P {1, 1, -2} and TIP5P
+// {1, 1, -1, -1} are compile-time constants; otherwise they are read.
+template <int S, int C0, bool STD>
+__device__ __forceinline__ float charge_ratio(const PairConst& c, int k) {
+  if (!STD) return c.q[k];
+  if (S == 3) return k == 0 ? -2.f : 1.f;
+  if (S == 4) return k == 3 ? -2.f : 1.f;
+  return k >= 3 ? -1.f : 1.f;
+}
+
+// The lane's n pairs with molecule li: entries row[0], row[+-kGroup], ... (near
+// pairs, IMG, are stored backwards).  ci, si: li's fixed-point centre and site
+// offsets.  The Coulomb terms of site kk carry a factor 8 / (q_kk u^2), u the unit
+// charge, that the switch's factor takes back once per site.
+template <int S, int C0, bool STD, bool IMG>
+__device__ __forceinline__ void pair_loop_f32(const DevPtrs& d, const PairConst& c, const F32Const& k32, int li,
+                                              const int* ci, const float (*si)[3], const uint16_t* row, int n,
+                                              F32Sums<S>& a) {
+  constexpr int STRIDE = ((3 + 3 * S) + 3) / 4 * 4;
+  constexpr int NV = STRIDE / 4;
+  const uint4* base = reinterpret_cast<const uint4*>(d.pack) + c.mol_off;
+  const int N = d.N;
+  const float Ls0 = k32.Ls[0], Ls1 = k32.Ls[1], Ls2 = k32.Ls[2];
+  const float rc = c.rc, rs = c.rs, coef = c.coef;
+  const float uu = c.uu;
+  constexpr int DIR = IMG ? -kGroup : kGroup;
+  // the neighbour's record one pair ahead in registers, its index two pairs ahead
+  // (2-5 % faster than loading the record at the top of its own iteration)
+  int jcur = (n > 0) ? row[0] : 0, jnext = (n > 1) ? row[DIR] : jcur;
+  uint4 next[NV];
+#pragma unroll
+  for (int m = 0; m < NV; m++) next[m] = __ldg(base + (m * N + jcur));
+  for (int k = 0; k < n; k++) {
+    const int jthis = jcur;
+    uint32_t wj[STRIDE];
+#pragma unroll
+    for (int m = 0; m < NV; m++) {
+      wj[4 * m] = next[m].x; wj[4 * m + 1] = next[m].y; wj[4 * m + 2] = next[m].z; wj[4 * m + 3] = next[m].w;
+    }
+    jcur = jnext;
+#pragma unroll
+    for (int m = 0; m < NV; m++) next[m] = __ldg(base + (m * N + jcur));
+    row += DIR;
+    if (k + 2 < n) jnext = row[DIR];
+    const float dx = (float)wrap_diff(ci[0], (int)wj[0]) * Ls0;
+    const float dy = (float)wrap_diff(ci[1], (int)wj[1]) * Ls1;
+    const float dz = (float)wrap_diff(ci[2], (int)wj[2]) * Ls2;
+    // vector between site kk of li (already added to d) and site l of j
+    auto vec = [&](float ax, float ay, float az, int kk, int l, float& x, float& y, float& z) {
+      x = ax - __uint_as_float(wj[3 + 3 * l]);
+      y = ay - __uint_as_float(wj[3 + 3 * l + 1]);
+      z = az - __uint_as_float(wj[3 + 3 * l + 2]);
+      if (IMG) {
+        const float hL0 = k32.hL[0], hL1 = k32.hL[1], hL2 = k32.hL[2];
+        if (fabsf(fabsf(x) - hL0) < kImageTol || fabsf(fabsf(y) - hL1) < kImageTol ||
+            fabsf(fabsf(z) - hL2) < kImageTol) {
+          const float3 v = site_vector_exact(d, c, k32.L, li, jthis, kk, l);
+          x = v.x; y = v.y; z = v.z;
+        } else {
+          if (x >= hL0) x -= k32.Lf[0];
+          if (x < -hL0) x += k32.Lf[0];
+          if (y >= hL1) y -= k32.Lf[1];
+          if (y < -hL1) y += k32.Lf[1];
+          if (z >= hL2) z -= k32.Lf[2];
+          if (z < -hL2) z += k32.Lf[2];
+        }
+      }
+    };
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    const float rinv = rsqrtf(r2);
+    const float r = r2 * rinv;
+    float sw = 1.f, dsw = 0.f;
+    if (r > rs) {
+      const float r01c = r - rc, r01l = r - rs;
+      const float cc = coef * r01c * r01c;
+      sw = cc * r01c * (10.f * r01l * r01l - 5.f * r01l * r01c + r01c * r01c);
+      dsw = cc * 30.f * r01l * r01l;
+    }
+    const float swu = sw * (0.125f * uu);
+    float elj = 0.f, ecl = 0.f;
+    float fpx = 0.f, fpy = 0.f, fpz = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < S; kk++) {
+      if (kk != 0 && kk < C0) continue;
+      const float ax = dx + si[kk][0], ay = dy + si[kk][1], az = dz + si[kk][2];
+      float tx = 0.f, ty = 0.f, tz = 0.f, ek = 0.f;
+#pragma unroll
+      for (int l = 0; l < S; l++) {
+        const bool lj_pair = (kk == 0 && l == 0);
+        const bool cl_pair = (kk >= C0 && l >= C0);
+        if (!lj_pair && !cl_pair) continue;
+        float x, y, z;
+        vec(ax, ay, az, kk, l, x, y, z);
+        const float ri = two_rsqrt(x * x + y * y + z * z);   // 2 / r
+        const float p = ri * ri;                              // 4 / r^2
+        if (lj_pair) {
+          float s6 = c.sgm2q * p;
+          s6 = s6 * s6 * s6;
+          const float e4 = c.eps4 * s6;
+          elj = e4 * (s6 - 1.f);
+          const float f = 3.f * sw * (e4 * (s6 - 0.5f)) * p;
+          a.fs[0][0] = fmaf(f, x, a.fs[0][0]);
+          a.fs[0][1] = fmaf(f, y, a.fs[0][1]);
+          a.fs[0][2] = fmaf(f, z, a.fs[0][2]);
+          fpx = f * x; fpy = f * y; fpz = f * z;
+        }
+        if (cl_pair) {
+          const float e = charge_ratio<S, C0, STD>(c, l) * ri;
+          ek += e;
+          const float f = e * p;
+          tx = fmaf(f, x, tx); ty = fmaf(f, y, ty); tz = fmaf(f, z, tz);
+        }
+      }
+      if (kk >= C0) {
+        // switch, charge and unit once per site (FFMA into the sums)
+        const float qk = charge_ratio<S, C0, STD>(c, kk);
+        ecl = fmaf(qk, ek, ecl);
+        const float w = swu * qk;
+        a.fs[kk][0] = fmaf(w, tx, a.fs[kk][0]);
+        a.fs[kk][1] = fmaf(w, ty, a.fs[kk][1]);
+        a.fs[kk][2] = fmaf(w, tz, a.fs[kk][2]);
+        fpx = fmaf(w, tx, fpx); fpy = fmaf(w, ty, fpy); fpz = fmaf(w, tz, fpz);
+      }
+    }
+    ecl *= 0.5f * uu;
+    const float g = -(dsw * rinv) * (elj + ecl);
+    const float cx = dx * g, cy = dy * g, cz = dz * g;
+    a.fc[0] += cx; a.fc[1] += cy; a.fc[2] += cz;
+    a.fv[0] = fmaf(fpx + cx, dx, a.fv[0]);
+    a.fv[1] = fmaf(fpy + cy, dy, a.fv[1]);
+    a.fv[2] = fmaf(fpz + cz, dz, a.fv[2]);
+    a.lj = fmaf(sw, elj, a.lj);
+    a.cl = fmaf(sw, ecl, a.cl);
+  }
+}
+
+// Force record of molecule li: its fixed-point centre and site offsets.
+template <int S>
+__device__ __forceinline__ void load_record(const DevPtrs& d, const PairConst& c, int li, int* ci, float (*si)[3]) {
+  constexpr int NV = ((3 + 3 * S) + 3) / 4;
+  const uint4* w = reinterpret_cast<const uint4*>(d.pack) + c.mol_off + li;
+  uint32_t r[4 * NV];
+#pragma unroll
+  for (int m = 0; m < NV; m++) {
+    const uint4 u = __ldg(w + m * d.N);
+    r[4 * m] = u.x; r[4 * m + 1] = u.y; r[4 * m + 2] = u.z; r[4 * m + 3] = u.w;
+  }
+#pragma unroll
+  for (int x = 0; x < 3; x++) ci[x] = (int)r[x];
+#pragma unroll
+  for (int k = 0; k < S; k++)
+#pragma unroll
+    for (int x = 0; x < 3; x++) si[k][x] = __uint_as_float(r[3 + 3 * k + x]);
+}
+
+// The near pairs of a segment (SIMG), as a call: its image tests and their FP64
+// branch would otherwise hold registers through the far pairs' loop (with it
+// inlined the kernel spilled 200 bytes at 128 registers; it runs for a few percent
+// of the pairs of the boxes close to the minimum-image bound only).
+template <int S, int C0>
+__device__ __noinline__ void near_pairs_f32(const DevPtrs& d, const PairConst& c, const F32Const& k32, int li,
+                                            const uint16_t* row, int n, F32Sums<S>* out) {
+  int ci[3];
+  float si[S][3];
+  load_record<S>(d, c, li, ci, si);
+  F32Sums<S> a;
+  a.zero();
+  pair_loop_f32<S, C0, false, true>(d, c, k32, li, ci, si, row, n, a);
+  *out = a;
+}
+
+// One exchange step of the sums' reduction: of 2H values per lane, the lane
+// with bit `o` clear keeps the first H and gets its partner's, the other keeps
+// the last H; both add the same two numbers.
+template <int H>
+__device__ __forceinline__ void exchange_sum(double* v, int sub, int o) {
+  const bool up = (sub & o) != 0;
+#pragma unroll
+  for (int k = 0; k < H; k++) {
+    const double give = up ? v[k] : v[k + H], keep = up ? v[k + H] : v[k];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+  }
+}
+
+// Adds the group's eight lanes' sums in FP64: lane sub ends with slot sub.
+template <int S>
+__device__ __forceinline__ void reduce_sums(const F32Sums<S>& a, int sub, double* acc) {
+  double v[12];
+  const bool up = (sub & 4) != 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+      // slots k (lower half) and k + 4: exchanged in FP32, added in FP64
+      if (k >= S && k + 4 < 5) { v[3 * k + x] = 0.0; continue; }
+      const float lo = a.at(k, x), hi = a.at(k + 4, x);
+      const float give = up ? lo : hi, keep = up ? hi : lo;
+      v[3 * k + x] = (double)keep + (double)__shfl_xor_sync(0xffffffffu, give, 4);
+    }
+  exchange_sum<6>(v, sub, 2);
+  exchange_sum<3>(v, sub, 1);
+#pragma unroll
+  for (int x = 0; x < 3; x++) acc[x] += v[x];
+}
+
+// Pair forces of molecules li0 .. li0 + kWarpMol - 1 by one warp from their
+// per-step lists.  Lane sub of a molecule's group ends with slot sub of its sums in
+// acc; returns the molecule's pair count (equal on the group's lanes).
+template <int S, int C0, bool STD>
+__device__ __forceinline__ int force_warp_f32(const DevPtrs& d, const PairBlk& b, const PairConst& c,
+                                              const F32Const& k32, int li0, int nc, double* acc) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, grp = lane / kGroup, sub = lane % kGroup;
+  const int lic = min(li0 + grp, b.nmol - 1);
+  const int nfar = nc & 0xffff, nnear = nc >> 16;
+  const uint16_t* row = d.nbt + b.nbr_off + (long long)lic * b.nbr_stride + sub;
+  // FP32 sums close every 32 pairs of a lane
+  const bool segments = __any_sync(kAll, nfar + nnear > kSegPairs);
+  F32Sums<S> a;
+  a.zero();
+  for (int p0 = 0; __any_sync(kAll, p0 < nnear); p0 += kSegPairs) {
+    const int n = min(nnear - p0, kSegPairs) - sub;
+    if (n > 0)
+      near_pairs_f32<S, C0>(d, c, k32, lic, row + (c.nbr_cap - 1 - p0 - 2 * sub), (n + kGroup - 1) / kGroup, &a);
+    if (segments) {
+      reduce_sums<S>(a, sub, acc);
+      a.zero();
+    }
+  }
+  int ci[3];
+  float si[S][3];
+  load_record<S>(d, c, lic, ci, si);
+  int p0 = 0;
+  do {
+    const int n = min(nfar - p0, kSegPairs) - sub;
+    pair_loop_f32<S, C0, STD, false>(d, c, k32, lic, ci, si, row + p0, (n + kGroup - 1) / kGroup, a);
+    __syncwarp();
+    reduce_sums<S>(a, sub, acc);
+    a.zero();
+    p0 += kSegPairs;
+  } while (segments && __any_sync(kAll, p0 < nfar));
+  return nfar + nnear;
+}
+
+// Wall and A2M (FP64) for molecule li of a group of kGroup lanes that hold its
+// sums by slot (F32Sums::at), in q4 one component each of q and in wf of the wall
+// term {force, energy} (lanes 0..3; both loaded before the pairs): writes d.f and
+// d.n, one component per lane.  On return lane 5 of the group holds {wall energy,
+// 0, 0}, lane 6 the virial and lane 7 {LJ, Coulomb, pairs} in acc.
+template <int S>
+__device__ __forceinline__ void finish_group(const DevPtrs& d, const PairConst& c, int li, int sub,
+                                             double q4, double wf, double* acc, int npairs) {
+  const int N = d.N, g = c.mol_off + li;
+  const bool valid = li < c.nmol;
+  double q[4];
+#pragma unroll
+  for (int x = 0; x < 4; x++) q[x] = __shfl_sync(0xffffffffu, q4, x, kGroup);
+  const double wall_e = __shfl_sync(0xffffffffu, wf, 3, kGroup);
+#pragma unroll
+  for (int x = 0; x < 3; x++) {
+    const double f = __shfl_sync(0xffffffffu, wf, x, kGroup);
+    if (sub == 0) acc[x] += f;
+  }
+  // A2M: molecular force and body torque (src/molecules.cxx:447-475); lane k has
+  // site k, lane 5 the switching correction
+  double v[8];
+  const bool force = sub < S || sub == 5;
+#pragma unroll
+  for (int x = 0; x < 3; x++) v[x] = force ? acc[x] : 0.0;
+  v[3] = v[4] = v[5] = v[6] = v[7] = 0.0;
+  if (sub < S) {
+    double fb[3];
+    space_to_body(q, acc, fb);
+    const double* b = c.body[sub];
+    v[3] = b[0] * fb[0] + b[1] * fb[1] + b[2] * fb[2];
+    v[4] = b[1] * fb[2] - b[2] * fb[1];
+    v[5] = b[2] * fb[0] - b[0] * fb[2];
+    v[6] = b[0] * fb[1] - b[1] * fb[0];
+  }
+  exchange_sum<4>(v, sub, 4);
+  exchange_sum<2>(v, sub, 2);
+  exchange_sum<1>(v, sub, 1);
+  if (valid && sub < 3) d.f[sub * N + g] = v[0];
+  if (valid && sub >= 3 && sub < 7) d.n[(sub - 3) * N + g] = v[0];
+  if (sub == 5) { acc[0] = wall_e; acc[1] = acc[2] = 0.0; }
+  if (sub == 7) acc[2] = (double)npairs;
 }
 
 // FP64 form: one launch per step after the replica head (list rebuild when
@@ -1296,7 +1368,7 @@ __global__ void __launch_bounds__(128, 1) k_force_f64(DevPtrs d, const RepState*
   extern __shared__ uint32_t bm[];
   __shared__ double Ls[3];
   __shared__ int rb;
-  const int tix = d.order ? d.order[blockIdx.x] : d.tile0 + blockIdx.x;   // costliest tiles first
+  const int tix = d.order ? d.order[blockIdx.x] : (int)blockIdx.x;   // costliest tiles first
   const Tile t = d.tiles[tix];
   const RepConst& c = d.rc[t.rep];
   if (threadIdx.x < 3) Ls[threadIdx.x] = X[t.rep].L[threadIdx.x];
@@ -1311,62 +1383,205 @@ __global__ void __launch_bounds__(128, 1) k_force_f64(DevPtrs d, const RepState*
     force_tile_f64<5, 1>(d, c, t, tix, L, rb != 0, tile_size, bm, d.bm_win);
 }
 
-// FP32 form, first launch after the replica head: skin-list rebuild when due,
-// pass 1; kListLanes x tile threads, the lanes of a molecule adjacent in a
-// warp.  Light on registers, so many warps hide the gathered loads.
-__global__ void __launch_bounds__(256, 4) k_force_lists(DevPtrs d, const RepState* __restrict__ X, int tile_size) {
-  step_kernel_entry();
-  extern __shared__ uint32_t bm[];
-  __shared__ double Ls[3];
-  __shared__ int rb;
-  const int tix = d.order ? d.order[blockIdx.x] : d.tile0 + blockIdx.x;
-  const Tile t = d.tiles[tix];
-  const RepConst& c = d.rc[t.rep];
-  if (threadIdx.x < 3) Ls[threadIdx.x] = X[t.rep].L[threadIdx.x];
-  if (threadIdx.x == 0) rb = d.cgrid[t.rep].rebuild;
-  __syncthreads();
-  const double L[3] = {Ls[0], Ls[1], Ls[2]};
-  const int i = threadIdx.x / kListLanes, sub = threadIdx.x % kListLanes;
-  const int li = t.start + i;
-  const bool valid = i < t.count;
-  uint16_t* nb = d.nbr + c.nbr_off + (long long)(tix - c.tile_off) * c.nbr_cap * tile_size + i;
-  int cnt;
-  if (rb) {
-    cnt = build_lists_f32(d, c, t, L, nb, tile_size, bm, d.bm_win);
-    if (valid && sub == 0) {
-      const int* w = reinterpret_cast<const int*>(d.pack) + c.pack_off + (long long)li * c.pack_stride;
-      d.ref_com[c.mol_off + li] = make_int4(w[0], w[1], w[2], 0);
-    }
-    if (threadIdx.x == 0)
-      for (int x = 0; x < 3; x++) d.Lbuild[3 * tix + x] = L[x];
-    __syncthreads();   // the group's list entries, written by all its lanes, are read below
-  } else {
-    cnt = valid ? d.nbr_cnt[c.mol_off + li] : 0;
-  }
-  if (!valid) cnt = 0;
-  uint16_t* nt = d.nbt + (nb - d.nbr);
-  if (site_image_needed(c, L)) tight_lists_f32<true>(d, c, li, valid, sub, L, nb, nt, cnt, tile_size);
-  else tight_lists_f32<false>(d, c, li, valid, sub, L, nb, nt, cnt, tile_size);
+// A lane's eight skin-list entries from k on, read 16 bytes at a time.  Also past
+// the list's end (the array is padded by kListPad entries); the caller masks those.
+__device__ __forceinline__ uint4 list_words(const uint16_t* nb, int k) {
+  return *reinterpret_cast<const uint4*>(nb + k);
 }
 
-// FP32 form, second launch of a step: pair forces, wall, A2M (box from X, which
-// k_force_lists has updated); kPairChunks x tile threads.
-__global__ void __launch_bounds__(128, 3) k_force_pairs(DevPtrs d, const RepState* __restrict__ X,
-                                                        int tile_size) {
+// Per-step list of molecule li by its group of kGroup lanes (the FP32 pair step,
+// above): 64 skin-list entries at a time, eight consecutive ones per lane (one
+// 16-byte load two rounds ahead, then eight centre loads in flight); a prefix over
+// the group places the kept ones.  w0, w1: the lane's entries of the first two
+// rounds; me: li's centre.
+__device__ __forceinline__ void step_list(const DevPtrs& d, const PairBlk& b, const PairConst& c, int li, int cnt,
+                                          const int4 me, uint4 w0, uint4 w1, const double* L) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int sub = threadIdx.x % kGroup;
+  const int lic = min(li, b.nmol - 1);
+  const int4* com = d.com + b.mol_off;
+  const long long off = b.nbr_off + (long long)lic * b.nbr_stride;
+  const uint16_t* nb = d.nbr + off;
+  uint16_t* row = d.nbt + off;
+  const float L0 = (float)L[0], L1 = (float)L[1], L2 = (float)L[2];
+  const float Ls0 = (float)(L[0] * kFixInv), Ls1 = (float)(L[1] * kFixInv), Ls2 = (float)(L[2] * kFixInv);
+  const float rc2 = c.rc2;
+  const bool simg = site_image_f32(c, L0, L1, L2);
+  // far bound: |d_x| below it keeps every site-pair component below L/2 - kImageTol
+  const float m = 2.f * c.reach + kImageTol + 1e-3f;
+  const float bnd0 = simg ? 0.5f * L0 - m : 1e30f, bnd1 = simg ? 0.5f * L1 - m : 1e30f,
+              bnd2 = simg ? 0.5f * L2 - m : 1e30f;
+  const int back = c.nbr_cap - 1;
+  int nfar = 0, nnear = 0;
+  for (int k = 8 * sub; __any_sync(kAll, k - 8 * sub < cnt); k += 8 * kGroup) {
+    const uint4 cur = w0;
+    w0 = w1;
+    if (k + 16 * kGroup < cnt) w1 = list_words(nb, k + 16 * kGroup);
+    int j[8];
+    int4 u[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const unsigned w = (e >> 1) == 0 ? cur.x : (e >> 1) == 1 ? cur.y : (e >> 1) == 2 ? cur.z : cur.w;
+      j[e] = (k + e < cnt) ? (int)((e & 1) ? (w >> 16) : (w & 0xffffu)) : 0;
+      u[e] = __ldg(com + j[e]);
+    }
+    unsigned in = 0u, nr = 0u;   // within rcut; of these, near
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const float dx = (float)wrap_diff(me.x, u[e].x) * Ls0, dy = (float)wrap_diff(me.y, u[e].y) * Ls1,
+                  dz = (float)wrap_diff(me.z, u[e].z) * Ls2;
+      if (k + e < cnt && dx * dx + dy * dy + dz * dz <= rc2) in |= 1u << e;
+      if (fabsf(dx) >= bnd0 || fabsf(dy) >= bnd1 || fabsf(dz) >= bnd2) nr |= 1u << e;
+    }
+    nr &= in;
+    const unsigned fr = in & ~nr;
+    const int n = __popc(fr) | (__popc(nr) << 16);
+    int incl = n;   // inclusive prefix over the group's lanes
+#pragma unroll
+    for (int o = 1; o < kGroup; o <<= 1) {
+      const int y = __shfl_up_sync(kAll, incl, o, kGroup);
+      if (sub >= o) incl += y;
+    }
+    const int total = __shfl_sync(kAll, incl, kGroup - 1, kGroup);
+    uint16_t* wf = row + nfar + ((incl - n) & 0xffff);
+#pragma unroll
+    for (int e = 0; e < 8; e++)
+      if (fr >> e & 1u) *wf++ = (uint16_t)j[e];
+    if (simg) {
+      uint16_t* wn = row + back - nnear - ((incl - n) >> 16);
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        if (nr >> e & 1u) *wn-- = (uint16_t)j[e];
+    }
+    nfar += total & 0xffff;
+    nnear += total >> 16;
+  }
+  if (sub == 0 && li < b.nmol) d.nt_cnt[b.mol_off + li] = nfar | (nnear << 16);
+}
+
+// FP32 form, first launch after the replica head, kPart2Mol molecules per block:
+// their skin lists where the replica's are due, their per-step lists and, where
+// confined, their wall terms.  A kernel of its own, light on registers: its many
+// warps hide the gathered loads' latency, which the pair kernel's four per
+// scheduler do not (the gather inside the pair kernel took 12 000 of a warp's
+// 43 000 cycles on 256 replicas, 111 432 molecules).  It is bound by the latency of
+// its loads, so all that need only the block's descriptor are issued together.
+__global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_lists(DevPtrs d, const RepState* __restrict__ X) {
   step_kernel_entry();
-  __shared__ double Ls[3];
-  const int tix = d.order ? d.order[blockIdx.x] : d.tile0 + blockIdx.x;
-  const Tile t = d.tiles[tix];
-  const RepConst& c = d.rc[t.rep];
-  if (threadIdx.x < 3) Ls[threadIdx.x] = X[t.rep].L[threadIdx.x];
+  extern __shared__ uint32_t bm[];
+  __shared__ PairConst c;
+  const PairBlk b = d.pblk[blockIdx.x];
+  const int li0 = b.li0 + (threadIdx.x >> 5) * kWarpMol;
+  const int sub = threadIdx.x % kGroup, li = li0 + (threadIdx.x & 31) / kGroup, lic = min(li, b.nmol - 1);
+  const int g = b.mol_off + lic;
+  const uint16_t* nb = d.nbr + b.nbr_off + (long long)lic * b.nbr_stride;
+  int cnt = (li < b.nmol) ? d.nbr_cnt[g] : 0;
+  uint4 w0 = list_words(nb, 8 * sub), w1 = list_words(nb, 8 * sub + 8 * kGroup);
+  const int4 me = d.com[g];
+  double qr[7];
+  if (b.confined) {
+    for (int x = 0; x < 4; x++) qr[x] = d.q[x * d.N + g];
+    for (int x = 0; x < 3; x++) qr[4 + x] = d.r[x * d.N + g];
+  }
+  const RepState& st = X[b.rep];
+  const double L[3] = {st.L[0], st.L[1], st.L[2]};
+  const int rebuild = d.cgrid[b.rep].rebuild;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(d.pc + b.rep);
+  for (int k = threadIdx.x; k < (int)(sizeof(PairConst) / 4); k += 32 * kPairWarps)
+    reinterpret_cast<uint32_t*>(&c)[k] = src[k];
   __syncthreads();
-  const double L[3] = {Ls[0], Ls[1], Ls[2]};
-  if (c.nsite == 3)
-    force_tile_f32<3, 0>(d, c, t, tix, L, tile_size);
-  else if (c.nsite == 4)
-    force_tile_f32<4, 1>(d, c, t, tix, L, tile_size);
+  if (li0 >= b.nmol) return;
+  if (rebuild) {
+    const RepConst& rc = d.rc[b.rep];
+    build_lists_f32(d, rc, b.rep, li0, L, bm, d.bm_win);
+    if (sub == 0 && li < b.nmol) d.ref_com[g] = make_int4(me.x, me.y, me.z, 0);
+    if (threadIdx.x < 3 && b.li0 % b.tile == 0)
+      d.Lbuild[3 * (rc.tile_off + b.li0 / b.tile) + threadIdx.x] = L[threadIdx.x];
+    __syncwarp();   // the lists, written by all lanes, are read below
+    cnt = (li < b.nmol) ? d.nbr_cnt[g] : 0;
+    w0 = list_words(nb, 8 * sub);
+    w1 = list_words(nb, 8 * sub + 8 * kGroup);
+  }
+  step_list(d, b, c, li, cnt, me, w0, w1, L);
+  if (b.confined && sub == 0 && li < b.nmol) {
+    double f[3] = {0.0, 0.0, 0.0};
+    const double e = wall_site(d, d.rc[b.rep], qr, qr + 4, L, f);
+    double2* w = reinterpret_cast<double2*>(d.wallf + 4 * (long long)g);
+    w[0] = make_double2(f[0], f[1]);
+    w[1] = make_double2(f[2], e);
+  }
+}
+
+// FP32 form, second launch of a step: pair forces, wall, A2M of kPart2Mol
+// molecules per block, and their partial sums.
+template <int S, int C0, bool STD>
+__device__ void force_block_f32(const DevPtrs& d, const PairBlk& b, const PairConst& c, const F32Const& k32, int nc,
+                                double q4, double wf, double (*wsum)[8]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % kGroup;
+  const int lw = b.li0 + warp * kWarpMol;
+  double acc[3] = {0.0, 0.0, 0.0};
+  const int npairs = force_warp_f32<S, C0, STD>(d, b, c, k32, lw, nc, acc);
+  finish_group<S>(d, c, lw + lane / kGroup, sub, q4, wf, acc, npairs);
+#pragma unroll
+  for (int x = 0; x < 3; x++)
+    for (int o = kGroup; o < 32; o <<= 1) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
+  if (lane == 5) wsum[warp][0] = acc[0];
+  if (lane == 6)
+    for (int x = 0; x < 3; x++) wsum[warp][1 + x] = acc[x];
+  if (lane == 7)
+    for (int x = 0; x < 3; x++) wsum[warp][4 + x] = acc[x];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s[7];
+    for (int k = 0; k < 7; k++) {
+      s[k] = wsum[0][k];
+      for (int w = 1; w < kPairWarps; w++) s[k] += wsum[w][k];
+    }
+    Part2 p;
+    p.wall = s[0];
+    p.vir[0] = s[1]; p.vir[1] = s[2]; p.vir[2] = s[3];
+    p.lj = s[4]; p.clmb = s[5];
+    p.npairs = (long long)llrint(s[6]);
+    p.pad = 0.0;
+    d.part2[c.part2_off + b.li0 / kPart2Mol] = p;
+  }
+}
+
+// S: the sites of every replica of the launch (0: mixed models, chosen per
+// block); STD: every replica has the charge ratios of charge_ratio.
+template <int S, bool STD>
+__global__ void __launch_bounds__(32 * kPairWarps, 64 / kPart2Mol) k_force_pairs(DevPtrs d, const RepState* __restrict__ X) {
+  step_kernel_entry();
+  __shared__ PairConst c;
+  __shared__ F32Const k32;
+  __shared__ double wsum[kPairWarps][8];
+  const PairBlk b = d.pblk[blockIdx.x];
+  // loads that need only the block's descriptor
+  const int sub = threadIdx.x % kGroup, li = b.li0 + threadIdx.x / kGroup, g = b.mol_off + min(li, b.nmol - 1);
+  const int nc = (li < b.nmol) ? d.nt_cnt[g] : 0;
+  double q4 = 0.0, wf = 0.0;   // one component each of q and of the wall term
+  if (sub < 4 && li < b.nmol) {
+    q4 = d.q[sub * d.N + g];
+    if (b.confined) wf = d.wallf[4 * (long long)g + sub];
+  }
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(d.pc + b.rep);
+  for (int k = threadIdx.x; k < (int)(sizeof(PairConst) / 4); k += 32 * kPairWarps)
+    reinterpret_cast<uint32_t*>(&c)[k] = src[k];
+  if (threadIdx.x < 3) {
+    const int x = threadIdx.x;
+    const double L = X[b.rep].L[x];
+    k32.Ls[x] = (float)(L * kFixInv);
+    k32.Lf[x] = (float)L;
+    k32.hL[x] = 0.5f * (float)L;
+    k32.L[x] = L;
+  }
+  __syncthreads();
+  if (S == 3 || (S == 0 && c.nsite == 3))
+    force_block_f32<3, 0, STD>(d, b, c, k32, nc, q4, wf, wsum);
+  else if (S == 4 || (S == 0 && c.nsite == 4))
+    force_block_f32<4, 1, STD>(d, b, c, k32, nc, q4, wf, wsum);
   else
-    force_tile_f32<5, 1>(d, c, t, tix, L, tile_size);
+    force_block_f32<5, 1, STD>(d, b, c, k32, nc, q4, wf, wsum);
 }
 
 // ------------------------------------------------------------------ per-replica kernels
@@ -1449,12 +1664,12 @@ __global__ void __launch_bounds__(kRepThreads) k_replica_end(DevPtrs d, RepState
   const int rep = blockIdx.x;
   const RepConst& c = d.rc[rep];
   P2Sum e;
-  if (threadIdx.x < 32) e = reduce_part2(d, c);
+  if (threadIdx.x < 32) e = reduce_part2(d, c.part2_off, c.npart2);
   if (threadIdx.x == 0) {
     RepState s = X[rep];
-    for (int x = 0; x < 3; x++) cv[x] = s.L[x] * s.s * c.dthalf;
+    for (int x = 0; x < 3; x++) cv[x] = s.L[x] * s.s * c.dthalf * c.im;
     cv[3] = 2.0 * s.s * c.dthalf;
-    d5_scalar(c, s, e.lj + e.clmb + e.wall, e.vir);
+    d5_apply(s, d5_terms(c, s, e.lj + e.clmb + e.wall, e.vir));
     d6(c, s);
     st = s;
   }
@@ -1465,7 +1680,7 @@ __global__ void __launch_bounds__(kRepThreads) k_replica_end(DevPtrs d, RepState
     double v[3], p[4], q[4], f[3], n[4];
     for (int x = 0; x < 3; x++) { v[x] = d.v[x * N + g]; f[x] = d.f[x * N + g]; }
     for (int x = 0; x < 4; x++) { q[x] = d.q[x * N + g]; p[x] = d.p[x * N + g]; n[x] = d.n[x * N + g]; }
-    kick(v, p, q, f, n, cv, cv[3], c.mass);
+    kick(v, p, q, f, n, cv, cv[3]);
     for (int x = 0; x < 3; x++) d.v[x * N + g] = v[x];
     for (int x = 0; x < 4; x++) d.p[x * N + g] = p[x];
   }
@@ -1491,7 +1706,7 @@ __global__ void __launch_bounds__(kRepThreads) k_replica_props(DevPtrs d, RepSta
   kinetic_sums(d, c, st.s, acc);
   block_sum<4>(acc, red);
   P2Sum e;
-  if (threadIdx.x < 32) e = reduce_part2(d, c);
+  if (threadIdx.x < 32) e = reduce_part2(d, c.part2_off, c.npart2);
   if (threadIdx.x == 0) {
     st.gkT = 6.0 * (double)c.nmol * st.T;
     double* avg = d.avg + (long long)rep * kNumAvg;
@@ -1603,7 +1818,7 @@ __global__ void __launch_bounds__(kRepThreads) k_replica_start(DevPtrs d, RepSta
   kinetic_sums(d, c, st.s, kacc);
   block_sum<4>(kacc, red);
   P2Sum e;
-  if (threadIdx.x < 32) e = reduce_part2(d, c);
+  if (threadIdx.x < 32) e = reduce_part2(d, c.part2_off, c.npart2);
   if (threadIdx.x == 0) {
     RepState s = st;
     s.P = Pn;
@@ -1685,7 +1900,7 @@ __global__ void __launch_bounds__(kRepThreads) k_replica_rescale(DevPtrs d, RepS
   kinetic_sums(d, c, st.s, k);
   block_sum<4>(k, red);
   P2Sum e;
-  if (threadIdx.x < 32) e = reduce_part2(d, c);
+  if (threadIdx.x < 32) e = reduce_part2(d, c.part2_off, c.npart2);
   if (threadIdx.x == 0) {
     RepState s = st;
     s.gkT = 6.0 * (double)c.nmol * s.T;
@@ -1936,14 +2151,17 @@ __global__ void k_noalloc_load(DevPtrs d, const NoAllocSetup setup, RepState* __
     for (int x = 0; x < 4; x++) q[x] = q_aos[4 * li + x];
     for (int x = 0; x < 3; x++) d.r[x * d.N + g] = r[x];
     for (int x = 0; x < 4; x++) d.q[x * d.N + g] = q[x];
-    write_pack(d, c, kF32, li, r, q);
+    const int fx[3] = {fix_coord(r[0]), fix_coord(r[1]), fix_coord(r[2])};
+    write_pack(d, c, kF32, li, r, q, fx);
   }
   if (i == 0) {
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     d.Lbuild[3 * blockIdx.x] = nan;
     if (blockIdx.x == 0) {
       *const_cast<RepConst*>(d.rc) = setup.c;
+      *const_cast<PairConst*>(d.pc) = setup.pc;
       for (int k = 0; k < d.ntiles; k++) const_cast<Tile*>(d.tiles)[k] = setup.tiles[k];
+      for (int k = 0; k < d.npblk; k++) const_cast<PairBlk*>(d.pblk)[k] = pair_blk(setup.c, 0, k * kPart2Mol, blockDim.x);
       *X = setup.rs;
       *d.err = 0;
       d.status[0] = 0;
@@ -1962,10 +2180,10 @@ __global__ void k_noalloc_store(DevPtrs d, double* __restrict__ f_aos, double* _
     for (int x = 0; x < 4; x++) n_aos[4 * li + x] = d.n[x * d.N + g];
   }
   P2Sum e;
-  if (threadIdx.x < 32) e = reduce_part2(d, c);
+  if (threadIdx.x < 32) e = reduce_part2(d, c.part2_off, c.npart2);
   if (threadIdx.x == 0) {
     long long np = 0;
-    for (int t = c.warp_off; t < c.warp_off + c.nwarp; t++) np += d.part2[t].npairs;
+    for (int t = c.part2_off; t < c.part2_off + c.npart2; t++) np += d.part2[t].npairs;
     out[0] = e.lj; out[1] = e.clmb; out[2] = e.wall;
     out[3] = e.vir[0]; out[4] = e.vir[1]; out[5] = e.vir[2];
     out[6] = (double)(np / 2);
@@ -2084,31 +2302,23 @@ static void launch_step_kernel(bool pdl, void (*k)(KArgs...), unsigned grid, uns
 void launch_integrate_prec(const DevPtrs& d, const RepState* X, RepState* Y, bool mid, int tile,
                            int prec, cudaStream_t s) {
   const bool pdl = d.ntiles <= sm_count();
-  if (mid)
-    launch_step_kernel(pdl, k_integrate<true>, d.ntiles, tile, 0, s, d, X, Y, prec);
-  else
-    launch_step_kernel(pdl, k_integrate<false>, d.ntiles, tile, 0, s, d, X, Y, prec);
+  // the chain's own warp where every block of the launch is resident with it
+  const bool chain = (long long)d.ntiles * (tile + 32) <= (long long)sm_count() * 3 * 160;
+  void (*k)(DevPtrs, const RepState*, RepState*, int) =
+      chain ? (mid ? k_integrate<true, true> : k_integrate<false, true>)
+            : (mid ? k_integrate<true, false> : k_integrate<false, false>);
+  launch_step_kernel(pdl, k, d.ntiles, tile + (chain ? 32 : 0), 0, s, d, X, Y, prec);
 }
-int max_force_tile(int prec) { return prec == kF32 ? 128 / kPairChunks : 128; }
+int max_force_tile(int prec) { return prec == kF32 ? 64 : 128; }
 
-size_t force_smem_bytes(int tile) { return (size_t)(3 * kMaxSites + 8) * tile * sizeof(double); }
-
-// Bitmap of the list rebuild: one row of (win | 1) words per thread.
-size_t bitmap_smem_bytes(int tile, int win) { return (size_t)tile * (size_t)(win | 1) * sizeof(uint32_t); }
+// Bitmap of the list rebuild: one row of (win | 1) words per molecule of a block.
+size_t bitmap_smem_bytes(int mols, int win) { return (size_t)mols * (size_t)(win | 1) * sizeof(uint32_t); }
 
 int bitmap_window(int max_nmol) { return std::min((max_nmol + 31) / 32, kBitmapMaxWords); }
 
 cudaError_t force_kernel_setup() {
-  // FP32 form: dynamic shared memory = the per-thread FP64 accumulators of a tile
-  // of up to 128 molecules (23.5 KB, under the default limit; set explicitly so
-  // that a larger tile or more accumulators only change force_smem_bytes); the
-  // list kernels' rebuild bitmaps (up to 128 rows of kBitmapMaxWords + 1 words)
-  cudaError_t e = cudaFuncSetAttribute(k_force_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)force_smem_bytes(128));
-  if (e != cudaSuccess) return e;
+  // rebuild bitmaps of the FP64 form's blocks: up to 128 rows of kBitmapMaxWords + 1 words
   const int bms = (int)bitmap_smem_bytes(128, kBitmapMaxWords);
-  e = cudaFuncSetAttribute(k_force_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, bms);
-  if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(k_force_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, bms);
 }
 
@@ -2121,15 +2331,25 @@ static void launch_force_impl(const DevPtrs& d, const RepState* Yin, RepState* X
   if (force_only) launch_step_kernel(pdl, k_replica_head<true>, d.nrep_l, kRepThreads, 0, s, d, Yin, Xout);
   else launch_step_kernel(pdl, k_replica_head<false>, d.nrep_l, kRepThreads, 0, s, d, Yin, Xout);
   if (e_head) cudaEventRecord(e_head, s);
-  const size_t bms = bitmap_smem_bytes(tile, d.bm_win);
   if (prec == kF32) {
-    launch_step_kernel(pdl, k_force_lists, d.ntiles, kListLanes * tile, bms, s, d, Xc, tile);
+    launch_step_kernel(pdl, k_force_lists, d.npblk, 32 * kPairWarps, bitmap_smem_bytes(kPart2Mol, d.bm_win), s, d,
+                       Xc);
     if (e_lists) cudaEventRecord(e_lists, s);
-    launch_step_kernel(pdl, k_force_pairs, d.ntiles, kPairChunks * tile, force_smem_bytes(kPairChunks * tile), s,
-                       d, Xc, tile);
+    void (*pairs)(DevPtrs, const RepState*);
+    switch (d.model_l) {
+      case 3: pairs = k_force_pairs<3, false>; break;
+      case 4: pairs = k_force_pairs<4, false>; break;
+      case 5: pairs = k_force_pairs<5, false>; break;
+      case 3 + kStdCharges: pairs = k_force_pairs<3, true>; break;
+      case 4 + kStdCharges: pairs = k_force_pairs<4, true>; break;
+      case 5 + kStdCharges: pairs = k_force_pairs<5, true>; break;
+      case kStdCharges: pairs = k_force_pairs<0, true>; break;
+      default: pairs = k_force_pairs<0, false>;
+    }
+    launch_step_kernel(pdl, pairs, d.npblk, 32 * kPairWarps, 0, s, d, Xc);
   } else {
     if (e_lists) cudaEventRecord(e_lists, s);
-    launch_step_kernel(pdl, k_force_f64, d.ntiles, tile, bms, s, d, Xc, tile);
+    launch_step_kernel(pdl, k_force_f64, d.ntiles, tile, bitmap_smem_bytes(tile, d.bm_win), s, d, Xc, tile);
   }
 }
 

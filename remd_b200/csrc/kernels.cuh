@@ -10,10 +10,10 @@
 //                   of mass + rotated site offsets) and the partial sums PsPv needs;
 //   k_replica_head  per replica: PsPv + D4 (scalar chain), the neighbour-list
 //                   decision and, when a rebuild is due, the cell lists;
-//   k_force_lists   per tile (FP32, four lanes per molecule): the list rebuild
-//                   when due, then the per-step list of the pairs within rcut;
-//   k_force_pairs   per tile (FP32): the switched LJ + Coulomb pair loop, the
-//                   wall, and the site -> molecule torque (A2M);
+//   k_force_lists   FP32, eight lanes per molecule: the list rebuild when due, then
+//                   the per-step list of the pairs within rcut, and the wall terms;
+//   k_force_pairs   FP32, eight lanes per molecule: the switched LJ + Coulomb pair
+//                   loop and the site -> molecule torque (A2M);
 //   k_force_f64     per tile (FP64 form): rebuild, pair loop, wall, A2M.
 //
 // An interval is k_replica_start (exchange tail), interval x (step chain),
@@ -30,7 +30,7 @@ enum Prec : int { kF32 = 0, kF64 = 1 };
 void launch_pack(const DevPtrs& d, int prec, int tile, cudaStream_t s);
 void launch_integrate_prec(const DevPtrs& d, const RepState* X, RepState* Y, bool mid, int tile,
                            int prec, cudaStream_t s);
-// Largest force tile (molecules per block) of a precision: FP32 blocks hold two threads per molecule.
+// Largest tile (molecules per integrate block; FP64 form: per force block) of a precision.
 int max_force_tile(int prec);
 // Kernel attributes the force launches need (call once per device before launching).
 cudaError_t force_kernel_setup();
@@ -54,11 +54,15 @@ void launch_exchange_k(const DevPtrs& d, const int* grid, const int* rep_off, co
 void launch_histogram(const DevPtrs& d, const HistEns* he, const int* rep_off, const int* index,
                       cudaStream_t s);
 int pack_stride(int nsite, int prec);
+// The FP32 pair step's constants of a replica, and the kStdCharges / nsite code of its model.
+PairConst pair_const(const RepConst& c);
+int pair_model(const RepConst& c);
 // Set-up of one remd_force_snapshot_noalloc call, passed by value to its load
 // kernel (kernel parameters, so no host staging buffer has to outlive the call).
 constexpr int kNoAllocMaxTiles = 32;
 struct NoAllocSetup {
   RepConst c;
+  PairConst pc;
   RepState rs;
   Tile tiles[kNoAllocMaxTiles];
 };

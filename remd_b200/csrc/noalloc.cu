@@ -38,7 +38,8 @@ constexpr double kNoAllocSkin = 1.0;
 constexpr size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 // scratch layout (byte offsets)
 constexpr size_t kOffRc = 0;
-constexpr size_t kOffTiles = kOffRc + al(sizeof(RepConst));
+constexpr size_t kOffPairC = kOffRc + al(sizeof(RepConst));
+constexpr size_t kOffTiles = kOffPairC + al(sizeof(PairConst));
 constexpr size_t kOffState = kOffTiles + al(sizeof(Tile) * kNoAllocMaxTiles);
 constexpr size_t kOffR = kOffState + al(sizeof(RepState));
 constexpr size_t kOffQ = kOffR + al(8 * 3 * kNoAllocMaxMol);
@@ -48,12 +49,13 @@ constexpr size_t kOffPack = kOffN + al(8 * 4 * kNoAllocMaxMol);
 constexpr size_t kOffRef = kOffPack + al(4 * 20 * kNoAllocMaxMol);
 constexpr size_t kOffLb = kOffRef + al(sizeof(int4) * kNoAllocMaxMol);
 constexpr size_t kOffNbr = kOffLb + al(8 * 3 * kNoAllocMaxTiles);
-constexpr size_t kOffNbt = kOffNbr + al(2 * (size_t)kNoAllocMaxNbr * kNoAllocTile * kNoAllocMaxTiles);
-constexpr size_t kOffNtc = kOffNbt + al(2 * (size_t)kNoAllocMaxNbr * kNoAllocTile * kNoAllocMaxTiles);
-constexpr size_t kOffCom = kOffNtc + al(4 * kNoAllocMaxMol);
-constexpr size_t kOffCnt = kOffCom + al(sizeof(int4) * kNoAllocMaxMol);
+constexpr size_t kOffPblk = kOffNbr + al(2 * ((size_t)kNoAllocMaxNbr * kNoAllocMaxMol + kListPad));
+constexpr size_t kOffNbt = kOffPblk + al(sizeof(PairBlk) * (kNoAllocMaxMol / kPart2Mol));
+constexpr size_t kOffNtc = kOffNbt + al(2 * (size_t)kNoAllocMaxNbr * kNoAllocMaxMol);
+constexpr size_t kOffWallf = kOffNtc + al(4 * kNoAllocMaxMol);
+constexpr size_t kOffCnt = kOffWallf + al(32 * kNoAllocMaxMol);
 constexpr size_t kOffPart = kOffCnt + al(4 * kNoAllocMaxMol);
-constexpr size_t kOffErr = kOffPart + al(sizeof(Part2) * (kNoAllocMaxMol / 32));
+constexpr size_t kOffErr = kOffPart + al(sizeof(Part2) * (kNoAllocMaxMol / kPart2Mol));
 constexpr size_t kOffGrid = kOffErr + al(16);
 constexpr size_t kOffCellStart = kOffGrid + al(sizeof(CellGrid));
 constexpr size_t kOffCellMol = kOffCellStart + al(4 * (size_t)(kMaxCells + 1));
@@ -158,9 +160,12 @@ extern "C" remd_status remd_force_snapshot_noalloc(const remd_system_desc* s, co
   c.coef_sw = 1.0 / (rlc * rlc * rlc * rlc * rlc);
   c.skin = kNoAllocSkin;
   c.nbr_cap = cap;
+  c.nbr_stride = (cap + 7) / 8 * 8;
   c.ntile = (s->nmol + kNoAllocTile - 1) / kNoAllocTile;
   c.warp_off = 0;
   c.nwarp = (s->nmol + 31) / 32;
+  c.part2_off = 0;
+  c.npart2 = (s->nmol + kPart2Mol - 1) / kPart2Mol;
   c.pack_stride = pack_stride(ns, kF32);
   const double wl = s->wall_length * 1e-10 / unit_length();
   c.wall_dr = (s->confined == 2) ? 0.5 * (wl / (double)s->nfwall) : wl / (double)(s->nfwall > 0 ? s->nfwall : 1);
@@ -172,6 +177,7 @@ extern "C" remd_status remd_force_snapshot_noalloc(const remd_system_desc* s, co
   }
   for (int k = 0; k < ns; k++)
     for (int l = 0; l < ns; l++) c.qq[k][l] = qr[k] * qr[l];
+  for (int k = 0; k < ns; k++) c.qr[k] = qr[k];
   for (int k = 0; k < ns; k++)
     c.site_reach = std::fmax(c.site_reach, std::sqrt(c.body[k][0] * c.body[k][0] + c.body[k][1] * c.body[k][1] +
                                                      c.body[k][2] * c.body[k][2]));
@@ -182,10 +188,15 @@ extern "C" remd_status remd_force_snapshot_noalloc(const remd_system_desc* s, co
   NoAllocSetup setup;
   std::memset(&setup, 0, sizeof(setup));
   setup.c = c;
+  setup.pc = pair_const(c);
   for (int t = 0; t < c.ntile; t++) {
     setup.tiles[t].rep = 0;
     setup.tiles[t].start = t * kNoAllocTile;
     setup.tiles[t].count = (s->nmol - t * kNoAllocTile < kNoAllocTile) ? s->nmol - t * kNoAllocTile : kNoAllocTile;
+    setup.tiles[t].mol_off = 0;
+    setup.tiles[t].part2_off = 0;
+    setup.tiles[t].npart2 = c.npart2;
+    setup.tiles[t].tile_off = 0;
     setup.tiles[t].pad = 0;
   }
   setup.rs.s = 1.0;
@@ -208,7 +219,8 @@ extern "C" remd_status remd_force_snapshot_noalloc(const remd_system_desc* s, co
   d.nbr = reinterpret_cast<uint16_t*>(b + kOffNbr);
   d.nbt = reinterpret_cast<uint16_t*>(b + kOffNbt);
   d.nt_cnt = reinterpret_cast<int*>(b + kOffNtc);
-  d.com = reinterpret_cast<int4*>(b + kOffCom);
+  d.wallf = reinterpret_cast<double*>(b + kOffWallf);
+  d.com = reinterpret_cast<int4*>(d.pack);   // the records' first pieces
   d.nbr_cnt = reinterpret_cast<int*>(b + kOffCnt);
   d.wall = d_wall;
   d.part1 = nullptr;
@@ -218,8 +230,11 @@ extern "C" remd_status remd_force_snapshot_noalloc(const remd_system_desc* s, co
   d.cgrid = reinterpret_cast<CellGrid*>(b + kOffGrid);
   d.cell_start = reinterpret_cast<int*>(b + kOffCellStart);
   d.cell_com = reinterpret_cast<int4*>(b + kOffCellMol);
-  d.rep0 = 0;
   d.nrep_l = 1;
+  d.model_l = pair_model(c);
+  d.pc = reinterpret_cast<PairConst*>(b + kOffPairC);
+  d.pblk = reinterpret_cast<PairBlk*>(b + kOffPblk);
+  d.npblk = c.npart2;
   d.bm_win = bitmap_window(s->nmol);
   RepState* X = reinterpret_cast<RepState*>(b + kOffState);
 
