@@ -223,9 +223,8 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     c.pack_off = pack_words;
     pack_words += (long long)c.nmol * c.pack_stride;
     c.nbr_off = nbr_words;
-    // FP32 form: one row per molecule; FP64 form: column-major inside a tile
-    c.nbr_stride = (c.nbr_cap + 7) / 8 * 8;
-    nbr_words += (h->prec == kF32) ? (long long)c.nmol * c.nbr_stride : (long long)c.ntile * c.nbr_cap * T;
+    c.nbr_stride = (c.nbr_cap + 7) / 8 * 8;   // one row per molecule
+    nbr_words += (long long)c.nmol * c.nbr_stride;
   }
   // force blocks in decreasing order of estimated pair work (longest first, so
   // the costliest tiles do not form the tail of the launch): molecules x
@@ -252,13 +251,12 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     const int K = std::min(npart2 <= 2400 ? kMaxChains : 4, h->nrep);
     std::vector<double> rcost(h->nrep, 0.0);
     std::map<int, double> mcost;   // cost per model
-    const bool by_model = h->prec == kF32;
     for (int r = 0; r < h->nrep; r++) {
       for (int t = h->rc[r].tile_off; t < h->rc[r].tile_off + h->rc[r].ntile; t++) rcost[r] += cost[t];
-      mcost[by_model ? h->rc[r].nsite : 0] += rcost[r];
+      mcost[h->rc[r].nsite] += rcost[r];
     }
     std::map<int, int> mchains, mreps;   // chains and replicas per model
-    for (int r = 0; r < h->nrep; r++) mreps[by_model ? h->rc[r].nsite : 0]++;
+    for (int r = 0; r < h->nrep; r++) mreps[h->rc[r].nsite]++;
     if ((int)mcost.size() > K) {
       double all = 0.0;
       for (auto& m : mcost) all += m.second;
@@ -285,7 +283,7 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
       double run = 0.0;
       int k = 0, used = 0, in_chain = 0, seen = 0;
       for (int r = 0; r < h->nrep; r++) {
-        if (m.first != -1 && m.first != 0 && h->rc[r].nsite != m.first) continue;
+        if (m.first != -1 && h->rc[r].nsite != m.first) continue;
         const int left_reps = mreps[m.first] - seen, left_chains = mchains[m.first] - k;
         if (in_chain > 0 && k + 1 < mchains[m.first] &&
             (run + 0.5 * rcost[r] > m.second * (k + 1) / mchains[m.first] || left_reps < left_chains)) {
@@ -359,7 +357,7 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
       N * sizeof(int4),                // 35 centres sorted by cell
       nr * sizeof(int2),               // 36 carried replicas' sources (serving batch changes)
       (size_t)h->nens * 4, (size_t)h->nens * 4,   // 37 carried ensembles' sources, 38 replicas per ensemble
-      nf * nr * sizeof(PairConst), nf * npart2 * sizeof(PairBlk), nf * npart2 * sizeof(PairBlk),   // 39 pair constants, 40 pair blocks, 41 per chain
+      nf * nr * sizeof(PairConst), npart2 * sizeof(PairBlk), npart2 * sizeof(PairBlk),   // 39 pair constants, 40 pair blocks, 41 per chain
       nf * nbr_words * 2, nf * N * 4, nf * N * 32,   // 42 nbt (per-step lists), 43 their counts, 44 wall terms
       nr * 4,                          // 45 replicas per chain
   };
@@ -475,9 +473,9 @@ static remd_status allocate(remd_engine_s* h) {
   if (h->prec == kF32) {
     for (const RepConst& c : h->rc) pc.push_back(pair_const(c));
     CK(cudaMemcpyAsync((void*)d.pc, pc.data(), pc.size() * sizeof(PairConst), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync((void*)d.pblk, h->pblk.data(), h->pblk.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_pblk2, h->pblk2.data(), h->pblk2.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
   }
+  CK(cudaMemcpyAsync((void*)d.pblk, h->pblk.data(), h->pblk.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->d_pblk2, h->pblk2.data(), h->pblk2.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
   if (!h->wall_h.empty())
     CK(cudaMemcpyAsync((void*)d.wall, h->wall_h.data(), h->wall_h.size() * 8, cudaMemcpyHostToDevice, h->stream));
   // later set-up copies use the default stream, which does not order with this
@@ -956,15 +954,14 @@ static remd_status create_impl(const remd_system_desc* systems, int nens, const 
       o->hT = o->hP = o->havg = nullptr;
       o->pinned_cap = 0;
     }
-    if (cudaSetDevice(device) != cudaSuccess || force_kernel_setup() != cudaSuccess) {
+    if (cudaSetDevice(device) != cudaSuccess) {
       set_error("cannot set up device");
       undo_carry(h, cy);
       return REMD_ERR_CUDA;
     }
   } else {
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        force_kernel_setup() != cudaSuccess) {
+        cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess) {
       set_error("cannot set up device/stream");
       delete h;
       return REMD_ERR_CUDA;

@@ -37,7 +37,7 @@ struct RepConst {
   int confined, tconstant, pconstant;
   int nfwall, wall_off;    // wall table entries and offset into the table array
   int nbr_cap;             // neighbour list capacity per molecule
-  int nbr_stride;          // FP32 form: words of a molecule's list (nbr_cap rounded up to 8)
+  int nbr_stride;          // words of a molecule's list (nbr_cap rounded up to 8)
   int ens;                 // ensemble index
   int pack_stride;         // words (FP32) or doubles (FP64) per pack record
   long long pack_off;      // FP64 form: first record double of this replica
@@ -157,7 +157,7 @@ struct DevPtrs {
   const double* newP;
   const int* changed;            // 1 = apply the exchange tail at the interval start
   const PairConst* pc;           // FP32 form, per replica
-  const PairBlk* pblk;           // FP32 form: list and pair blocks, costliest first
+  const PairBlk* pblk;           // list and pair blocks, costliest first
   int npblk;                     // pair blocks of a launch
   int model_l;                   // sites of every replica of a launch (0 when they differ) + kStdCharges
   const int* reps;               // replicas of a launch of the replica head (NULL: all)

@@ -512,160 +512,36 @@ __global__ void __launch_bounds__(kRepThreads) k_replica_head(DevPtrs d, const R
   }
 }
 
-// Neighbour-list rebuild for the molecules of this tile, one lane per molecule
-// (build_lists, the FP64 form; the FP32 form's build_lists_f32 below gives the
-// same lists with eight lanes per molecule).  The list of molecule i holds, in
-// ascending j, every j that passes the list test (below):
-//  * a replica not cut into cells (CellGrid 1 x 1 x 1): every molecule of the
-//    replica is tested, 128 candidates at a time from shared memory (all lanes
-//    read the same candidate: a broadcast), which emits them in ascending j;
-//  * a replica cut into cells (k_replica_head): molecule i tests the molecules
-//    of its neighbouring cells only (their centres, sorted by cell, carry the
-//    local index in .w) and sets their bits in its row of a bitmap in shared
-//    memory (`win` words per row: molecules [32 w0, 32 (w0 + win)) at a time),
-//    then emits the set bits in ascending j -- the same list as the scan.
-// FP32 form: the skin list only has to contain every pair within rcut+skin
-// (pass 1 then keeps exactly the pairs within rcut), so the test is a
+// Skin-list rebuild, kGroup lanes per molecule: a warp builds the lists of kWarpMol
+// consecutive molecules from li0 on, row-major (molecule li's list at d.nbr +
+// nbr_off + li * nbr_stride).  The list of molecule i holds, in ascending j, every j
+// that passes the list test:
+//  * a replica not cut into cells (CellGrid 1 x 1 x 1): every molecule is tested.  A
+//    lane loads one candidate and tests it against the warp's molecules, so that one
+//    load serves kWarpMol tests and 32 candidates advance per round; a ballot per
+//    molecule places the kept ones in ascending j;
+//  * a replica cut into cells (k_replica_head): the molecule's kGroup lanes split
+//    the molecules of its neighbouring cells (their centres, sorted by cell, carry
+//    the local index in .w) and set the molecule's bitmap row with shared-memory
+//    atomics (`win` words per row: molecules [32 w0, 32 (w0 + win)) at a time); the
+//    row is then emitted in ascending j, lane sub taking words sub, sub + kGroup,
+//    ..., placed by a prefix of their popcounts over the group: the same list.
+// The skin list only has to contain every pair within rcut + skin (the per-step
+// lists then keep exactly the pairs within rcut), so the test, of both forms, is a
 // conservative one in FP32 on the top 16 bits of each fixed-point difference
-// (converted with the 1.5*2^23 bit trick, on the FMA pipe), against
-// rcut+skin widened by the truncation error sqrt(3) L_max 2^-16 and a relative
-// 1e-5.  It may keep a few pairs just beyond rcut+skin; the lists, and
-// therefore the results, of pass 1 do not change.
-template <int PREC>
+// (converted with the 1.5*2^23 bit trick, on the FMA pipe), against rcut + skin
+// widened by the truncation error sqrt(3) L_max 2^-16 and a relative 1e-5.  It may
+// keep a few pairs just beyond rcut + skin; the per-step lists, and therefore the
+// results, do not change.
 __device__ __forceinline__ bool list_test(const int4 me, const int4 cj, float lsc0, float lsc1, float lsc2,
-                                          float rl2f, double rx, double ry, double rz, const double* wj,
-                                          const double* L, double rl2) {
-  if (PREC == kF32) {
-    const float fx = (__int_as_float(0x4B400000 + (wrap_diff(me.x, cj.x) >> 16)) - 12582912.f) * lsc0;
-    const float fy = (__int_as_float(0x4B400000 + (wrap_diff(me.y, cj.y) >> 16)) - 12582912.f) * lsc1;
-    const float fz = (__int_as_float(0x4B400000 + (wrap_diff(me.z, cj.z) >> 16)) - 12582912.f) * lsc2;
-    return fx * fx + fy * fy + fz * fz < rl2f;
-  }
-  double dx = (rx - wj[0]) * L[0];
-  double dy = (ry - wj[1]) * L[1];
-  double dz = (rz - wj[2]) * L[2];
-  if (dx >= 0.5 * L[0]) dx -= L[0];
-  if (dx < -0.5 * L[0]) dx += L[0];
-  if (dy >= 0.5 * L[1]) dy -= L[1];
-  if (dy < -0.5 * L[1]) dy += L[1];
-  if (dz >= 0.5 * L[2]) dz -= L[2];
-  if (dz < -0.5 * L[2]) dz += L[2];
-  return dx * dx + dy * dy + dz * dz < rl2;
+                                          float rl2f) {
+  const float fx = (__int_as_float(0x4B400000 + (wrap_diff(me.x, cj.x) >> 16)) - 12582912.f) * lsc0;
+  const float fy = (__int_as_float(0x4B400000 + (wrap_diff(me.y, cj.y) >> 16)) - 12582912.f) * lsc1;
+  const float fz = (__int_as_float(0x4B400000 + (wrap_diff(me.z, cj.z) >> 16)) - 12582912.f) * lsc2;
+  return fx * fx + fy * fy + fz * fz < rl2f;
 }
 
-__device__ void build_lists(const DevPtrs& d, const RepConst& c, const Tile& t, const double* L,
-                            uint16_t* nb, int tile_size, uint32_t* bm, int win) {
-  __shared__ double4 cand[128];
-  const int i = threadIdx.x;
-  const bool valid = i < t.count;
-  const int li = t.start + i;
-  const double rl = c.rc + c.skin;
-  const double rl2 = rl * rl;
-  const int4* com = d.com + c.mol_off;   // cell coordinates of the centres
-  const double* pk = reinterpret_cast<const double*>(d.pack) + c.pack_off;
-  int4 me = make_int4(0, 0, 0, 0);
-  double rx = 0, ry = 0, rz = 0;
-  if (valid) {
-    me = com[li];
-    rx = pk[(long long)li * c.pack_stride];
-    ry = pk[(long long)li * c.pack_stride + 1];
-    rz = pk[(long long)li * c.pack_stride + 2];
-  }
-  const CellGrid g = d.cgrid[t.rep];
-  int cnt = 0;
-  if (g.nx * g.ny * g.nz == 1) {
-    // every molecule, 128 at a time through shared memory (uniform over the block)
-    for (int base = 0; base < c.nmol; base += 128) {
-      __syncthreads();
-      for (int k = threadIdx.x; k < 128 && base + k < c.nmol; k += blockDim.x) {
-        const double* w = pk + (long long)(base + k) * c.pack_stride;
-        cand[k] = make_double4(w[0], w[1], w[2], 0);
-      }
-      __syncthreads();
-      if (valid) {
-        const int nk = min(128, c.nmol - base);
-        for (int k = 0; k < nk; k++) {
-          const int j = base + k;
-          const bool in = list_test<kF64>(me, make_int4(0, 0, 0, 0), 0.f, 0.f, 0.f, 0.f, rx, ry, rz,
-                                          reinterpret_cast<const double*>(&cand[k]), L, rl2);
-          if (j != li && in) {
-            if (cnt < c.nbr_cap) nb[(long long)cnt * tile_size] = (uint16_t)j;
-            cnt++;
-          }
-        }
-      }
-    }
-  } else if (valid) {
-    uint32_t* row = bm + i * (win | 1);   // odd row length: the lanes' words fall in distinct banks
-    const int W = (c.nmol + 31) >> 5;
-    const int cx = cell_coord(me.x, g.nx), cy = cell_coord(me.y, g.ny), cz = cell_coord(me.z, g.nz);
-    const int ox = (g.nx == 1) ? 0 : 1, oy = (g.ny == 1) ? 0 : 1, oz = (g.nz == 1) ? 0 : 1;
-    const int* cs = d.cell_start + (long long)t.rep * (kMaxCells + 1);
-    const int4* cm = d.cell_com + c.mol_off;
-    for (int w0 = 0; w0 < W; w0 += win) {
-      const int nw = min(win, W - w0);
-      for (int w = 0; w < nw; w++) row[w] = 0u;
-      const int jlo = 32 * w0, jhi = 32 * (w0 + nw);
-      for (int dz = -oz; dz <= oz; dz++) {
-        int zc = cz + dz;
-        zc += (zc < 0) ? g.nz : 0;
-        zc -= (zc >= g.nz) ? g.nz : 0;
-        for (int dy = -oy; dy <= oy; dy++) {
-          int yc = cy + dy;
-          yc += (yc < 0) ? g.ny : 0;
-          yc -= (yc >= g.ny) ? g.ny : 0;
-          for (int dx = -ox; dx <= ox; dx++) {
-            int xc = cx + dx;
-            xc += (xc < 0) ? g.nx : 0;
-            xc -= (xc >= g.nx) ? g.nx : 0;
-            const int cell = (zc * g.ny + yc) * g.nx + xc;
-            const int e = cs[cell + 1];
-            for (int k = cs[cell]; k < e; k++) {
-              const int4 cj = cm[k];
-              const int j = cj.w;
-              if (j < jlo || j >= jhi || j == li) continue;
-              if (list_test<kF64>(me, cj, 0.f, 0.f, 0.f, 0.f, rx, ry, rz, pk + (long long)j * c.pack_stride, L,
-                                  rl2))
-                row[(j - jlo) >> 5] |= 1u << (j & 31);
-            }
-          }
-        }
-      }
-      for (int w = 0; w < nw; w++) {
-        uint32_t bits = row[w];
-        while (bits) {
-          const int j = jlo + 32 * w + (__ffs(bits) - 1);
-          bits &= bits - 1u;
-          if (cnt < c.nbr_cap) nb[(long long)cnt * tile_size] = (uint16_t)j;
-          cnt++;
-        }
-      }
-    }
-  }
-  if (valid) {
-    if (cnt > c.nbr_cap) {
-      atomicOr(d.err, kErrNbrOverflow);
-      atomicMax(&d.status[t.rep], 8);
-      cnt = c.nbr_cap;
-    }
-    d.nbr_cnt[c.mol_off + li] = cnt;
-  }
-}
-
-// FP32 skin-list build, kGroup lanes per molecule: a warp builds the lists of
-// kWarpMol consecutive molecules from li0 on, row-major (molecule li's list at
-// d.nbr + nbr_off + li * nbr_stride).  The lists are entry for entry those that
-// build_lists gives with one lane per molecule (the FP64 form still builds its
-// lists that way):
-//  * all-molecule scan: a lane loads one candidate and tests it against the
-//    warp's molecules, so that one load serves kWarpMol tests and 32 candidates
-//    advance per round; a ballot per molecule places the kept ones in
-//    ascending j;
-//  * cell lists: the molecule's kGroup lanes split each neighbouring cell's
-//    molecules and set its bitmap row with shared-memory atomics; the row is
-//    then emitted in ascending j, lane sub taking words sub, sub + kGroup, ...,
-//    placed by a prefix of their popcounts over the group.
-__device__ void build_lists_f32(const DevPtrs& d, const RepConst& c, int rep, int li0, const double* L,
+__device__ void build_lists(const DevPtrs& d, const RepConst& c, int rep, int li0, const double* L,
                                 uint32_t* bm, int win) {
   const int lane = threadIdx.x & 31, grp = lane / kGroup, sub = lane % kGroup;
   const float lsc0 = (float)(L[0] * (1.0 / 65536.0)), lsc1 = (float)(L[1] * (1.0 / 65536.0)),
@@ -692,7 +568,7 @@ __device__ void build_lists_f32(const DevPtrs& d, const RepConst& c, int rep, in
 #pragma unroll
       for (int m = 0; m < kWarpMol; m++) {
         const bool in = j < nmol && j != li0 + m &&
-                        list_test<kF32>(me[m], cj, lsc0, lsc1, lsc2, rl2f, 0.0, 0.0, 0.0, nullptr, L, 0.0);
+                        list_test(me[m], cj, lsc0, lsc1, lsc2, rl2f);
         const unsigned b = __ballot_sync(0xffffffffu, in);
         const int pos = n[m] + __popc(b & below);
         if (in && pos < cap && li0 + m < nmol) nb0[(long long)m * c.nbr_stride + pos] = (uint16_t)j;
@@ -736,7 +612,7 @@ __device__ void build_lists_f32(const DevPtrs& d, const RepConst& c, int rep, in
                 const int4 cj = cm[k];
                 const int j = cj.w;
                 if (j < jlo || j >= jhi || j == li) continue;
-                if (list_test<kF32>(me, cj, lsc0, lsc1, lsc2, rl2f, 0.0, 0.0, 0.0, nullptr, L, 0.0))
+                if (list_test(me, cj, lsc0, lsc1, lsc2, rl2f))
                   atomicOr(&row[(j - jlo) >> 5], 1u << (j & 31));
               }
             }
@@ -776,92 +652,6 @@ __device__ void build_lists_f32(const DevPtrs& d, const RepConst& c, int rep, in
   }
 }
 
-// Accumulators of one molecule i.
-struct IAcc {
-  double fs[kMaxSites][3];   // site forces (switched pair terms + wall on site 0)
-  double fc[3];              // switching correction -E dS/dr r^ (acts on the molecule only)
-  double vir[3], lj, clmb;
-  long long npair;
-};
-
-template <int S, int C0, bool SIMG>
-__device__ void pair_loop_f64(const DevPtrs& d, const RepConst& c, const Tile& t, const double* L,
-                              const uint16_t* nb, int cnt, IAcc& a) {
-  constexpr int STRIDE = ((3 + 3 * S) + 1) / 2 * 2;
-  const int li = t.start + threadIdx.x;
-  const double* base = reinterpret_cast<const double*>(d.pack) + c.pack_off;
-  double wi[STRIDE];
-#pragma unroll
-  for (int k = 0; k < STRIDE; k++) wi[k] = base[(long long)li * STRIDE + k];
-  const double rc = c.rc, rl = c.rs, coef = c.coef_sw, rc2 = c.rc * c.rc;
-  for (int k = 0; k < cnt; k++) {
-    const int j = nb[(long long)k * blockDim.x];
-    const double* wj = base + (long long)j * STRIDE;
-    double gr[3];
-    for (int x = 0; x < 3; x++) {
-      gr[x] = (wi[x] - wj[x]) * L[x];
-      if (gr[x] >= 0.5 * L[x]) gr[x] -= L[x];
-      if (gr[x] < -0.5 * L[x]) gr[x] += L[x];
-    }
-    const double r02 = gr[0] * gr[0] + gr[1] * gr[1] + gr[2] * gr[2];
-    if (r02 > rc2) continue;
-    a.npair++;
-    const double r01 = sqrt(r02);
-    double sw = 1.0, dsw = 0.0;
-    if (r01 > rl) {
-      const double r01c = r01 - rc, r01l = r01 - rl;
-      sw = coef * r01c * r01c * r01c * (10.0 * r01l * r01l - 5.0 * r01l * r01c + r01c * r01c);
-      dsw = coef * 30.0 * r01c * r01c * r01l * r01l;
-    }
-    double dswr[3];
-    for (int x = 0; x < 3; x++) dswr[x] = gr[x] * (dsw / r01);
-#pragma unroll
-    for (int kk = 0; kk < S; kk++) {
-      if (kk != 0 && kk < C0) continue;
-      double e = 0.0, f[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-      for (int l = 0; l < S; l++) {
-        const bool lj_pair = (kk == 0 && l == 0);
-        const bool cl_pair = (kk >= C0 && l >= C0);
-        if (!lj_pair && !cl_pair) continue;
-        double rv[3];
-        for (int x = 0; x < 3; x++) {
-          rv[x] = gr[x] + wi[3 + 3 * kk + x] - wj[3 + 3 * l + x];
-          if (SIMG) {
-            if (rv[x] >= 0.5 * L[x]) rv[x] -= L[x];
-            if (rv[x] < -0.5 * L[x]) rv[x] += L[x];
-          }
-        }
-        const double rr = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-        const double r02i = 1.0 / rr;
-        const double r01i = sqrt(r02i);
-        const double qq = cl_pair ? c.qq[kk][l] : 0.0;
-        double elj = 0.0, flj = 0.0;
-        if (lj_pair) {
-          double rs06i = c.sgm2 * r02i;
-          rs06i = rs06i * rs06i * rs06i;
-          elj = 4.0 * c.eps * rs06i * (rs06i - 1.0);
-          flj = 48.0 * c.eps * rs06i * (rs06i - 0.5) * r02i;
-        }
-        const double ecl = qq * r01i;
-        a.lj += sw * elj;
-        a.clmb += sw * ecl;
-        const double ftmp = (flj + qq * r01i * r02i) * sw;
-        e += elj + ecl;
-        for (int x = 0; x < 3; x++) {
-          f[x] += rv[x] * ftmp;
-          a.fs[kk][x] += rv[x] * ftmp;
-        }
-      }
-      for (int x = 0; x < 3; x++) {
-        const double cx = -dswr[x] * e;
-        a.fc[x] += cx;
-        a.vir[x] += (f[x] + cx) * gr[x];
-      }
-    }
-  }
-}
-
 // Wall on the oxygen site of a molecule at (r, q): adds the force to f and
 // returns the energy (ForceCalculator::Confined, src/force_calculator.cxx:1527-1566;
 // slit: src/remdgpu.cu:1708-1720).
@@ -890,102 +680,6 @@ __device__ __forceinline__ double wall_site(const DevPtrs& d, const RepConst& c,
   const double fz = (w1.x - w0.x) / dr * (za - dr * idx) + w0.x;
   f[2] += fz * dir;
   return (w1.y - w0.y) / dr * (za - dr * idx) + w0.y;
-}
-
-// Wall and A2M for molecule g (FP64 form): writes d.f, d.n.
-template <int S>
-__device__ void finish_molecule(const DevPtrs& d, const RepConst& c, int g, const double* L, IAcc& a,
-                                double& wall_e) {
-  const int N = d.N;
-  double q[4], r[3];
-  for (int x = 0; x < 4; x++) q[x] = d.q[x * N + g];
-  for (int x = 0; x < 3; x++) r[x] = d.r[x * N + g];
-  if (c.confined > 0) wall_e = wall_site(d, c, q, r, L, a.fs[0]);
-  // A2M: molecular force and body torque (src/molecules.cxx:447-475)
-  double F[3] = {a.fc[0], a.fc[1], a.fc[2]};
-  double nq[4] = {0, 0, 0, 0};
-#pragma unroll
-  for (int k = 0; k < S; k++) {
-    for (int x = 0; x < 3; x++) F[x] += a.fs[k][x];
-    double fb[3];
-    space_to_body(q, a.fs[k], fb);
-    const double* b = c.body[k];
-    nq[0] += b[0] * fb[0] + b[1] * fb[1] + b[2] * fb[2];
-    nq[1] += b[1] * fb[2] - b[2] * fb[1];
-    nq[2] += b[2] * fb[0] - b[0] * fb[2];
-    nq[3] += b[0] * fb[1] - b[1] * fb[0];
-  }
-  for (int x = 0; x < 3; x++) d.f[x * N + g] = F[x];
-  for (int x = 0; x < 4; x++) d.n[x * N + g] = nq[x];
-}
-
-// Force partials of the tile's units of kPart2Mol molecules (a fixed shuffle tree
-// over kPart2Mol lanes; FP64 form, one lane per molecule).
-__device__ inline void write_part2(const DevPtrs& d, const RepConst& c, const Tile& t, const IAcc& a,
-                                   double wall_e) {
-  double s7[7] = {a.lj, a.clmb, wall_e, a.vir[0], a.vir[1], a.vir[2], (double)a.npair};
-#pragma unroll
-  for (int k = 0; k < 7; k++)
-    for (int o = kPart2Mol / 2; o > 0; o >>= 1) s7[k] += __shfl_xor_sync(0xffffffffu, s7[k], o);
-  const int w = (t.start + threadIdx.x) / kPart2Mol;
-  if (threadIdx.x % kPart2Mol == 0 && w < c.npart2) {
-    Part2 p;
-    p.lj = s7[0]; p.clmb = s7[1]; p.wall = s7[2];
-    p.vir[0] = s7[3]; p.vir[1] = s7[4]; p.vir[2] = s7[5];
-    p.npairs = (long long)llrint(s7[6]);
-    p.pad = 0.0;
-    d.part2[c.part2_off + w] = p;
-  }
-}
-
-__device__ inline void zero_acc(IAcc& a) {
-#pragma unroll
-  for (int k = 0; k < kMaxSites; k++) a.fs[k][0] = a.fs[k][1] = a.fs[k][2] = 0.0;
-  a.fc[0] = a.fc[1] = a.fc[2] = 0.0;
-  a.vir[0] = a.vir[1] = a.vir[2] = 0.0;
-  a.lj = a.clmb = 0.0;
-  a.npair = 0;
-}
-
-// FP64 form: skin-list rebuild of tile t when due, with the build's reference
-// centres and box.
-__device__ void rebuild_tile(const DevPtrs& d, const RepConst& c, const Tile& t, int tix, const double* L,
-                             uint16_t* nb, int tile_size, uint32_t* bm, int win) {
-  const int i = threadIdx.x;
-  const int li = t.start + i;
-  build_lists(d, c, t, L, nb, tile_size, bm, win);
-  if (i < t.count) {
-    const double* wd = reinterpret_cast<const double*>(d.pack) + c.pack_off + (long long)li * c.pack_stride;
-    d.ref_com[c.mol_off + li] = make_int4(fix_coord(wd[0]), fix_coord(wd[1]), fix_coord(wd[2]), 0);
-  }
-  if (i == 0)
-    for (int x = 0; x < 3; x++) d.Lbuild[3 * tix + x] = L[x];
-}
-
-__device__ inline bool site_image_needed(const RepConst& c, const double* L) {
-  const double reach = c.rc + 2.0 * c.site_reach;
-  return (L[0] < 2.0 * reach) || (L[1] < 2.0 * reach) || (L[2] < 2.0 * reach);
-}
-
-// FP64 form: rebuild when due, pair loop, wall, A2M.
-template <int S, int C0>
-__device__ void force_tile_f64(const DevPtrs& d, const RepConst& c, const Tile& t, int tix, const double* L,
-                               bool rebuild, int tile_size, uint32_t* bm, int win) {
-  const int i = threadIdx.x;
-  const int li = t.start + i;
-  const int g = c.mol_off + li;
-  uint16_t* nb = d.nbr + c.nbr_off + (long long)(tix - c.tile_off) * c.nbr_cap * tile_size + i;
-  if (rebuild) rebuild_tile(d, c, t, tix, L, nb, tile_size, bm, win);
-  IAcc a;
-  zero_acc(a);
-  double wall_e = 0.0;
-  if (i < t.count) {
-    const int cnt = d.nbr_cnt[g];
-    if (site_image_needed(c, L)) pair_loop_f64<S, C0, true>(d, c, t, L, nb, cnt, a);
-    else pair_loop_f64<S, C0, false>(d, c, t, L, nb, cnt, a);
-    finish_molecule<S>(d, c, g, L, a, wall_e);
-  }
-  write_part2(d, c, t, a, wall_e);
 }
 
 // ------------------------------------------------------------------ FP32 pair step
@@ -1321,8 +1015,8 @@ __device__ __forceinline__ int force_warp_f32(const DevPtrs& d, const PairBlk& b
 // term {force, energy} (lanes 0..3; both loaded before the pairs): writes d.f and
 // d.n, one component per lane.  On return lane 5 of the group holds {wall energy,
 // 0, 0}, lane 6 the virial and lane 7 {LJ, Coulomb, pairs} in acc.
-template <int S>
-__device__ __forceinline__ void finish_group(const DevPtrs& d, const PairConst& c, int li, int sub,
+template <int S, class Const>
+__device__ __forceinline__ void finish_group(const DevPtrs& d, const Const& c, int li, int sub,
                                              double q4, double wf, double* acc, int npairs) {
   const int N = d.N, g = c.mol_off + li;
   const bool valid = li < c.nmol;
@@ -1360,27 +1054,306 @@ __device__ __forceinline__ void finish_group(const DevPtrs& d, const PairConst& 
   if (sub == 7) acc[2] = (double)npairs;
 }
 
-// FP64 form: one launch per step after the replica head (list rebuild when
-// due, pairs, wall, A2M); the box and the rebuild decision come from
-// k_replica_head.
-__global__ void __launch_bounds__(128, 1) k_force_f64(DevPtrs d, const RepState* __restrict__ X, int tile_size) {
+// ------------------------------------------------------------------ FP64 form
+// One launch per step after the replica head (k_force_f64): per warp of kWarpMol
+// molecules, kGroup lanes each, the skin lists where due, then in segments of up to
+// kSegPairs pairs per molecule the gather of the neighbours within rcut (tested in
+// FP64, ballot-placed in ascending j) into a shared-memory row and the pairs, lane
+// sub entries sub, sub + 8, ..., all sums FP64; at the end wall and A2M.  As in the
+// FP32 form the pairs a lane sums depend on the positions only.  1/r is one rsqrt
+// (its square for 1/r^2) instead of a division and a square root per site pair.
+// With one lane per molecule and 128 molecules per block, 800 TIP4P molecules were
+// seven blocks, each thread walking a whole list: 224 us a launch; bound by FP64
+// latency then, and where the grid fills the GPU by the FP64 pipe.
+template <int S>
+struct F64Sums {
+  double fs[S][3], fc[3], fv[3], lj, cl;
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int k = 0; k < S; k++) fs[k][0] = fs[k][1] = fs[k][2] = 0.0;
+    fc[0] = fc[1] = fc[2] = 0.0;
+    fv[0] = fv[1] = fv[2] = 0.0;
+    lj = cl = 0.0;
+  }
+  __device__ __forceinline__ double at(int slot, int x) const {   // slots as F32Sums::at
+    if (slot < S) return fs[slot][x];
+    if (slot == 5) return fc[x];
+    if (slot == 6) return fv[x];
+    if (slot == 7) return x == 0 ? lj : x == 1 ? cl : 0.0;
+    return 0.0;
+  }
+};
+
+// COM vector of a pair in the minimum image (r: box fractions).
+__device__ __forceinline__ void com_vector(const double* ri, const double* rj, const double* L, double* gr) {
+#pragma unroll
+  for (int x = 0; x < 3; x++) {
+    gr[x] = (ri[x] - rj[x]) * L[x];
+    if (gr[x] >= 0.5 * L[x]) gr[x] -= L[x];
+    if (gr[x] < -0.5 * L[x]) gr[x] += L[x];
+  }
+}
+
+// SIMG: the minimum image of every site pair, as the reference takes it
+// (src/force_calculator.cxx:737-741); it matters only when a box length is below
+// 2 (rc + 2 site_reach), and the caller enables it just then.
+template <int S, int C0, bool SIMG>
+__device__ __forceinline__ void pair_loop_f64(const RepConst& c, const double* pack, const double* L,
+                                              const double* wi, const uint16_t* row, int n, F64Sums<S>& a) {
+  constexpr int STRIDE = ((3 + 3 * S) + 1) / 2 * 2;
+  const double rc = c.rc, rs = c.rs, coef = c.coef_sw;
+  for (int k = 0; k < n; k++) {
+    const double2* w2 = reinterpret_cast<const double2*>(pack + (long long)row[k * kGroup] * STRIDE);
+    double wj[STRIDE];
+#pragma unroll
+    for (int m = 0; m < STRIDE / 2; m++) {
+      const double2 u = __ldg(w2 + m);
+      wj[2 * m] = u.x; wj[2 * m + 1] = u.y;
+    }
+    double gr[3];
+    com_vector(wi, wj, L, gr);
+    const double r02 = gr[0] * gr[0] + gr[1] * gr[1] + gr[2] * gr[2];
+    const double rinv = rsqrt(r02);
+    const double r = r02 * rinv;
+    double sw = 1.0, dsw = 0.0;
+    if (r > rs) {
+      const double r01c = r - rc, r01l = r - rs, cc = coef * r01c * r01c;
+      sw = cc * r01c * (10.0 * r01l * r01l - 5.0 * r01l * r01c + r01c * r01c);
+      dsw = cc * 30.0 * r01l * r01l;
+    }
+    double elj = 0.0, ecl = 0.0, fp[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int kk = 0; kk < S; kk++) {
+      if (kk != 0 && kk < C0) continue;
+      double t[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int l = 0; l < S; l++) {
+        const bool lj_pair = (kk == 0 && l == 0);
+        const bool cl_pair = (kk >= C0 && l >= C0);
+        if (!lj_pair && !cl_pair) continue;
+        double v[3];
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+          v[x] = gr[x] + wi[3 + 3 * kk + x] - wj[3 + 3 * l + x];
+          if (SIMG) {
+            if (v[x] >= 0.5 * L[x]) v[x] -= L[x];
+            if (v[x] < -0.5 * L[x]) v[x] += L[x];
+          }
+        }
+        const double ri = rsqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+        const double ri2 = ri * ri;
+        double f = 0.0;
+        if (lj_pair) {
+          double s6 = c.sgm2 * ri2;
+          s6 = s6 * s6 * s6;
+          elj = 4.0 * c.eps * s6 * (s6 - 1.0);
+          f = 48.0 * c.eps * s6 * (s6 - 0.5) * ri2;
+        }
+        if (cl_pair) {
+          const double e = c.qq[kk][l] * ri;
+          ecl += e;
+          f += e * ri2;
+        }
+#pragma unroll
+        for (int x = 0; x < 3; x++) t[x] += v[x] * f;
+      }
+#pragma unroll
+      for (int x = 0; x < 3; x++) {
+        a.fs[kk][x] += sw * t[x];
+        fp[x] += sw * t[x];
+      }
+    }
+    const double g = -(dsw * rinv) * (elj + ecl);
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+      const double cx = gr[x] * g;
+      a.fc[x] += cx;
+      a.fv[x] += (fp[x] + cx) * gr[x];
+    }
+    a.lj += sw * elj;
+    a.cl += sw * ecl;
+  }
+}
+
+// Pair forces of molecules li0 .. li0 + kWarpMol - 1 by one warp, as force_warp_f32;
+// `row0` is the warp's buffer.
+template <int S, int C0, bool SIMG>
+__device__ int force_warp_f64(const DevPtrs& d, const RepConst& c, const double* L, int li0, uint16_t* row0,
+                              double* acc) {
+  constexpr int STRIDE = ((3 + 3 * S) + 1) / 2 * 2;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, grp = lane / kGroup, sub = lane % kGroup;
+  const unsigned group = ((1u << kGroup) - 1u) << (lane - sub), below = group & ((1u << lane) - 1u);
+  const int li = li0 + grp, lic = min(li, c.nmol - 1);
+  const double* pack = reinterpret_cast<const double*>(d.pack) + c.pack_off;
+  const uint16_t* nb = d.nbr + c.nbr_off + (long long)lic * c.nbr_stride;
+  const int cnt = (li < c.nmol) ? d.nbr_cnt[c.mol_off + li] : 0;
+  double wi[STRIDE];
+#pragma unroll
+  for (int k = 0; k < STRIDE; k++) wi[k] = pack[(long long)lic * STRIDE + k];
+  const double rc2 = c.rc * c.rc;
+  auto within = [&](int j) {
+    const double* w = pack + (long long)j * STRIDE;
+    const double rj[3] = {__ldg(w), __ldg(w + 1), __ldg(w + 2)};
+    double gr[3];
+    com_vector(wi, rj, L, gr);
+    return !(gr[0] * gr[0] + gr[1] * gr[1] + gr[2] * gr[2] > rc2);
+  };
+  uint16_t* row = row0 + grp * kSegPairs;
+  F64Sums<S> a;
+  a.zero();
+  int pos = 0, skip = 0, npairs = 0;   // list position; pairs of the round at pos already taken
+  do {
+    int n = 0;
+    constexpr int B = 4;   // rounds whose loads are in flight together
+    while (true) {
+      const bool go = pos < cnt && n < kSegPairs;
+      if (!__any_sync(kAll, go)) break;
+      if (!__any_sync(kAll, go && (skip > 0 || n + B * kGroup > kSegPairs))) {
+        int j[B];
+        bool in[B];
+#pragma unroll
+        for (int m = 0; m < B; m++) {
+          const int k = pos + m * kGroup + sub;
+          j[m] = (go && k < cnt) ? (int)nb[k] : -1;
+        }
+#pragma unroll
+        for (int m = 0; m < B; m++) in[m] = within(max(j[m], 0)) && j[m] >= 0;
+#pragma unroll
+        for (int m = 0; m < B; m++) {
+          const unsigned b = __ballot_sync(kAll, in[m]);
+          if (in[m]) row[n + __popc(b & below)] = (uint16_t)j[m];
+          n += __popc(b & group);
+        }
+        if (go) pos += B * kGroup;
+      } else {
+        // one round, cut exactly at the segment's last pair
+        const int k = pos + sub;
+        const int j = (go && k < cnt) ? (int)nb[k] : -1;
+        const bool in = j >= 0 && within(j);
+        const unsigned b = __ballot_sync(kAll, in);
+        const int ord = __popc(b & below) - skip, left = __popc(b & group) - skip;
+        const int take = min(left, kSegPairs - n);
+        if (in && ord >= 0 && ord < take) row[n + ord] = (uint16_t)j;
+        if (go) {
+          n += take;
+          const bool all = take == left;
+          skip = all ? 0 : skip + take;
+          pos += all ? kGroup : 0;
+        }
+      }
+    }
+    npairs += n;
+    __syncwarp();
+    pair_loop_f64<S, C0, SIMG>(c, pack, L, wi, row + sub, (n - sub + kGroup - 1) / kGroup, a);
+    __syncwarp();   // the row is free again
+  } while (__any_sync(kAll, pos < cnt));
+  // the group's lanes added by the exchange tree: lane sub ends with slot sub
+  double v[24];
+#pragma unroll
+  for (int s = 0; s < 8; s++)
+#pragma unroll
+    for (int x = 0; x < 3; x++) v[3 * s + x] = a.at(s, x);
+  exchange_sum<12>(v, sub, 4);
+  exchange_sum<6>(v, sub, 2);
+  exchange_sum<3>(v, sub, 1);
+#pragma unroll
+  for (int x = 0; x < 3; x++) acc[x] = v[x];
+  return npairs;
+}
+
+// The block's partial sums from its lanes' {wall}, {virial}, {LJ, Coulomb, pairs}
+// (lanes 5, 6, 7 of each group, finish_group).
+__device__ __forceinline__ void write_part2(const DevPtrs& d, int record, double* acc, double (*wsum)[8]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int x = 0; x < 3; x++)
+    for (int o = kGroup; o < 32; o <<= 1) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
+  if (lane == 5) wsum[warp][0] = acc[0];
+  if (lane == 6)
+    for (int x = 0; x < 3; x++) wsum[warp][1 + x] = acc[x];
+  if (lane == 7)
+    for (int x = 0; x < 3; x++) wsum[warp][4 + x] = acc[x];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s[7];
+    for (int k = 0; k < 7; k++) {
+      s[k] = wsum[0][k];
+      for (int w = 1; w < kPairWarps; w++) s[k] += wsum[w][k];
+    }
+    Part2 p;
+    p.wall = s[0];
+    p.vir[0] = s[1]; p.vir[1] = s[2]; p.vir[2] = s[3];
+    p.lj = s[4]; p.clmb = s[5];
+    p.npairs = (long long)llrint(s[6]);
+    p.pad = 0.0;
+    d.part2[record] = p;
+  }
+}
+
+__device__ inline bool site_image_needed(const RepConst& c, const double* L) {
+  const double reach = c.rc + 2.0 * c.site_reach;
+  return (L[0] < 2.0 * reach) || (L[1] < 2.0 * reach) || (L[2] < 2.0 * reach);
+}
+
+template <int S, int C0>
+__device__ void force_block_f64(const DevPtrs& d, const PairBlk& b, const RepConst& c, const double* L,
+                                uint16_t* rows, double (*wsum)[8]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % kGroup;
+  const int lw = b.li0 + warp * kWarpMol, li = lw + lane / kGroup, g = b.mol_off + min(li, b.nmol - 1);
+  double q4 = 0.0, w[4] = {0.0, 0.0, 0.0, 0.0};   // one component of q; wall force and energy
+  if (sub < 4 && li < b.nmol) q4 = d.q[sub * d.N + g];
+  if (b.confined && sub == 0 && li < b.nmol) {
+    double q[4], r[3];
+    for (int x = 0; x < 4; x++) q[x] = d.q[x * d.N + g];
+    for (int x = 0; x < 3; x++) r[x] = d.r[x * d.N + g];
+    w[3] = wall_site(d, c, q, r, L, w);
+  }
+  double wf = 0.0;
+#pragma unroll
+  for (int x = 0; x < 4; x++) {
+    const double t = __shfl_sync(0xffffffffu, w[x], 0, kGroup);
+    if (sub == x) wf = t;
+  }
+  double acc[3];
+  uint16_t* row0 = rows + warp * kWarpMol * kSegPairs;
+  const int npairs = site_image_needed(c, L) ? force_warp_f64<S, C0, true>(d, c, L, lw, row0, acc)
+                                             : force_warp_f64<S, C0, false>(d, c, L, lw, row0, acc);
+  finish_group<S>(d, c, li, sub, q4, wf, acc, npairs);
+  write_part2(d, c.part2_off + b.li0 / kPart2Mol, acc, wsum);
+}
+
+// S as k_force_pairs.
+template <int S>
+__global__ void __launch_bounds__(32 * kPairWarps, 2) k_force_f64(DevPtrs d, const RepState* __restrict__ X) {
   step_kernel_entry();
   extern __shared__ uint32_t bm[];
-  __shared__ double Ls[3];
-  __shared__ int rb;
-  const int tix = d.order ? d.order[blockIdx.x] : (int)blockIdx.x;   // costliest tiles first
-  const Tile t = d.tiles[tix];
-  const RepConst& c = d.rc[t.rep];
-  if (threadIdx.x < 3) Ls[threadIdx.x] = X[t.rep].L[threadIdx.x];
-  if (threadIdx.x == 0) rb = d.cgrid[t.rep].rebuild;
+  __shared__ RepConst c;
+  __shared__ uint16_t rows[kPairWarps * kWarpMol * kSegPairs];
+  __shared__ double wsum[kPairWarps][8];
+  const PairBlk b = d.pblk[blockIdx.x];
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(d.rc + b.rep);
+  for (int k = threadIdx.x; k < (int)(sizeof(RepConst) / 4); k += 32 * kPairWarps)
+    reinterpret_cast<uint32_t*>(&c)[k] = src[k];
+  const double L[3] = {X[b.rep].L[0], X[b.rep].L[1], X[b.rep].L[2]};
+  const int rebuild = d.cgrid[b.rep].rebuild;
   __syncthreads();
-  const double L[3] = {Ls[0], Ls[1], Ls[2]};
-  if (c.nsite == 3)
-    force_tile_f64<3, 0>(d, c, t, tix, L, rb != 0, tile_size, bm, d.bm_win);
-  else if (c.nsite == 4)
-    force_tile_f64<4, 1>(d, c, t, tix, L, rb != 0, tile_size, bm, d.bm_win);
+  const int li0 = b.li0 + (threadIdx.x >> 5) * kWarpMol;
+  if (rebuild) {
+    if (li0 < b.nmol) {
+      build_lists(d, c, b.rep, li0, L, bm, d.bm_win);
+      const int li = li0 + (threadIdx.x & 31) / kGroup;
+      if (threadIdx.x % kGroup == 0 && li < b.nmol) d.ref_com[b.mol_off + li] = d.com[b.mol_off + li];
+      __syncwarp();   // the lists, written by all lanes, are read below
+    }
+    if (threadIdx.x < 3 && b.li0 % b.tile == 0) d.Lbuild[3 * (c.tile_off + b.li0 / b.tile) + threadIdx.x] = L[threadIdx.x];
+  }
+  if (S == 3 || (S == 0 && c.nsite == 3))
+    force_block_f64<3, 0>(d, b, c, L, rows, wsum);
+  else if (S == 4 || (S == 0 && c.nsite == 4))
+    force_block_f64<4, 1>(d, b, c, L, rows, wsum);
   else
-    force_tile_f64<5, 1>(d, c, t, tix, L, rb != 0, tile_size, bm, d.bm_win);
+    force_block_f64<5, 1>(d, b, c, L, rows, wsum);
 }
 
 // A lane's eight skin-list entries from k on, read 16 bytes at a time.  Also past
@@ -1493,7 +1466,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_list
   if (li0 >= b.nmol) return;
   if (rebuild) {
     const RepConst& rc = d.rc[b.rep];
-    build_lists_f32(d, rc, b.rep, li0, L, bm, d.bm_win);
+    build_lists(d, rc, b.rep, li0, L, bm, d.bm_win);
     if (sub == 0 && li < b.nmol) d.ref_com[g] = make_int4(me.x, me.y, me.z, 0);
     if (threadIdx.x < 3 && b.li0 % b.tile == 0)
       d.Lbuild[3 * (rc.tile_off + b.li0 / b.tile) + threadIdx.x] = L[threadIdx.x];
@@ -1522,29 +1495,7 @@ __device__ void force_block_f32(const DevPtrs& d, const PairBlk& b, const PairCo
   double acc[3] = {0.0, 0.0, 0.0};
   const int npairs = force_warp_f32<S, C0, STD>(d, b, c, k32, lw, nc, acc);
   finish_group<S>(d, c, lw + lane / kGroup, sub, q4, wf, acc, npairs);
-#pragma unroll
-  for (int x = 0; x < 3; x++)
-    for (int o = kGroup; o < 32; o <<= 1) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
-  if (lane == 5) wsum[warp][0] = acc[0];
-  if (lane == 6)
-    for (int x = 0; x < 3; x++) wsum[warp][1 + x] = acc[x];
-  if (lane == 7)
-    for (int x = 0; x < 3; x++) wsum[warp][4 + x] = acc[x];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s[7];
-    for (int k = 0; k < 7; k++) {
-      s[k] = wsum[0][k];
-      for (int w = 1; w < kPairWarps; w++) s[k] += wsum[w][k];
-    }
-    Part2 p;
-    p.wall = s[0];
-    p.vir[0] = s[1]; p.vir[1] = s[2]; p.vir[2] = s[3];
-    p.lj = s[4]; p.clmb = s[5];
-    p.npairs = (long long)llrint(s[6]);
-    p.pad = 0.0;
-    d.part2[c.part2_off + b.li0 / kPart2Mol] = p;
-  }
+  write_part2(d, c.part2_off + b.li0 / kPart2Mol, acc, wsum);
 }
 
 // S: the sites of every replica of the launch (0: mixed models, chosen per
@@ -2316,11 +2267,8 @@ size_t bitmap_smem_bytes(int mols, int win) { return (size_t)mols * (size_t)(win
 
 int bitmap_window(int max_nmol) { return std::min((max_nmol + 31) / 32, kBitmapMaxWords); }
 
-cudaError_t force_kernel_setup() {
-  // rebuild bitmaps of the FP64 form's blocks: up to 128 rows of kBitmapMaxWords + 1 words
-  const int bms = (int)bitmap_smem_bytes(128, kBitmapMaxWords);
-  return cudaFuncSetAttribute(k_force_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, bms);
-}
+// every block's rebuild bitmaps fit the default limit beside the kernels' static arrays
+static_assert(kPart2Mol * (kBitmapMaxWords + 1) * 4 <= 8192, "rebuild bitmaps");
 
 // The force launches of one step; e_head / e_lists (may be null) are recorded
 // after the head and after the list kernel (profiling: remd_profile_split).
@@ -2349,7 +2297,10 @@ static void launch_force_impl(const DevPtrs& d, const RepState* Yin, RepState* X
     launch_step_kernel(pdl, pairs, d.npblk, 32 * kPairWarps, 0, s, d, Xc);
   } else {
     if (e_lists) cudaEventRecord(e_lists, s);
-    launch_step_kernel(pdl, k_force_f64, d.ntiles, tile, bitmap_smem_bytes(tile, d.bm_win), s, d, Xc, tile);
+    const int sites = d.model_l % kStdCharges;
+    void (*force)(DevPtrs, const RepState*) =
+        sites == 3 ? k_force_f64<3> : sites == 4 ? k_force_f64<4> : sites == 5 ? k_force_f64<5> : k_force_f64<0>;
+    launch_step_kernel(pdl, force, d.npblk, 32 * kPairWarps, bitmap_smem_bytes(kPart2Mol, d.bm_win), s, d, Xc);
   }
 }
 

@@ -2,7 +2,7 @@
 //
 // One MD step of every replica of every ensemble is a short chain of launches
 // (a tile = 32 or 64 consecutive molecules of one replica, up to 128 in the
-// FP64 form):
+// FP64 form, a block of k_integrate):
 //
 //   k_integrate     [end of the previous step: D5 kick, D5/D6 scalars]
 //                   D6, D5, D4, D3 D2 D1 D2 D3 (src/integrator.cxx:646-673),
@@ -14,7 +14,7 @@
 //                   the per-step list of the pairs within rcut, and the wall terms;
 //   k_force_pairs   FP32, eight lanes per molecule: the switched LJ + Coulomb pair
 //                   loop and the site -> molecule torque (A2M);
-//   k_force_f64     per tile (FP64 form): rebuild, pair loop, wall, A2M.
+//   k_force_f64     FP64 form, eight lanes per molecule: rebuild, pairs, wall, A2M.
 //
 // An interval is k_replica_start (exchange tail), interval x (step chain),
 // k_replica_end (last D5/D6 + CalcProperties -> Average), captured once as a
@@ -32,8 +32,6 @@ void launch_integrate_prec(const DevPtrs& d, const RepState* X, RepState* Y, boo
                            int prec, cudaStream_t s);
 // Largest tile (molecules per integrate block; FP64 form: per force block) of a precision.
 int max_force_tile(int prec);
-// Kernel attributes the force launches need (call once per device before launching).
-cudaError_t force_kernel_setup();
 // Words per row of the list-rebuild bitmap for replicas of up to max_nmol molecules (DevPtrs::bm_win).
 int bitmap_window(int max_nmol);
 void launch_force(const DevPtrs& d, const RepState* Yin, RepState* Xout, int prec, bool force_only,
