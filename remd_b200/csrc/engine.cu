@@ -89,6 +89,8 @@ struct remd_engine_s {
   double last_graph_ms = 0.0;       // host time of the last interval-graph capture + update/instantiate
   cudaMemPool_t mempool = nullptr;  // the pool comes from this memory pool (serving loop), else cudaMalloc
   int pinned_cap = 0;               // replicas the pinned host buffers hold
+  double* hstate = nullptr;         // pinned: one replica's state (remd_get_state), made at its first use
+  size_t hstate_words = 0;
   int2* d_carry_src = nullptr;      // per replica: {old first molecule, old replica} of a carried replica
   int* d_carry_ens = nullptr;       // per ensemble: old ensemble or -1
   int* d_ens_nrep = nullptr;        // per ensemble: replicas
@@ -1032,6 +1034,7 @@ remd_status remd_destroy(remd_handle h) {
   if (h->hT) cudaFreeHost(h->hT);
   if (h->hP) cudaFreeHost(h->hP);
   if (h->havg) cudaFreeHost(h->havg);
+  if (h->hstate) cudaFreeHost(h->hstate);
   for (auto& H : h->hist) {
     if (H.hist) cudaFree(H.hist);
     if (H.ave) cudaFree(H.ave);
@@ -1236,36 +1239,37 @@ remd_status remd_get_all_averages(remd_handle h, double* out) {
 
 remd_status remd_get_state(remd_handle h, int rep, remd_state_view* o) {
   if (!h || !o || rep < 0 || rep >= h->nrep) { set_error("remd_get_state: bad argument"); return REMD_ERR_INVALID; }
-  CK(cudaStreamSynchronize(h->stream));
   const RepConst& c = h->rc[rep];
-  const int n = c.nmol, N = h->N;
-  std::vector<double> tmp((size_t)n);
-  auto pull = [&](const double* src, int ncomp, double* dst) -> remd_status {
-    if (!dst) return REMD_OK;
-    for (int x = 0; x < ncomp; x++) {
-      CK(cudaMemcpy(tmp.data(), src + (size_t)x * N + c.mol_off, n * 8, cudaMemcpyDeviceToHost));
-      for (int i = 0; i < n; i++) dst[(size_t)ncomp * i + x] = tmp[i];
+  const size_t n = (size_t)c.nmol, words = kStateWords * n + kStateTail;
+  if (words > h->hstate_words) {   // pinned, sized for the handle's largest replica so far
+    if (h->hstate) cudaFreeHost(h->hstate);
+    h->hstate = nullptr;
+    h->hstate_words = 0;
+    if (cudaMallocHost(&h->hstate, words * sizeof(double)) != cudaSuccess) {
+      cudaGetLastError();
+      set_error("remd_get_state: pinned host allocation failed");
+      return REMD_ERR_OOM;
     }
-    return REMD_OK;
-  };
-  remd_status s;
-  if ((s = pull(h->d.r, 3, o->r)) != REMD_OK) return s;
-  if ((s = pull(h->d.v, 3, o->v)) != REMD_OK) return s;
-  if ((s = pull(h->d.q, 4, o->q)) != REMD_OK) return s;
-  if ((s = pull(h->d.p, 4, o->p)) != REMD_OK) return s;
-  if ((s = pull(h->d.f, 3, o->f)) != REMD_OK) return s;
-  if ((s = pull(h->d.n, 4, o->n)) != REMD_OK) return s;
+    h->hstate_words = words;
+  }
+  launch_gather_state(h->d, h->X, rep, c.nmol, h->hstate, h->stream);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(h->stream));
+  const double* src = h->hstate;
+  double* const dst[6] = {o->r, o->v, o->q, o->p, o->f, o->n};
+  for (int a = 0; a < 6; a++) {
+    const size_t len = ((a == 0 || a == 1 || a == 4) ? 3 : 4) * n;
+    if (dst[a]) std::memcpy(dst[a], src, len * sizeof(double));
+    src += len;
+  }
   RepState st;
-  CK(cudaMemcpy(&st, h->X + rep, sizeof(st), cudaMemcpyDeviceToHost));
+  std::memcpy(&st, src, sizeof(st));
+  src += sizeof(st) / sizeof(double);
   o->s = st.s; o->Ps = st.Ps; o->Q = c.Q; o->W = c.W;
   for (int x = 0; x < 3; x++) { o->Pv[x] = st.Pv[x]; o->L[x] = st.L[x]; }
   o->T = st.T; o->P = st.P; o->H0 = st.H0;
-  std::vector<Part2> p2(c.npart2);
-  CK(cudaMemcpy(p2.data(), h->d.part2 + c.part2_off, c.npart2 * sizeof(Part2), cudaMemcpyDeviceToHost));
-  double lj = 0, cl = 0, w = 0, v[3] = {0, 0, 0};
-  for (auto& p : p2) { lj += p.lj; cl += p.clmb; w += p.wall; for (int x = 0; x < 3; x++) v[x] += p.vir[x]; }
-  o->lj = lj * 0.5; o->clmb = cl * 0.5; o->wall = w;
-  for (int x = 0; x < 3; x++) o->vir[x] = v[x] * 0.5;
+  o->lj = src[0]; o->clmb = src[1]; o->wall = src[2];
+  for (int x = 0; x < 3; x++) o->vir[x] = src[3 + x];
   o->pot = o->lj + o->clmb + o->wall;
   return REMD_OK;
 }

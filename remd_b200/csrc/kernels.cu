@@ -2150,6 +2150,38 @@ void launch_noalloc_store(const DevPtrs& d, double* f_aos, double* n_aos, double
   k_noalloc_store<<<1, 256, 0, s>>>(d, f_aos, n_aos, out);
 }
 
+// ------------------------------------------------------------------ state read-back
+// The state of replica `rep` (remd_get_state) laid out as its caller wants it --
+// r, v (3 per molecule), q, p (4), f (3), n (4), molecule-major -- straight into
+// pinned host memory, followed by the replica's scalars and force sums, so that one
+// launch and one wait replace a copy per component (22 of them took 330 us).
+__global__ void k_gather_state(DevPtrs d, const RepState* __restrict__ X, int rep, double* __restrict__ out) {
+  const RepConst& c = d.rc[rep];
+  const int n = c.nmol, N = d.N, per = gridDim.x * blockDim.x;
+  const double* src[6] = {d.r, d.v, d.q, d.p, d.f, d.n};
+  long long off = 0;
+  for (int a = 0; a < 6; a++) {
+    const int m = (a == 0 || a == 1 || a == 4) ? 3 : 4;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m * n; k += per)
+      out[off + k] = src[a][(long long)(k % m) * N + c.mol_off + k / m];
+    off += (long long)m * n;
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    const P2Sum e = reduce_part2(d, c.part2_off, c.npart2);
+    if (threadIdx.x == 0) {
+      *reinterpret_cast<RepState*>(out + off) = X[rep];
+      double* s = out + off + sizeof(RepState) / sizeof(double);
+      s[0] = e.lj; s[1] = e.clmb; s[2] = e.wall;
+      s[3] = e.vir[0]; s[4] = e.vir[1]; s[5] = e.vir[2];
+    }
+  }
+}
+
+void launch_gather_state(const DevPtrs& d, const RepState* X, int rep, int nmol, double* out, cudaStream_t s) {
+  const int blocks = std::max(1, std::min((4 * nmol + 255) / 256, 64));
+  k_gather_state<<<blocks, 256, 0, s>>>(d, X, rep, out);
+}
+
 // ------------------------------------------------------------------ carrying replicas between handles
 // The serving loop's batch changes: replicas that keep running are copied from
 // the previous handle's arrays into the new handle's, on the device.

@@ -67,6 +67,11 @@ struct NoAllocSetup {
 void launch_noalloc_load(const DevPtrs& d, const NoAllocSetup& setup, RepState* X, const double* r_aos,
                          const double* q_aos, int tile, cudaStream_t s);
 void launch_noalloc_store(const DevPtrs& d, double* f_aos, double* n_aos, double* out, cudaStream_t s);
+// State of a replica as remd_get_state returns it, into pinned host memory:
+// kStateWords doubles per molecule, then RepState, then lj, clmb, wall, vir[3].
+constexpr int kStateWords = 21;
+constexpr int kStateTail = (int)(sizeof(RepState) / sizeof(double)) + 6;
+void launch_gather_state(const DevPtrs& d, const RepState* X, int rep, int nmol, double* out, cudaStream_t s);
 int measure_fp32_fma(int device, double* ms, long long* flops);
 int measure_atomics(int device, double* rates);
 // Copies carried replicas from handle arrays `o` into `d` (serving batch changes):
