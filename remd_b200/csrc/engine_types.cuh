@@ -6,16 +6,17 @@
 //     g = global molecule index = RepConst::mol_off + local index;
 //   * per-step force records ("pack"), rebuilt by the integrate kernel after
 //     the positions move: FP32 form = {int32 x,y,z fixed-point centre of mass,
-//     float site offsets R(q) b_k} padded to 16 B; FP64 form = {double box
-//     fraction, double site offsets};
-//   * full neighbour lists, uint16 local indices, column-major inside a force
-//     tile so that the lanes of a warp read consecutive words;
+//     float site offsets R(q) b_k} in 16-byte pieces, piece m of molecule g at
+//     m N + g (lanes with neighbouring molecules read neighbouring words);
+//     FP64 form = {double box fraction, double site offsets} by molecule;
+//   * full neighbour lists, uint16 local indices, a row per molecule (the
+//     molecule's eight lanes read consecutive words);
 //   * per-replica scalars (thermostat, barostat, box, H0, condition) in two
 //     buffers that the integrate and force kernels ping-pong between;
-//   * partial sums per 32 consecutive molecules of a replica (one warp),
-//     written by one kernel and reduced in molecule order by every CTA of the
-//     same replica in the next kernel (deterministic: a replica's result
-//     depends neither on its batch mates nor on the tile size).
+//   * partial sums per 32 (integrate) or kPart2Mol (forces) consecutive
+//     molecules of a replica, written by one kernel and reduced in a fixed order
+//     by every CTA of the same replica in the next kernel (deterministic: a
+//     replica's result depends neither on its batch mates nor on the tile size).
 #pragma once
 #include <cstdint>
 

@@ -229,7 +229,7 @@ struct StepCoef {
 // One MD step's integration.  It is bound by latency, not by throughput (a block's
 // FP64 scalar chain, then each molecule's): what a block needs -- the replica's
 // constants and scalars, the force partials -- is requested at once from the tile's
-// descriptor.  CHAIN: one more warp runs the scalar chain while the molecules' warps
+// descriptor (14.5 -> 11.8 us a launch at 64 molecules).  CHAIN: one more warp runs the scalar chain while the molecules' warps
 // load their state, into registers; for grids that leave room for the extra warp
 // (launch_integrate_prec).
 template <bool MID, bool CHAIN>
@@ -1063,8 +1063,9 @@ __device__ __forceinline__ void finish_group(const DevPtrs& d, const Const& c, i
 // FP32 form the pairs a lane sums depend on the positions only.  1/r is one rsqrt
 // (its square for 1/r^2) instead of a division and a square root per site pair.
 // With one lane per molecule and 128 molecules per block, 800 TIP4P molecules were
-// seven blocks, each thread walking a whole list: 224 us a launch; bound by FP64
-// latency then, and where the grid fills the GPU by the FP64 pipe.
+// seven blocks, each thread walking a whole list: 224 us a launch, now 22 us (5832
+// TIP3P molecules 468 -> 63 us); bound by FP64 latency, and where the grid fills the
+// GPU by the FP64 pipe.
 template <int S>
 struct F64Sums {
   double fs[S][3], fc[3], fv[3], lj, cl;
@@ -1438,7 +1439,8 @@ __device__ __forceinline__ void step_list(const DevPtrs& d, const PairBlk& b, co
 // warps hide the gathered loads' latency, which the pair kernel's four per
 // scheduler do not (the gather inside the pair kernel took 12 000 of a warp's
 // 43 000 cycles on 256 replicas, 111 432 molecules).  It is bound by the latency of
-// its loads, so all that need only the block's descriptor are issued together.
+// its loads, so all that need only the block's descriptor are issued together (75 us
+// on those 256 replicas, of which 25 us the rebuild of 14 of them).
 __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_lists(DevPtrs d, const RepState* __restrict__ X) {
   step_kernel_entry();
   extern __shared__ uint32_t bm[];
@@ -1485,8 +1487,14 @@ __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_list
   }
 }
 
-// FP32 form, second launch of a step: pair forces, wall, A2M of kPart2Mol
-// molecules per block, and their partial sums.
+// FP32 form, second launch of a step: pair forces and A2M of kPart2Mol molecules per
+// block, and their partial sums.  Bound by the issue of FP32 instructions: 67 % of the
+// issue slots and 47 % of the FMA pipe at four warps per scheduler (256 replicas,
+// 111 432 molecules: 228 us, 166 M warp instructions; with two threads per molecule
+// 267 us at 62 %), then by the latency of a warp's other phases (lists and constants
+// 6 000, exchange and A2M 4 200 of 37 000 cycles).  16 TIP5P replicas of 1728
+// molecules: 148 -> 142 us of pairs, 8 TIP4P replicas of 512: 47 -> 18 us.  128
+// registers for all models: 168 measured 2-4 % slower and 96 spills.
 template <int S, int C0, bool STD>
 __device__ void force_block_f32(const DevPtrs& d, const PairBlk& b, const PairConst& c, const F32Const& k32, int nc,
                                 double q4, double wf, double (*wsum)[8]) {
