@@ -247,10 +247,11 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     // pair kernel compiled for one model needs fewer registers and instructions
     // than the one for all), of about equal cost within a model
     // Eight chains while a quarter of the batch is no more than one wave of pair
-    // blocks (about 2400 blocks in all), else two: 8 replicas of 4096 molecules run
-    // 785 us a 10-step interval on four and 730 us on eight; 256 replicas, 111 432
-    // molecules, 3880 us on one, 3620 on two, 3680 on four, 3718 on eight.
-    const int K = std::min(npart2 <= 2400 ? kMaxChains : 2, h->nrep);
+    // blocks (about 2400 blocks in all), else four: 8 replicas of 4096 molecules run
+    // 785 us a 10-step interval on four and 730 us on eight.  256-replica batches on
+    // two / four / eight: 3611 / 3670 / 3718 us (111 432 molecules), 1136 / 1063 /
+    // 1108 and 2436 / 2390 / 2418 us (mixes of small tubes).
+    const int K = std::min(npart2 <= 2400 ? kMaxChains : 4, h->nrep);
     std::vector<double> rcost(h->nrep, 0.0);
     std::map<int, double> mcost;   // cost per model
     for (int r = 0; r < h->nrep; r++) {
