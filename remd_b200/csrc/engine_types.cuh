@@ -67,8 +67,8 @@ struct PairConst {
   long long nbr_off;
   float rc, rs, rc2, coef;     // switching: coef = 1/(rs-rc)^5
   float sgm2q, eps4, reach;    // sigma^2 / 4, 4 epsilon, site_reach
-  float uu;                    // square of the unit charge (that of the second charged site)
-  float q[kMaxSites];          // site charges in units of it
+  float uu;                    // standard charges (pair_model): square of the second charged site's
+  float qq[kMaxSites][kMaxSites];   // otherwise: products of the site charges
   float pad1;
   double body[kMaxSites][3];
 };

@@ -35,20 +35,20 @@ PairConst pair_const(const RepConst& c) {
   p.nbr_off = c.nbr_off;
   p.rc = (float)c.rc; p.rs = (float)c.rs; p.rc2 = (float)(c.rc * c.rc); p.coef = (float)c.coef_sw;
   p.sgm2q = (float)(0.25 * c.sgm2); p.eps4 = (float)(4.0 * c.eps); p.reach = (float)c.site_reach;
-  const double unit = c.qr[c.c0 + 1];
-  p.uu = (float)(unit * unit);
-  for (int k = c.c0; k < c.nsite; k++) p.q[k] = (float)(c.qr[k] / unit);
+  p.uu = (float)c.qq[c.c0 + 1][c.c0 + 1];
+  for (int k = 0; k < c.nsite; k++)
+    for (int l = 0; l < c.nsite; l++) p.qq[k][l] = (float)c.qq[k][l];
   for (int k = 0; k < kMaxSites; k++)
     for (int x = 0; x < 3; x++) p.body[k][x] = c.body[k][x];
   return p;
 }
 
 int pair_model(const RepConst& c) {
-  const PairConst p = pair_const(c);
-  const float* q = p.q;
-  const bool std_q = c.nsite == 3   ? (q[0] == -2.f && q[1] == 1.f && q[2] == 1.f)
-                     : c.nsite == 4 ? (q[1] == 1.f && q[2] == 1.f && q[3] == -2.f)
-                                    : (q[1] == 1.f && q[2] == 1.f && q[3] == -1.f && q[4] == -1.f);
+  const double* q = c.qr;
+  const auto is = [&](int k, int l, float ratio) { return (float)(q[k] / q[l]) == ratio; };
+  const bool std_q = c.nsite == 3   ? is(0, 1, -2.f) && is(2, 1, 1.f)
+                     : c.nsite == 4 ? is(2, 1, 1.f) && is(3, 1, -2.f)
+                                    : is(2, 1, 1.f) && is(3, 1, -1.f) && is(4, 1, -1.f);
   return c.nsite + (std_q ? kStdCharges : 0);
 }
 
@@ -766,20 +766,19 @@ __device__ __forceinline__ float two_rsqrt(float x) {
 }
 
 // Site charge in units of the second charged site's (the hydrogens of the water
-// models).  STD: the ratios of TIP3P {-2, 1, 1}, TIP4P {1, 1, -2} and TIP5P
-// {1, 1, -1, -1} are compile-time constants; otherwise they are read.
-template <int S, int C0, bool STD>
-__device__ __forceinline__ float charge_ratio(const PairConst& c, int k) {
-  if (!STD) return c.q[k];
-  if (S == 3) return k == 0 ? -2.f : 1.f;
-  if (S == 4) return k == 3 ? -2.f : 1.f;
-  return k >= 3 ? -1.f : 1.f;
+// models): TIP3P {-2, 1, 1}, TIP4P {1, 1, -2}, TIP5P {1, 1, -1, -1}.  Powers of two, so
+// that their products with the unit's square round as the charges' own would.
+template <int S>
+__device__ __forceinline__ constexpr float charge_ratio(int k) {
+  return S == 3 ? (k == 0 ? -2.f : 1.f) : S == 4 ? (k == 3 ? -2.f : 1.f) : (k >= 3 ? -1.f : 1.f);
 }
 
 // The lane's n pairs with molecule li: entries row[0], row[+-kGroup], ... (near
 // pairs, IMG, are stored backwards).  ci, si: li's fixed-point centre and site
-// offsets.  The Coulomb terms of site kk carry a factor 8 / (q_kk u^2), u the unit
-// charge, that the switch's factor takes back once per site.
+// offsets.  STD: the charges have the ratios of charge_ratio, and the Coulomb terms of
+// site kk carry a factor 8 / (q_kk u^2), u the unit charge, that the switch's factor
+// takes back once per site.  Other charges enter as their products, each rounded once
+// (in units of one of them they could overflow), with the factor 8 alone.
 template <int S, int C0, bool STD, bool IMG>
 __device__ __forceinline__ void pair_loop_f32(const DevPtrs& d, const PairConst& c, const F32Const& k32, int li,
                                               const int* ci, const float (*si)[3], const uint16_t* row, int n,
@@ -790,7 +789,7 @@ __device__ __forceinline__ void pair_loop_f32(const DevPtrs& d, const PairConst&
   const int N = d.N;
   const float Ls0 = k32.Ls[0], Ls1 = k32.Ls[1], Ls2 = k32.Ls[2];
   const float rc = c.rc, rs = c.rs, coef = c.coef;
-  const float uu = c.uu;
+  const float uu = STD ? c.uu : 1.f;
   constexpr int DIR = IMG ? -kGroup : kGroup;
   // the neighbour's record one pair ahead in registers, its index two pairs ahead
   // (2-5 % faster than loading the record at the top of its own iteration)
@@ -873,7 +872,7 @@ __device__ __forceinline__ void pair_loop_f32(const DevPtrs& d, const PairConst&
           fpx = f * x; fpy = f * y; fpz = f * z;
         }
         if (cl_pair) {
-          const float e = charge_ratio<S, C0, STD>(c, l) * ri;
+          const float e = (STD ? charge_ratio<S>(l) : c.qq[kk][l]) * ri;
           ek += e;
           const float f = e * p;
           tx = fmaf(f, x, tx); ty = fmaf(f, y, ty); tz = fmaf(f, z, tz);
@@ -881,7 +880,7 @@ __device__ __forceinline__ void pair_loop_f32(const DevPtrs& d, const PairConst&
       }
       if (kk >= C0) {
         // switch, charge and unit once per site (FFMA into the sums)
-        const float qk = charge_ratio<S, C0, STD>(c, kk);
+        const float qk = STD ? charge_ratio<S>(kk) : 1.f;
         ecl = fmaf(qk, ek, ecl);
         const float w = swu * qk;
         a.fs[kk][0] = fmaf(w, tx, a.fs[kk][0]);

@@ -61,6 +61,17 @@ def test_charges_other_than_the_water_models_ratios(model):
     _check(spec, e.states[0], "fp32")
 
 
+@pytest.mark.parametrize("model,charges", [("tip3p", (-0.834, 1e-24, 0.834)), ("tip4p", (0.0, 0.52, 1e-24, -0.52)),
+                                           ("tip5p", (0.0, 0.241, 1e-24, -0.12, -0.121))])
+def test_charges_far_apart(model, charges):
+    """A charged site that is switched off by a tiny charge (a zero is refused): no
+    charge may be taken in units of another, their ratio's square overflows."""
+    e = S.make_ensemble("far", model, 0, 512, 0.0, 10.0, 9.0, 1, 1, 300, 300, 0.1e6, 0.1e6, 321)
+    spec = copy.deepcopy(e.spec)
+    spec.moltype.charge[:] = charges
+    _check(spec, e.states[0], "fp32")
+
+
 def test_fp64_form_with_cell_lists():
     """A tube long enough to be cut into cells: the FP64 form takes the list rebuild
     of the FP32 form and tests its entries in FP64."""
