@@ -40,6 +40,18 @@ using namespace remd;
 
 constexpr int kMaxChains = 8;   // independent chains of the interval graph
 
+// Makes a device current for a scope and then gives the thread its own back: launches
+// and new streams go to the current device, whatever device the handle is on.
+struct DeviceScope {
+  int before = -1;
+  bool ok;
+  explicit DeviceScope(int device) {
+    ok = cudaGetDevice(&before) == cudaSuccess && (before == device || cudaSetDevice(device) == cudaSuccess);
+    if (before == device) before = -1;
+  }
+  ~DeviceScope() { if (before >= 0) cudaSetDevice(before); }
+};
+
 struct remd_engine_s {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -549,6 +561,8 @@ static void launch_step_integrate(remd_engine_s* h, int s) {
 }
 
 static remd_status build_graph(remd_engine_s* h) {
+  const DeviceScope on(h->device);   // the chains' streams are the device's
+  if (!on.ok) { set_error("graph capture: cannot use the handle's device"); return REMD_ERR_CUDA; }
   cudaGraph_t g;
   if (!h->vscale)   // the chains' streams, when first needed
     for (int k = 0; k < h->nchain - 1; k++) {
@@ -1240,6 +1254,8 @@ remd_status remd_get_all_averages(remd_handle h, double* out) {
 
 remd_status remd_get_state(remd_handle h, int rep, remd_state_view* o) {
   if (!h || !o || rep < 0 || rep >= h->nrep) { set_error("remd_get_state: bad argument"); return REMD_ERR_INVALID; }
+  const DeviceScope on(h->device);
+  if (!on.ok) { set_error("remd_get_state: cannot use the handle's device"); return REMD_ERR_CUDA; }
   const RepConst& c = h->rc[rep];
   const size_t n = (size_t)c.nmol, words = kStateWords * n + kStateTail;
   if (words > h->hstate_words) {   // pinned, sized for the handle's largest replica so far

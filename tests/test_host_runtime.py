@@ -1,0 +1,64 @@
+"""The engine's host code on the CPU, against a stand-in for the CUDA runtime
+(fake_runtime.cpp) that records what the host asks for: launches, streams, pinned
+buffers, graphs.  It has two devices, which a one-GPU machine does not."""
+import ctypes as C
+import glob
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from remd_b200 import engine as E
+from remd_b200 import systems as S
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    """The engine linked against the stand-in, in place of the engine library."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no CUDA headers")
+    E.build_library()
+    out = str(tmp_path_factory.mktemp("fake") / "libremd_fake.so")
+    objects = [o for o in sorted(glob.glob(os.path.join(os.path.dirname(E.__file__), "csrc", "_build", "*.o")))]
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-o", out,
+                    "-I" + os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include"),
+                    os.path.join(HERE, "fake_runtime.cpp"), *objects, "-lpthread", "-ldl", "-lrt"], check=True)
+    kept = E._LIB, E.LIB_PATH
+    E._LIB, E.LIB_PATH = None, out
+    L = E.lib()
+    L.fake_launch.restype = C.c_char_p
+    L.fake_count.restype = C.c_long
+    yield L
+    E._LIB, E.LIB_PATH = kept
+
+
+@pytest.fixture(autouse=True)
+def device_zero(fake):
+    fake.cudaSetDevice(0)
+    fake.fake_reset()
+
+
+def _grid(nmol, nrep, model="tip4p", confined=0, interval=3, wall=7.0):
+    e = S.small_ensemble(model, confined, nmol=nmol, ntemp=nrep, npress=1, seed=5, interval=interval, wall=wall)
+    return e
+
+
+def test_state_is_read_whatever_device_is_current(fake):
+    """The copies of an earlier read-back worked whatever device was current; a kernel
+    launch does only with the stream's own."""
+    eng = E.REMDGPU([_grid(64, 2)], device=0)
+    other = E.REMDGPU([_grid(64, 1)], device=1)   # leaves device 1 current
+    eng.ConvertVariablesToHost(1)
+    now = C.c_int(-1)
+    fake.cudaGetDevice(C.byref(now))
+    assert now.value == 1   # the caller's device is left as it was
+    fake.cudaSetDevice(0)   # as on a host thread that never chose a device
+    other.ConvertVariablesToHost(0)
+    fake.cudaGetDevice(C.byref(now))
+    assert now.value == 0
+    eng.close(), other.close()
