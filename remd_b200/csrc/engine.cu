@@ -102,7 +102,6 @@ struct remd_engine_s {
   cudaMemPool_t mempool = nullptr;  // the pool comes from this memory pool (serving loop), else cudaMalloc
   int pinned_cap = 0;               // replicas the pinned host buffers hold
   double* hstate = nullptr;         // pinned: one replica's state (remd_get_state), made at its first use
-  size_t hstate_words = 0;
   int2* d_carry_src = nullptr;      // per replica: {old first molecule, old replica} of a carried replica
   int* d_carry_ens = nullptr;       // per ensemble: old ensemble or -1
   int* d_ens_nrep = nullptr;        // per ensemble: replicas
@@ -1257,17 +1256,16 @@ remd_status remd_get_state(remd_handle h, int rep, remd_state_view* o) {
   const DeviceScope on(h->device);
   if (!on.ok) { set_error("remd_get_state: cannot use the handle's device"); return REMD_ERR_CUDA; }
   const RepConst& c = h->rc[rep];
-  const size_t n = (size_t)c.nmol, words = kStateWords * n + kStateTail;
-  if (words > h->hstate_words) {   // pinned, sized for the handle's largest replica so far
-    if (h->hstate) cudaFreeHost(h->hstate);
-    h->hstate = nullptr;
-    h->hstate_words = 0;
-    if (cudaMallocHost(&h->hstate, words * sizeof(double)) != cudaSuccess) {
+  const size_t n = (size_t)c.nmol;
+  if (!h->hstate) {   // pinned, for the handle's largest replica
+    size_t largest = 0;
+    for (const RepConst& x : h->rc) largest = std::max(largest, (size_t)x.nmol);
+    if (cudaMallocHost(&h->hstate, (kStateWords * largest + kStateTail) * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
+      h->hstate = nullptr;
       set_error("remd_get_state: pinned host allocation failed");
       return REMD_ERR_OOM;
     }
-    h->hstate_words = words;
   }
   launch_gather_state(h->d, h->X, rep, c.nmol, h->hstate, h->stream);
   CK(cudaGetLastError());

@@ -62,3 +62,14 @@ def test_state_is_read_whatever_device_is_current(fake):
     fake.cudaGetDevice(C.byref(now))
     assert now.value == 0
     eng.close(), other.close()
+
+
+def test_read_back_buffer_is_made_once(fake):
+    """One pinned buffer for the handle's largest replica, also where replicas are read
+    from the smallest to the largest."""
+    eng = E.REMDGPU([_grid(n, 1) for n in (64, 100, 200)])
+    fake.fake_reset()
+    for k in range(3):
+        eng.ConvertVariablesToHost(k)
+    assert fake.fake_count(b"host_allocs") == 1
+    eng.close()
