@@ -202,6 +202,30 @@ static remd_status check_desc(const remd_system_desc& s, std::string& why) {
   return REMD_OK;
 }
 
+// Estimated neighbours of a molecule within rcut at liquid density: a sphere, in a tube
+// or a slit no more than the tube's or slit's part within rcut along it.
+static double neighbours(const RepConst& c) {
+  const double density = 0.0334;   // molecules per A^3
+  double vol = 4.0 / 3.0 * M_PI * c.rc * c.rc * c.rc;
+  if (c.confined == 1) vol = std::min(vol, 2.0 * c.rc * c.bottom_area);
+  if (c.confined == 2) vol = std::min(vol, M_PI * c.rc * c.rc * std::max(c.slit_width - 1.7, 0.0));
+  return std::min((double)(c.nmol - 1), density * vol);
+}
+
+// Programmatic launch of the step kernels (launch_step_kernel) pays while a step's pair
+// kernels are short, up to about 4500 pairs per SM in all: the next kernel's blocks are
+// scheduled early and wait on SMs that would idle.  Above, they hold slots that the
+// other chains' kernels would use.  Interval times with it / without: 16 replicas of 128
+// tube molecules (430 pairs per SM) 1087 / 1162 us, 4 x 2000 tube molecules (3200) 350 /
+// 378, 8 x 512 bulk molecules (3900) 389 / 402, 64 x 200 tube molecules (4300) 421 /
+// 431; 4096 bulk molecules (5200) 498 / 474, FP64 8 x 729 (5500) 566 / 549, 16 x 512 bulk
+// (7800) 496 / 487, 64 x 512 slit (19000) 1850 / 1636, 64 x 729 bulk (44000) 1580 / 1437.
+static bool programmatic_steps(const remd_engine_s* h) {
+  double pairs = 0.0;
+  for (const RepConst& c : h->rc) pairs += c.nmol * neighbours(c);
+  return pairs <= 4500.0 * sm_count();
+}
+
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Build RepConst/tiles for the current tile size; returns pool layout size.
@@ -246,9 +270,8 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     std::vector<double> cost(h->tiles.size());
     for (size_t t = 0; t < h->tiles.size(); t++) {
       const RepConst& c = h->rc[h->tiles[t].rep];
-      const double nbr = std::min((double)(c.nmol - 1), 0.0334 * 4.0 / 3.0 * M_PI * c.rc * c.rc * c.rc);
       const int nq = c.nsite - c.c0;
-      cost[t] = h->tiles[t].count * nbr * (51.0 + 32.0 + 27.0 * nq * nq);
+      cost[t] = h->tiles[t].count * neighbours(c) * (51.0 + 32.0 + 27.0 * nq * nq);
     }
     h->order.resize(h->tiles.size());
     for (size_t t = 0; t < h->order.size(); t++) h->order[t] = (int)t;
@@ -470,6 +493,8 @@ static remd_status allocate(remd_engine_s* h) {
   h->d_reps2 = reinterpret_cast<int*>(b + offs[45]);
   d.reps = nullptr;
   d.nrep_l = h->nrep;
+  d.pdl = programmatic_steps(h);
+  d.ntiles_h = d.ntiles;
   d.model_l = common_model(h, nullptr, h->nrep);
   {
     int nmax = 1;

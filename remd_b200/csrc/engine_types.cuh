@@ -160,6 +160,8 @@ struct DevPtrs {
   const PairConst* pc;           // FP32 form, per replica
   const PairBlk* pblk;           // list and pair blocks, costliest first
   int npblk;                     // pair blocks of a launch
+  int pdl;                       // the step's launches are programmatic (launch_step_kernel)
+  int ntiles_h;                  // tiles of all chains of the handle
   int model_l;                   // sites of every replica of a launch (0 when they differ) + kStdCharges
   const int* reps;               // replicas of a launch of the replica head (NULL: all)
   int nrep_l;                    // their number

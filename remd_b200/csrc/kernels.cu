@@ -2256,7 +2256,7 @@ void launch_carry(const DevPtrs& d, const DevPtrs& o, int tile, const int2* src,
 void launch_pack(const DevPtrs& d, int prec, int tile, cudaStream_t s) {
   k_pack<<<d.ntiles, tile, 0, s>>>(d, prec);
 }
-static int sm_count() {
+int sm_count() {
   static int n[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -2265,14 +2265,8 @@ static int sm_count() {
   return n[dev];
 }
 
-// A step kernel (it calls step_kernel_entry first).  With `pdl` it is launched
-// with programmatic stream serialisation.  That pays where a step's tile grid
-// is smaller than the GPU (one block per SM or fewer): the launches are
-// latency-bound and the early-scheduled blocks wait on otherwise idle SMs
-// (16 replicas of 128 TIP4P molecules: 55 -> 58.5 M mol-steps/s).  Where the
-// grid fills the GPU, the waiting blocks hold slots that the other chains of
-// the interval graph would use (256 replicas, 111 432 molecules: 288 -> 253 M
-// with it), so those launches are plain.
+// A step kernel (it calls step_kernel_entry first).  With `pdl` (DevPtrs::pdl, the
+// engine's rule) it is launched with programmatic stream serialisation.
 template <typename... KArgs, typename... Args>
 static void launch_step_kernel(bool pdl, void (*k)(KArgs...), unsigned grid, unsigned block, size_t smem,
                                cudaStream_t s, Args... args) {
@@ -2291,13 +2285,16 @@ static void launch_step_kernel(bool pdl, void (*k)(KArgs...), unsigned grid, uns
 
 void launch_integrate_prec(const DevPtrs& d, const RepState* X, RepState* Y, bool mid, int tile,
                            int prec, cudaStream_t s) {
-  const bool pdl = d.ntiles <= sm_count();
-  // the chain's own warp where every block of the launch is resident with it
-  const bool chain = (long long)d.ntiles * (tile + 32) <= (long long)sm_count() * 3 * 160;
+  // the scalar chain's own warp where the blocks of all the handle's chains, which run
+  // side by side, are resident with it: 16 replicas of 128 molecules 1161 us a 50-step
+  // interval with it and 1208 without; 96 replicas of 729 molecules (2208 tiles) 2785 us
+  // a 10-step interval with it and 2741 without, 256 replicas (111 432 molecules) 3299
+  // and 3239
+  const bool chain = (long long)d.ntiles_h * (tile + 32) <= (long long)sm_count() * 3 * 160;
   void (*k)(DevPtrs, const RepState*, RepState*, int) =
       chain ? (mid ? k_integrate<true, true> : k_integrate<false, true>)
             : (mid ? k_integrate<true, false> : k_integrate<false, false>);
-  launch_step_kernel(pdl, k, d.ntiles, tile + (chain ? 32 : 0), 0, s, d, X, Y, prec);
+  launch_step_kernel(d.pdl, k, d.ntiles, tile + (chain ? 32 : 0), 0, s, d, X, Y, prec);
 }
 int max_force_tile(int prec) { return prec == kF32 ? 64 : 128; }
 
@@ -2314,7 +2311,7 @@ static_assert(kPart2Mol * (kBitmapMaxWords + 1) * 4 <= 8192, "rebuild bitmaps");
 static void launch_force_impl(const DevPtrs& d, const RepState* Yin, RepState* Xout, int prec, bool force_only,
                               int tile, cudaStream_t s, cudaEvent_t e_head, cudaEvent_t e_lists) {
   const RepState* Xc = Xout;
-  const bool pdl = d.ntiles <= sm_count();   // the step's tile grid (see launch_step_kernel)
+  const bool pdl = d.pdl;
   if (force_only) launch_step_kernel(pdl, k_replica_head<true>, d.nrep_l, kRepThreads, 0, s, d, Yin, Xout);
   else launch_step_kernel(pdl, k_replica_head<false>, d.nrep_l, kRepThreads, 0, s, d, Yin, Xout);
   if (e_head) cudaEventRecord(e_head, s);

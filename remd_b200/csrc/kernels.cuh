@@ -52,6 +52,8 @@ void launch_exchange_k(const DevPtrs& d, const int* grid, const int* rep_off, co
 void launch_histogram(const DevPtrs& d, const HistEns* he, const int* rep_off, const int* index,
                       cudaStream_t s);
 int pack_stride(int nsite, int prec);
+// SMs of the current device.
+int sm_count();
 // The FP32 pair step's constants of a replica, and the kStdCharges / nsite code of its model.
 PairConst pair_const(const RepConst& c);
 int pair_model(const RepConst& c);

@@ -231,6 +231,8 @@ extern "C" remd_status remd_force_snapshot_noalloc(const remd_system_desc* s, co
   d.cell_start = reinterpret_cast<int*>(b + kOffCellStart);
   d.cell_com = reinterpret_cast<int4*>(b + kOffCellMol);
   d.nrep_l = 1;
+  d.pdl = 1;   // one replica, one stream: nothing else wants the waiting blocks' slots
+  d.ntiles_h = c.ntile;
   d.model_l = pair_model(c);
   d.pc = reinterpret_cast<PairConst*>(b + kOffPairC);
   d.pblk = reinterpret_cast<PairBlk*>(b + kOffPblk);

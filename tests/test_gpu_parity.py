@@ -185,10 +185,10 @@ def test_batch_equals_alone_bitwise():
 
 
 def test_dependent_launch_and_plain_launch_agree_bitwise():
-    """A step whose tile grid is no larger than the SM count is launched with
-    programmatic stream serialisation, a larger one plainly.  A small ensemble
-    alone (dependent launches) and the same ensemble inside a batch of more than
-    148 tiles per interval-graph chain (plain launches) give the same bits."""
+    """The steps of a handle with little pair work are launched with programmatic
+    stream serialisation, those of a larger one plainly.  A small ensemble alone
+    (dependent launches) and the same ensemble inside a batch of some 3 million
+    pairs (plain launches) give the same bits."""
     small = S.small_ensemble("tip4p", 0, nmol=70, ntemp=2, npress=1, seed=34, interval=10)
     filler = S.make_ensemble("filler", "tip3p", 0, 512, 0.0, 9.0, 8.0, 16, 4, 250, 350, 0.1e6, 0.1e6, 35,
                              interval=10)
@@ -197,7 +197,7 @@ def test_dependent_launch_and_plain_launch_agree_bitwise():
     alone.ExecuteSteps(small.T, small.P)
     both = E.REMDGPU([small, filler], precision="fp32")
     both.set_tuning(32, 1.0)
-    assert filler.nreplica * 16 // 4 > 148   # 512 molecules = 16 tiles of 32, over four chains
+    assert filler.nreplica * 512 * 100 > 2 * 4500 * 148   # pairs within 9 A, the rule's bound at 148 SMs
     both.ExecuteSteps(np.concatenate([small.T, filler.T]), np.concatenate([small.P, filler.P]))
     for r in range(small.nreplica):
         assert np.array_equal(alone.GetAverages(r), both.GetAverages(r))

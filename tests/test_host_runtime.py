@@ -73,3 +73,43 @@ def test_read_back_buffer_is_made_once(fake):
         eng.ConvertVariablesToHost(k)
     assert fake.fake_count(b"host_allocs") == 1
     eng.close()
+
+
+def _launches(fake):
+    """(kernel, grid, block, programmatic, stream) of every launch since the last reset."""
+    g, b, p, s = C.c_int(), C.c_int(), C.c_int(), C.c_int()
+    out = []
+    for k in range(fake.fake_count(b"launches")):
+        name = fake.fake_launch(k, C.byref(g), C.byref(b), C.byref(p), C.byref(s)).decode()
+        out.append((name, g.value, b.value, p.value, s.value))
+    return out
+
+
+def _interval(fake, eng):
+    """The launches of one more interval."""
+    fake.fake_reset()
+    eng.ExecuteSteps(eng.T, eng.P)
+    return _launches(fake)
+
+
+def _steps(launches):
+    return [x for x in launches if any(k in x[0] for k in ("k_integrate", "k_replica_head", "k_force"))]
+
+
+@pytest.mark.parametrize("nmol,nrep,expected", [(128, 16, 1), (512, 8, 1), (512, 16, 0), (512, 64, 0), (900, 64, 0)])
+def test_programmatic_launch_follows_the_work_of_all_chains(fake, nmol, nrep, expected):
+    """Chains run side by side: what one chain launches programmatically must depend on
+    the work of all of them, not on how many chains share it."""
+    eng = E.REMDGPU([_grid(nmol, nrep)])
+    steps = _steps(_interval(fake, eng))
+    assert len(steps) >= 3 * 4 and all(x[3] == expected for x in steps)
+    eng.close()
+
+
+@pytest.mark.parametrize("nmol,nrep,extra", [(128, 16, 32), (729, 96, 0)])
+def test_chain_warp_only_where_all_chains_leave_room(fake, nmol, nrep, extra):
+    """The integrate kernel's extra warp: 2208 tiles of 64 threads are more than the GPU
+    holds at once, however they are split over chains."""
+    eng = E.REMDGPU([_grid(nmol, nrep)])
+    assert all(x[2] == 32 + extra for x in _interval(fake, eng) if "k_integrate" in x[0])
+    eng.close()
