@@ -277,9 +277,9 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     for (size_t t = 0; t < h->order.size(); t++) h->order[t] = (int)t;
     std::stable_sort(h->order.begin(), h->order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     // groups of whole replicas for the independent chains of the interval graph:
-    // each of one water model where there are no more models than chains (the
-    // pair kernel compiled for one model needs fewer registers and instructions
-    // than the one for all), of about equal cost within a model
+    // each of one water model (there are at most three; the pair kernel compiled for
+    // one model needs fewer registers and instructions than the one for all), of
+    // about equal cost within a model
     // Eight chains while a quarter of the batch is no more than one wave of pair
     // blocks (about 2400 blocks in all), else four: 8 replicas of 4096 molecules run
     // 785 us a 10-step interval on four and 730 us on eight.  256-replica batches on
@@ -294,20 +294,14 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     }
     std::map<int, int> mchains, mreps;   // chains and replicas per model
     for (int r = 0; r < h->nrep; r++) mreps[h->rc[r].nsite]++;
-    if ((int)mcost.size() > K) {
-      double all = 0.0;
-      for (auto& m : mcost) all += m.second;
-      mcost = {{-1, all}};
-      mreps = {{-1, h->nrep}};
-    }
     for (auto& m : mcost) mchains[m.first] = 1;
     for (int left = K - (int)mcost.size(); left > 0; left--) {   // to the model whose chains are costliest
-      int best = -2;
+      int best = -1;
       for (auto& m : mcost)
         if (mchains[m.first] < mreps[m.first] &&
-            (best == -2 || m.second / mchains[m.first] > mcost[best] / mchains[best]))
+            (best == -1 || m.second / mchains[m.first] > mcost[best] / mchains[best]))
           best = m.first;
-      if (best == -2) break;
+      if (best == -1) break;
       mchains[best]++;
     }
     h->reps2.clear();
@@ -320,7 +314,7 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
       double run = 0.0;
       int k = 0, used = 0, in_chain = 0, seen = 0;
       for (int r = 0; r < h->nrep; r++) {
-        if (m.first != -1 && h->rc[r].nsite != m.first) continue;
+        if (h->rc[r].nsite != m.first) continue;
         const int left_reps = mreps[m.first] - seen, left_chains = mchains[m.first] - k;
         if (in_chain > 0 && k + 1 < mchains[m.first] &&
             (run + 0.5 * rcost[r] > m.second * (k + 1) / mchains[m.first] || left_reps < left_chains)) {
@@ -562,7 +556,7 @@ static remd_status upload_state(remd_engine_s* h, const std::vector<double>& r, 
 
 static remd_status initial_force(remd_engine_s* h) {
   launch_pack(h->d, h->prec, h->tile, h->stream);
-  launch_force(h->d, h->X, h->X, h->prec, true, h->tile, h->stream);
+  launch_force(h->d, h->X, h->X, h->prec, true, h->stream);
   launch_replica_props(h->d, h->X, h->stream);
   CK(cudaGetLastError());
   return sync_and_check(h);
@@ -617,7 +611,7 @@ static remd_status build_graph(remd_engine_s* h) {
       for (int k = 0; k < h->nchain; k++) {
         cudaStream_t st = k ? h->stream2[k - 1] : h->stream;
         launch_integrate_prec(dg[k], h->X, h->Y, s > 0, h->tile, h->prec, st);
-        launch_force(dg[k], h->Y, h->X, h->prec, false, h->tile, st);
+        launch_force(dg[k], h->Y, h->X, h->prec, false, st);
       }
     for (int k = 1; k < h->nchain; k++) {
       cudaEventRecord(h->ev_join[k - 1], h->stream2[k - 1]);
@@ -626,7 +620,7 @@ static remd_status build_graph(remd_engine_s* h) {
   } else {
     for (int s = 0; s < h->interval; s++) {
       launch_step_integrate(h, s);
-      launch_force(h->d, h->Y, h->X, h->prec, false, h->tile, h->stream);
+      launch_force(h->d, h->Y, h->X, h->prec, false, h->stream);
     }
   }
   launch_replica_end(h->d, h->X, h->stream);
@@ -760,7 +754,7 @@ static remd_status carry_in(remd_engine_s* h, const Carry* cy) {
   };
   carry(true);
   launch_pack(h->d, h->prec, h->tile, h->stream);
-  launch_force(h->d, h->X, h->X, h->prec, true, h->tile, h->stream);
+  launch_force(h->d, h->X, h->X, h->prec, true, h->stream);
   launch_replica_props(h->d, h->X, h->stream);
   carry(false);
   CK(cudaGetLastError());
@@ -1151,7 +1145,7 @@ static remd_status relayout(remd_engine_s* h, int tile, double skin, const Saved
   CK(cudaMemcpy(h->d_seed, sv.seed.data(), sv.seed.size() * 8, cudaMemcpyHostToDevice));
   // forces are a pure function of positions: recompute, keep H0
   launch_pack(h->d, h->prec, h->tile, h->stream);
-  launch_force(h->d, h->X, h->X, h->prec, true, h->tile, h->stream);
+  launch_force(h->d, h->X, h->X, h->prec, true, h->stream);
   CK(cudaGetLastError());
   return sync_and_check(h);
 }
@@ -1247,7 +1241,7 @@ remd_status remd_execute_nsteps(remd_handle h, int nsteps) {
   launch_replica_start(h->d, h->X, h->stream);
   for (int s = 0; s < nsteps; s++) {
     launch_step_integrate(h, s);
-    launch_force(h->d, h->Y, h->X, h->prec, false, h->tile, h->stream);
+    launch_force(h->d, h->Y, h->X, h->prec, false, h->stream);
   }
   launch_replica_end(h->d, h->X, h->stream);
   CK(cudaGetLastError());
@@ -1317,7 +1311,7 @@ remd_status remd_get_state(remd_handle h, int rep, remd_state_view* o) {
 remd_status remd_compute_forces(remd_handle h) {
   if (!h) return REMD_ERR_INVALID;
   launch_pack(h->d, h->prec, h->tile, h->stream);
-  launch_force(h->d, h->X, h->X, h->prec, true, h->tile, h->stream);
+  launch_force(h->d, h->X, h->X, h->prec, true, h->stream);
   CK(cudaGetLastError());
   remd_status s = sync_and_check(h);
   h->last_pairs = host_pairs(h);
@@ -1367,7 +1361,7 @@ remd_status remd_profile_steps(remd_handle h, int nsteps, double* ms_out) {
     CK(cudaEventRecord(ev[0], h->stream));
     launch_step_integrate(h, s);
     CK(cudaEventRecord(ev[1], h->stream));
-    launch_force(h->d, h->Y, h->X, h->prec, false, h->tile, h->stream);
+    launch_force(h->d, h->Y, h->X, h->prec, false, h->stream);
     CK(cudaEventRecord(ev[2], h->stream));
     CK(cudaEventSynchronize(ev[2]));
     float a = 0.f, b = 0.f;
@@ -1394,7 +1388,7 @@ remd_status remd_profile_split(remd_handle h, int nsteps, double* ms_out) {
     CK(cudaEventRecord(ev[0], h->stream));
     launch_step_integrate(h, s);
     CK(cudaEventRecord(ev[1], h->stream));
-    launch_force_timed(h->d, h->Y, h->X, h->prec, h->tile, h->stream, ev[2], ev[3]);
+    launch_force_timed(h->d, h->Y, h->X, h->prec, h->stream, ev[2], ev[3]);
     CK(cudaEventRecord(ev[4], h->stream));
     CK(cudaEventSynchronize(ev[4]));
     for (int k = 0; k < 4; k++) {

@@ -959,7 +959,6 @@ __device__ __forceinline__ void reduce_sums(const F32Sums<S>& a, int sub, double
 #pragma unroll
     for (int x = 0; x < 3; x++) {
       // slots k (lower half) and k + 4: exchanged in FP32, added in FP64
-      if (k >= S && k + 4 < 5) { v[3 * k + x] = 0.0; continue; }
       const float lo = a.at(k, x), hi = a.at(k + 4, x);
       const float give = up ? lo : hi, keep = up ? hi : lo;
       v[3 * k + x] = (double)keep + (double)__shfl_xor_sync(0xffffffffu, give, 4);
@@ -2309,7 +2308,7 @@ static_assert(kPart2Mol * (kBitmapMaxWords + 1) * 4 <= 8192, "rebuild bitmaps");
 // The force launches of one step; e_head / e_lists (may be null) are recorded
 // after the head and after the list kernel (profiling: remd_profile_split).
 static void launch_force_impl(const DevPtrs& d, const RepState* Yin, RepState* Xout, int prec, bool force_only,
-                              int tile, cudaStream_t s, cudaEvent_t e_head, cudaEvent_t e_lists) {
+                              cudaStream_t s, cudaEvent_t e_head, cudaEvent_t e_lists) {
   const RepState* Xc = Xout;
   const bool pdl = d.pdl;
   if (force_only) launch_step_kernel(pdl, k_replica_head<true>, d.nrep_l, kRepThreads, 0, s, d, Yin, Xout);
@@ -2341,13 +2340,13 @@ static void launch_force_impl(const DevPtrs& d, const RepState* Yin, RepState* X
 }
 
 void launch_force(const DevPtrs& d, const RepState* Yin, RepState* Xout, int prec, bool force_only,
-                  int tile, cudaStream_t s) {
-  launch_force_impl(d, Yin, Xout, prec, force_only, tile, s, nullptr, nullptr);
+                  cudaStream_t s) {
+  launch_force_impl(d, Yin, Xout, prec, force_only, s, nullptr, nullptr);
 }
 
-void launch_force_timed(const DevPtrs& d, const RepState* Yin, RepState* Xout, int prec, int tile, cudaStream_t s,
+void launch_force_timed(const DevPtrs& d, const RepState* Yin, RepState* Xout, int prec, cudaStream_t s,
                         cudaEvent_t e_head, cudaEvent_t e_lists) {
-  launch_force_impl(d, Yin, Xout, prec, false, tile, s, e_head, e_lists);
+  launch_force_impl(d, Yin, Xout, prec, false, s, e_head, e_lists);
 }
 void launch_replica_start(const DevPtrs& d, RepState* X, cudaStream_t s) {
   k_replica_start<<<d.nrep, kRepThreads, 0, s>>>(d, X);

@@ -245,7 +245,7 @@ extern "C" remd_status remd_force_snapshot_noalloc(const remd_system_desc* s, co
   // / partial sums by the kernels after it (the load kernel also marks the lists
   // invalid, so they are rebuilt)
   launch_noalloc_load(d, setup, X, d_r, d_q, kNoAllocTile, cs);
-  launch_force(d, X, X, kF32, true, kNoAllocTile, cs);
+  launch_force(d, X, X, kF32, true, cs);
   launch_noalloc_store(d, d_f, d_n, d_out, cs);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
