@@ -38,7 +38,21 @@ using namespace remd;
     }                                                                              \
   } while (0)
 
-constexpr int kMaxChains = 8;   // independent chains of the interval graph
+constexpr int kChains = 4;      // independent chains of a handle's first interval graph
+constexpr int kMaxChains = 8;   // of its second one (remd_engine_s::wide)
+constexpr int kWidenAfter = 32; // intervals on the first one
+
+// The handle's replicas cut into independent chains: chain k's replicas are reps[rep[k]
+// .. rep[k+1]), its tiles (costliest first) order[tile[k] .. tile[k+1]), its list and
+// pair blocks blk[pblk[k] .. pblk[k+1]).
+struct Chains {
+  int n = 1;
+  int tile[kMaxChains + 1] = {}, rep[kMaxChains + 1] = {}, pblk[kMaxChains + 1] = {};
+  std::vector<int> order, reps;
+  std::vector<PairBlk> blk;
+  int *d_order = nullptr, *d_reps = nullptr;
+  PairBlk* d_blk = nullptr;
+};
 
 // Makes a device current for a scope and then gives the thread its own back: launches
 // and new streams go to the current device, whatever device the handle is on.
@@ -66,16 +80,11 @@ struct remd_engine_s {
   std::vector<RepConst> rc;
   std::vector<Tile> tiles;
   std::vector<int> order;          // force blocks -> tiles, costliest first
-  std::vector<int> order2;         // the same per chain: chain k's tiles [chain_tile[k], chain_tile[k+1])
-  int nchain = 1;                  // independent chains of the interval graph
-  int chain_tile[kMaxChains + 1] = {};
-  std::vector<int> reps2;          // replicas by chain: chain k's are reps2[chain_rep[k] .. chain_rep[k+1])
-  int chain_rep[kMaxChains + 1] = {};
-  int* d_reps2 = nullptr;
-  int* d_order2 = nullptr;
-  std::vector<PairBlk> pblk, pblk2;   // FP32 form: list and pair blocks in the order of `order`, `order2`
-  int chain_pblk[kMaxChains + 1] = {};
-  PairBlk* d_pblk2 = nullptr;
+  std::vector<PairBlk> pblk;       // list and pair blocks in that order
+  Chains chains[2];                // of the interval graph: the first one's, and the second one's
+  bool may_widen = true;           // a second one may be made (not in the serving loop)
+  bool wide = false;               // the interval graph is the second one
+  int graph_runs = 0;              // intervals run by graph, up to kWidenAfter
   std::vector<double> curT, curP;
   std::vector<double> wall_h;
   DevPtrs d{};
@@ -228,6 +237,78 @@ static bool programmatic_steps(const remd_engine_s* h) {
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// The 16-molecule blocks of the tiles of `order`.
+static std::vector<PairBlk> force_blocks(const remd_engine_s* h, const std::vector<int>& order) {
+  std::vector<PairBlk> out;
+  for (int t : order) {
+    const Tile& tt = h->tiles[t];
+    for (int k = 0; k < tt.count; k += kPart2Mol)
+      out.push_back(pair_blk(h->rc[tt.rep], tt.rep, tt.start + k, h->tile));
+  }
+  return out;
+}
+
+// Groups of whole replicas for K independent chains of the interval graph: each of one
+// water model (there are at most three; the pair kernel compiled for one model needs
+// fewer registers and instructions than the one for all), of about equal cost within a
+// model.  cost: of each tile.
+static void split_chains(const remd_engine_s* h, const std::vector<double>& cost, int K, Chains& ch) {
+  std::vector<double> rcost(h->nrep, 0.0);
+  std::map<int, double> mcost;   // cost, chains and replicas per model
+  std::map<int, int> mchains, mreps;
+  for (int r = 0; r < h->nrep; r++) {
+    for (int t = h->rc[r].tile_off; t < h->rc[r].tile_off + h->rc[r].ntile; t++) rcost[r] += cost[t];
+    mcost[h->rc[r].nsite] += rcost[r];
+    mreps[h->rc[r].nsite]++;
+  }
+  for (auto& m : mcost) mchains[m.first] = 1;
+  for (int left = K - (int)mcost.size(); left > 0; left--) {   // to the model whose chains are costliest
+    int best = -1;
+    for (auto& m : mcost)
+      if (mchains[m.first] < mreps[m.first] &&
+          (best == -1 || m.second / mchains[m.first] > mcost[best] / mchains[best]))
+        best = m.first;
+    if (best == -1) break;
+    mchains[best]++;
+  }
+  ch = Chains();
+  ch.n = 0;
+  std::vector<int> chain_of(h->nrep, 0);
+  for (auto& m : mcost) {
+    // the model's replicas in order, cut where the cost passes k / chains of its total
+    double run = 0.0;
+    int k = 0, used = 0, in_chain = 0, seen = 0;
+    for (int r = 0; r < h->nrep; r++) {
+      if (h->rc[r].nsite != m.first) continue;
+      const int left_reps = mreps[m.first] - seen, left_chains = mchains[m.first] - k;
+      if (in_chain > 0 && k + 1 < mchains[m.first] &&
+          (run + 0.5 * rcost[r] > m.second * (k + 1) / mchains[m.first] || left_reps < left_chains)) {
+        k++;
+        in_chain = 0;
+      }
+      chain_of[r] = ch.n + k;
+      run += rcost[r];
+      in_chain++;
+      seen++;
+      used = k + 1;
+    }
+    ch.n += used;
+  }
+  for (int k = 0; k < ch.n; k++) {
+    ch.pblk[k + 1] = ch.pblk[k];
+    for (int r = 0; r < h->nrep; r++)
+      if (chain_of[r] == k) {
+        ch.reps.push_back(r);
+        ch.pblk[k + 1] += h->rc[r].npart2;
+      }
+    for (int t : h->order)
+      if (chain_of[h->tiles[t].rep] == k) ch.order.push_back(t);
+    ch.rep[k + 1] = (int)ch.reps.size();
+    ch.tile[k + 1] = (int)ch.order.size();
+  }
+  ch.blk = force_blocks(h, ch.order);
+}
+
 // Build RepConst/tiles for the current tile size; returns pool layout size.
 static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
   const int T = h->tile;
@@ -276,84 +357,20 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     h->order.resize(h->tiles.size());
     for (size_t t = 0; t < h->order.size(); t++) h->order[t] = (int)t;
     std::stable_sort(h->order.begin(), h->order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-    // groups of whole replicas for the independent chains of the interval graph:
-    // each of one water model (there are at most three; the pair kernel compiled for
-    // one model needs fewer registers and instructions than the one for all), of
-    // about equal cost within a model
-    // Eight chains while a quarter of the batch is no more than one wave of pair
-    // blocks (about 2400 blocks in all), else four: 8 replicas of 4096 molecules run
-    // 785 us a 10-step interval on four and 730 us on eight.  256-replica batches on
-    // two / four / eight: 3611 / 3670 / 3718 us (111 432 molecules), 1136 / 1063 /
-    // 1108 and 2436 / 2390 / 2418 us (mixes of small tubes).
-    const int K = std::min(npart2 <= 2400 ? kMaxChains : 4, h->nrep);
-    std::vector<double> rcost(h->nrep, 0.0);
-    std::map<int, double> mcost;   // cost per model
-    for (int r = 0; r < h->nrep; r++) {
-      for (int t = h->rc[r].tile_off; t < h->rc[r].tile_off + h->rc[r].ntile; t++) rcost[r] += cost[t];
-      mcost[h->rc[r].nsite] += rcost[r];
-    }
-    std::map<int, int> mchains, mreps;   // chains and replicas per model
-    for (int r = 0; r < h->nrep; r++) mreps[h->rc[r].nsite]++;
-    for (auto& m : mcost) mchains[m.first] = 1;
-    for (int left = K - (int)mcost.size(); left > 0; left--) {   // to the model whose chains are costliest
-      int best = -1;
-      for (auto& m : mcost)
-        if (mchains[m.first] < mreps[m.first] &&
-            (best == -1 || m.second / mchains[m.first] > mcost[best] / mchains[best]))
-          best = m.first;
-      if (best == -1) break;
-      mchains[best]++;
-    }
-    h->reps2.clear();
-    h->order2.clear();
-    h->nchain = 0;
-    h->chain_tile[0] = h->chain_rep[0] = 0;
-    std::vector<int> chain_of(h->nrep, 0);
-    for (auto& m : mcost) {
-      // the model's replicas in order, cut where the cost passes k / chains of its total
-      double run = 0.0;
-      int k = 0, used = 0, in_chain = 0, seen = 0;
-      for (int r = 0; r < h->nrep; r++) {
-        if (h->rc[r].nsite != m.first) continue;
-        const int left_reps = mreps[m.first] - seen, left_chains = mchains[m.first] - k;
-        if (in_chain > 0 && k + 1 < mchains[m.first] &&
-            (run + 0.5 * rcost[r] > m.second * (k + 1) / mchains[m.first] || left_reps < left_chains)) {
-          k++;
-          in_chain = 0;
-        }
-        chain_of[r] = h->nchain + k;
-        run += rcost[r];
-        in_chain++;
-        seen++;
-        used = k + 1;
-      }
-      h->nchain += used;
-    }
-    for (int k = 0; k < h->nchain; k++) {
-      for (int r = 0; r < h->nrep; r++)
-        if (chain_of[r] == k) h->reps2.push_back(r);
-      for (int t : h->order)
-        if (chain_of[h->tiles[t].rep] == k) h->order2.push_back(t);
-      h->chain_rep[k + 1] = (int)h->reps2.size();
-      h->chain_tile[k + 1] = (int)h->order2.size();
-    }
-    auto blocks = [&](const std::vector<int>& order, std::vector<PairBlk>& out) {
-      out.clear();
-      for (int t : order)
-        for (int k = 0; k < h->tiles[t].count; k += kPart2Mol)
-          out.push_back(pair_blk(h->rc[h->tiles[t].rep], h->tiles[t].rep, h->tiles[t].start + k, T));
-    };
-    blocks(h->order, h->pblk);
-    blocks(h->order2, h->pblk2);
-    h->chain_pblk[0] = 0;
-    for (int k = 0; k < h->nchain; k++) {
-      int n = 0;
-      for (int r = h->chain_rep[k]; r < h->chain_rep[k + 1]; r++) n += h->rc[h->reps2[r]].npart2;
-      h->chain_pblk[k + 1] = h->chain_pblk[k] + n;
-    }
+    h->pblk = force_blocks(h, h->order);
+    split_chains(h, cost, std::min(kChains, h->nrep), h->chains[0]);
+    // A second graph of eight chains where they win 3 % or more, between 3 and 25 pair
+    // blocks per SM (interval times on four / eight chains: 16 x 512 bulk molecules 489 /
+    // 471 us, 64 x 512 slit 1636 / 1555, 8 x 4096 tube 766 / 723, 64 x 900 tube 1079 /
+    // 1039; below, 16 x 300 slit 342 / 333, 16 x 128 tube 1087 / 1084; above, 96 x 729
+    // bulk 2741 / 2706, 256-replica batches 3241 / 3225, 2142 / 2113, 3473 / 3474).
+    const double per_sm = (double)npart2 / sm_count();
+    h->chains[1] = Chains();
+    if (h->may_widen && !h->vscale && h->nrep > kChains && per_sm >= 3.0 && per_sm <= 25.0)
+      split_chains(h, cost, std::min(kMaxChains, h->nrep), h->chains[1]);
   }
   const size_t N = h->N, nt = h->tiles.size(), nr = h->nrep;
-  const size_t nf = (h->prec == kF32) ? 1 : 0;
+  const size_t nf = (h->prec == kF32) ? 1 : 0, w = h->chains[1].reps.empty() ? 0 : 1;
   if (nf) {   // 16-byte pieces of every molecule, as many as the largest record has
     int stride = 0;
     for (const RepConst& c : h->rc) stride = std::max(stride, c.pack_stride);
@@ -382,15 +399,16 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
       (size_t)h->nens * 8,             // 29 per-ensemble exchange seed
       nt * 4,                          // 30 order
       nf ? 0 : N * sizeof(int4),       // 31 com (FP64 form; FP32: the records' first pieces)
-      nt * 4,                          // 32 order per chain (multi-chain interval graph)
+      nt * 4,                          // 32 tiles by chain (first interval graph)
       nr * sizeof(CellGrid),           // 33 cell grid + rebuild decision per replica
       nr * (size_t)(kMaxCells + 1) * 4,   // 34 cell offsets per replica
       N * sizeof(int4),                // 35 centres sorted by cell
       nr * sizeof(int2),               // 36 carried replicas' sources (serving batch changes)
       (size_t)h->nens * 4, (size_t)h->nens * 4,   // 37 carried ensembles' sources, 38 replicas per ensemble
-      nf * nr * sizeof(PairConst), npart2 * sizeof(PairBlk), npart2 * sizeof(PairBlk),   // 39 pair constants, 40 pair blocks, 41 per chain
+      nf * nr * sizeof(PairConst), npart2 * sizeof(PairBlk), npart2 * sizeof(PairBlk),   // 39 pair constants, 40 pair blocks, 41 by chain
       nf * nbr_words * 2, nf * N * 4, nf * N * 32,   // 42 nbt (per-step lists), 43 their counts, 44 wall terms
-      nr * 4,                          // 45 replicas per chain
+      nr * 4,                          // 45 replicas by chain
+      w * nt * 4, w * npart2 * sizeof(PairBlk), w * nr * 4,   // 46..48 the same for the second interval graph
   };
   offs.clear();
   total = 0;
@@ -470,7 +488,6 @@ static remd_status allocate(remd_engine_s* h) {
   h->d_seed = reinterpret_cast<unsigned long long*>(b + offs[29]);
   d.order = reinterpret_cast<int*>(b + offs[30]);
   d.com = reinterpret_cast<int4*>(h->prec == kF32 ? d.pack : b + offs[31]);
-  h->d_order2 = reinterpret_cast<int*>(b + offs[32]);
   d.cgrid = reinterpret_cast<CellGrid*>(b + offs[33]);
   d.cell_start = reinterpret_cast<int*>(b + offs[34]);
   d.cell_com = reinterpret_cast<int4*>(b + offs[35]);
@@ -480,11 +497,14 @@ static remd_status allocate(remd_engine_s* h) {
   d.pc = reinterpret_cast<PairConst*>(b + offs[39]);
   d.pblk = reinterpret_cast<PairBlk*>(b + offs[40]);
   d.npblk = (int)h->pblk.size();
-  h->d_pblk2 = reinterpret_cast<PairBlk*>(b + offs[41]);
   d.nbt = reinterpret_cast<uint16_t*>(b + offs[42]);
   d.nt_cnt = reinterpret_cast<int*>(b + offs[43]);
   d.wallf = reinterpret_cast<double*>(b + offs[44]);
-  h->d_reps2 = reinterpret_cast<int*>(b + offs[45]);
+  for (int k = 0; k < 2; k++) {
+    h->chains[k].d_order = reinterpret_cast<int*>(b + offs[k ? 46 : 32]);
+    h->chains[k].d_blk = reinterpret_cast<PairBlk*>(b + offs[k ? 47 : 41]);
+    h->chains[k].d_reps = reinterpret_cast<int*>(b + offs[k ? 48 : 45]);
+  }
   d.reps = nullptr;
   d.nrep_l = h->nrep;
   d.pdl = programmatic_steps(h);
@@ -500,15 +520,18 @@ static remd_status allocate(remd_engine_s* h) {
   CK(cudaMemcpyAsync((void*)d.rc, h->rc.data(), h->rc.size() * sizeof(RepConst), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync((void*)d.tiles, h->tiles.data(), h->tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync((void*)d.order, h->order.data(), h->order.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(h->d_order2, h->order2.data(), h->order2.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(h->d_reps2, h->reps2.data(), h->reps2.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  for (const Chains& ch : h->chains) {
+    if (ch.reps.empty()) continue;
+    CK(cudaMemcpyAsync(ch.d_order, ch.order.data(), ch.order.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(ch.d_reps, ch.reps.data(), ch.reps.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(ch.d_blk, ch.blk.data(), ch.blk.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
+  }
   std::vector<PairConst> pc;
   if (h->prec == kF32) {
     for (const RepConst& c : h->rc) pc.push_back(pair_const(c));
     CK(cudaMemcpyAsync((void*)d.pc, pc.data(), pc.size() * sizeof(PairConst), cudaMemcpyHostToDevice, h->stream));
   }
   CK(cudaMemcpyAsync((void*)d.pblk, h->pblk.data(), h->pblk.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(h->d_pblk2, h->pblk2.data(), h->pblk2.size() * sizeof(PairBlk), cudaMemcpyHostToDevice, h->stream));
   if (!h->wall_h.empty())
     CK(cudaMemcpyAsync((void*)d.wall, h->wall_h.data(), h->wall_h.size() * 8, cudaMemcpyHostToDevice, h->stream));
   // later set-up copies use the default stream, which does not order with this
@@ -578,42 +601,51 @@ static void launch_step_integrate(remd_engine_s* h, int s) {
   }
 }
 
+// Streams and events of n chains, those that are not there yet (on the current device).
+static remd_status chain_streams(remd_engine_s* h, int n) {
+  for (int k = 0; k < n - 1; k++) {
+    if (!h->stream2[k]) CK(cudaStreamCreateWithFlags(&h->stream2[k], cudaStreamNonBlocking));
+    if (!h->ev_join[k]) CK(cudaEventCreateWithFlags(&h->ev_join[k], cudaEventDisableTiming));
+  }
+  return REMD_OK;
+}
+
 static remd_status build_graph(remd_engine_s* h) {
   const DeviceScope on(h->device);   // the chains' streams are the device's
   if (!on.ok) { set_error("graph capture: cannot use the handle's device"); return REMD_ERR_CUDA; }
   cudaGraph_t g;
-  if (!h->vscale)   // the chains' streams, when first needed
-    for (int k = 0; k < h->nchain - 1; k++) {
-      if (!h->stream2[k]) CK(cudaStreamCreateWithFlags(&h->stream2[k], cudaStreamNonBlocking));
-      if (!h->ev_join[k]) CK(cudaEventCreateWithFlags(&h->ev_join[k], cudaEventDisableTiming));
-    }
+  const Chains& ch = h->chains[h->wide ? 1 : 0];
+  if (!h->vscale) {
+    const remd_status s = chain_streams(h, ch.n);
+    if (s != REMD_OK) return s;
+  }
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   launch_replica_start(h->d, h->X, h->stream);
-  if (h->nchain > 1 && !h->vscale) {
+  if (ch.n > 1 && !h->vscale) {
     // independent chains, one per group of replicas (no data crosses between
     // them), so one group's latency-bound phases -- the integrate kernel's
     // scalar chains, the list kernel's heads, the pair kernel's tail -- overlap
     // the other groups' work
     DevPtrs dg[kMaxChains];
-    for (int k = 0; k < h->nchain; k++) {
+    for (int k = 0; k < ch.n; k++) {
       dg[k] = h->d;
-      dg[k].ntiles = h->chain_tile[k + 1] - h->chain_tile[k];
-      dg[k].order = h->d_order2 + h->chain_tile[k];
-      dg[k].reps = h->d_reps2 + h->chain_rep[k];
-      dg[k].nrep_l = h->chain_rep[k + 1] - h->chain_rep[k];
-      dg[k].model_l = common_model(h, &h->reps2[h->chain_rep[k]], dg[k].nrep_l);
-      dg[k].pblk = h->d_pblk2 + h->chain_pblk[k];
-      dg[k].npblk = h->chain_pblk[k + 1] - h->chain_pblk[k];
+      dg[k].ntiles = ch.tile[k + 1] - ch.tile[k];
+      dg[k].order = ch.d_order + ch.tile[k];
+      dg[k].reps = ch.d_reps + ch.rep[k];
+      dg[k].nrep_l = ch.rep[k + 1] - ch.rep[k];
+      dg[k].model_l = common_model(h, &ch.reps[ch.rep[k]], dg[k].nrep_l);
+      dg[k].pblk = ch.d_blk + ch.pblk[k];
+      dg[k].npblk = ch.pblk[k + 1] - ch.pblk[k];
     }
     cudaEventRecord(h->ev_fork, h->stream);
-    for (int k = 1; k < h->nchain; k++) cudaStreamWaitEvent(h->stream2[k - 1], h->ev_fork, 0);
+    for (int k = 1; k < ch.n; k++) cudaStreamWaitEvent(h->stream2[k - 1], h->ev_fork, 0);
     for (int s = 0; s < h->interval; s++)
-      for (int k = 0; k < h->nchain; k++) {
+      for (int k = 0; k < ch.n; k++) {
         cudaStream_t st = k ? h->stream2[k - 1] : h->stream;
         launch_integrate_prec(dg[k], h->X, h->Y, s > 0, h->tile, h->prec, st);
         launch_force(dg[k], h->Y, h->X, h->prec, false, st);
       }
-    for (int k = 1; k < h->nchain; k++) {
+    for (int k = 1; k < ch.n; k++) {
       cudaEventRecord(h->ev_join[k - 1], h->stream2[k - 1]);
       cudaStreamWaitEvent(h->stream, h->ev_join[k - 1], 0);
     }
@@ -1002,7 +1034,9 @@ static remd_status create_impl(const remd_system_desc* systems, int nens, const 
       return REMD_ERR_CUDA;
     }
   }
+  h->may_widen = !cy;
   remd_status st = allocate(h);
+  if (st == REMD_OK && !h->vscale) st = chain_streams(h, h->chains[0].n);
   if (st != REMD_OK) { undo_carry(h, cy); return st; }
   // host SoA staging
   const int N = h->N;
@@ -1200,16 +1234,31 @@ remd_status remd_execute_steps_async(remd_handle h, const double* T, const doubl
     CK(cudaMemcpyAsync(h->dT, h->hT, h->nrep * 8, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->dP, h->hP, h->nrep * 8, cudaMemcpyHostToDevice, h->stream));
   }
+  // Eight chains win a few percent of an interval; capturing their graph costs two to
+  // three times four chains' (0.6 + 2.6 + 0.9 us a node to capture, instantiate and
+  // upload: a first interval of 16 x 128 molecules, 50 steps, 7.4 ms on eight chains and
+  // 4.3 on four), that is as much as some 15 to 40 intervals win.  So a handle starts on
+  // four and goes over once it has run that many.  The serving loop's handles, whose
+  // graph is updated in place at batch changes, stay on four.
+  const bool widen = !h->wide && !h->chains[1].reps.empty() && h->graph_runs >= kWidenAfter;
   if (!h->gexec || h->graph_tile != h->tile || h->graph_exchange != h->exch_enabled ||
-      h->graph_hist != h->hist_on) {
+      h->graph_hist != h->hist_on || widen) {
     const auto g0 = std::chrono::steady_clock::now();
+    if (widen) h->wide = true;
     remd_status s = build_graph(h);
+    if (widen && s != REMD_OK) {   // no room for it: back to the first one
+      cudaGetLastError();
+      h->wide = false;
+      h->chains[1] = Chains();
+      s = build_graph(h);
+    }
     h->last_graph_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - g0).count();
     if (s != REMD_OK) return s;
   } else {
     h->last_graph_ms = 0.0;
   }
   CK(cudaGraphLaunch(h->gexec, h->stream));
+  if (h->graph_runs < kWidenAfter) h->graph_runs++;
   h->steps_done += h->interval;
   return REMD_OK;
 }
@@ -1332,7 +1381,7 @@ int remd_launches_per_interval(remd_handle h) {
   // + replica_end + the device exchange when enabled (and the histogram before it)
   if (!h) return 0;
   // (the multi-chain graph, without velocity scaling, launches each step kernel once per chain)
-  const int chains = h->vscale ? 1 : h->nchain;
+  const int chains = h->vscale ? 1 : h->chains[h->wide ? 1 : 0].n;
   const int per_step = ((h->prec == kF32 ? 4 : 3) + (h->vscale ? 1 : 0)) * chains;
   return per_step * h->interval + (h->vscale ? h->interval - 1 : 0) + 2 + (h->exch_enabled ? 1 : 0) +
          (h->exch_enabled && h->hist_on ? 1 : 0);

@@ -25,6 +25,7 @@ namespace remd {
 constexpr int kMaxSites = 5;
 constexpr int kNumAvg = 19;
 constexpr int kPart2Mol = 16;                   // molecules of a force partial sum (Part2)
+constexpr int kPairBlocks = 64 / kPart2Mol;     // pair blocks that an SM holds (FP32 form)
 constexpr double kFix = 4294967296.0;          // 2^32: fixed-point box fraction
 constexpr double kFixInv = 1.0 / 4294967296.0;
 

@@ -1507,7 +1507,7 @@ __device__ void force_block_f32(const DevPtrs& d, const PairBlk& b, const PairCo
 // S: the sites of every replica of the launch (0: mixed models, chosen per
 // block); STD: every replica has the charge ratios of charge_ratio.
 template <int S, bool STD>
-__global__ void __launch_bounds__(32 * kPairWarps, 64 / kPart2Mol) k_force_pairs(DevPtrs d, const RepState* __restrict__ X) {
+__global__ void __launch_bounds__(32 * kPairWarps, kPairBlocks) k_force_pairs(DevPtrs d, const RepState* __restrict__ X) {
   step_kernel_entry();
   __shared__ PairConst c;
   __shared__ F32Const k32;

@@ -113,3 +113,54 @@ def test_chain_warp_only_where_all_chains_leave_room(fake, nmol, nrep, extra):
     eng = E.REMDGPU([_grid(nmol, nrep)])
     assert all(x[2] == 32 + extra for x in _interval(fake, eng) if "k_integrate" in x[0])
     eng.close()
+
+
+def _chains(launches):
+    return len({x[4] for x in _steps(launches)})
+
+
+def test_first_interval_is_cheap_to_set_up(fake):
+    """Streams are made with the handle, not inside its first timed call, and the first
+    interval's graph holds four chains however large the batch is."""
+    for n, nrep in ((128, 16), (512, 64)):
+        eng = E.REMDGPU([_grid(n, nrep)])
+        first = _interval(fake, eng)
+        assert fake.fake_count(b"streams_made") == 0
+        assert fake.fake_count(b"nodes") == 4 * 4 * 3 + 2 == len(first)   # chains x kernels x steps, start and end
+        assert _chains(first) == 4 and eng.launches_per_interval() == len(first)
+        eng.close()
+
+
+@pytest.mark.parametrize("nmol,nrep,later", [(512, 64, 8), (128, 16, 4), (512, 4, 4), (64, 1, 1)])
+def test_eight_chains_come_once_they_pay(fake, nmol, nrep, later):
+    """A handle that keeps running goes over to a second graph, once, where eight chains
+    are faster; every replica is in exactly one chain of it."""
+    eng = E.REMDGPU([_grid(nmol, nrep)])
+    for _ in range(32):
+        assert _chains(_interval(fake, eng)) == min(4, nrep)
+    second = _interval(fake, eng)
+    assert _chains(second) == later and eng.launches_per_interval() == len(second)
+    for kernel, per in (("k_integrate", nrep * -(-nmol // 32)), ("k_replica_head", nrep), ("k_force_pairs", nrep * -(-nmol // 16))):
+        assert sum(x[1] for x in second if kernel in x[0]) == 3 * per
+    fake.fake_reset()
+    eng.ExecuteSteps(eng.T, eng.P)
+    assert fake.fake_count(b"instantiated") == 0
+    eng.set_tuning(64, 1.0)   # a new layout keeps the chains
+    assert _chains(_interval(fake, eng)) == later
+    eng.close()
+
+
+def test_serving_loop_updates_its_graph_in_place(fake):
+    """A batch that grows and shrinks keeps one graph topology, so the executable graph
+    is updated and not made anew, also after many rounds."""
+    srv = E.Server(budget_bytes=1 << 33)
+    e = _grid(200, 64)
+    srv.submit(e, 40)
+    for _ in range(36):
+        srv.step()
+    fake.fake_reset()
+    srv.submit(_grid(400, 64), 20)
+    srv.step()
+    assert fake.fake_count(b"instantiated") == 0 and fake.fake_count(b"updated") == 1
+    assert _chains(_launches(fake)) == 4
+    srv.close()
