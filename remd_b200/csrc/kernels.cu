@@ -1432,13 +1432,16 @@ __device__ __forceinline__ void step_list(const DevPtrs& d, const PairBlk& b, co
 }
 
 // FP32 form, first launch after the replica head, kPart2Mol molecules per block:
-// their skin lists where the replica's are due, their per-step lists and, where
-// confined, their wall terms.  A kernel of its own, light on registers: its many
-// warps hide the gathered loads' latency, which the pair kernel's four per
-// scheduler do not (the gather inside the pair kernel took 12 000 of a warp's
-// 43 000 cycles on 256 replicas, 111 432 molecules).  It is bound by the latency of
-// its loads, so all that need only the block's descriptor are issued together (75 us
-// on those 256 replicas, of which 25 us the rebuild of 14 of them).
+// their wall terms where confined, their skin lists where the replica's are due, and
+// their per-step lists.  A kernel of its own, light on registers: its many warps hide
+// the gathered loads' latency, which the pair kernel's four per scheduler do not (the
+// gather inside the pair kernel took 12 000 of a warp's 43 000 cycles on 256 replicas,
+// 111 432 molecules).  It is bound by the latency of its loads, so all that need only
+// the block's descriptor are issued together, and the wall's FP64 chain runs under
+// them, a molecule per thread of the first warp (one lane in eight of every warp,
+// after the lists: 88.6 us there, now 83.4, of which 25 the rebuild of 14 replicas;
+// 256 tubes of 128 .. 420 molecules 41.0 -> 36.0).  Two and four lanes per molecule
+// measured slower at every length of the lists (158 and 112 us; on the tubes 64 and 45).
 __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_lists(DevPtrs d, const RepState* __restrict__ X) {
   step_kernel_entry();
   extern __shared__ uint32_t bm[];
@@ -1452,9 +1455,11 @@ __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_list
   uint4 w0 = list_words(nb, 8 * sub), w1 = list_words(nb, 8 * sub + 8 * kGroup);
   const int4 me = d.com[g];
   double qr[7];
-  if (b.confined) {
-    for (int x = 0; x < 4; x++) qr[x] = d.q[x * d.N + g];
-    for (int x = 0; x < 3; x++) qr[4 + x] = d.r[x * d.N + g];
+  const int wli = b.li0 + threadIdx.x, wg = b.mol_off + min(wli, b.nmol - 1);
+  const bool wall = b.confined && threadIdx.x < kPart2Mol && wli < b.nmol;
+  if (wall) {
+    for (int x = 0; x < 4; x++) qr[x] = d.q[x * d.N + wg];
+    for (int x = 0; x < 3; x++) qr[4 + x] = d.r[x * d.N + wg];
   }
   const RepState& st = X[b.rep];
   const double L[3] = {st.L[0], st.L[1], st.L[2]};
@@ -1464,6 +1469,13 @@ __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_list
     reinterpret_cast<uint32_t*>(&c)[k] = src[k];
   __syncthreads();
   if (li0 >= b.nmol) return;
+  if (wall) {
+    double f[3] = {0.0, 0.0, 0.0};
+    const double e = wall_site(d, d.rc[b.rep], qr, qr + 4, L, f);
+    double2* w = reinterpret_cast<double2*>(d.wallf + 4 * (long long)wg);
+    w[0] = make_double2(f[0], f[1]);
+    w[1] = make_double2(f[2], e);
+  }
   if (rebuild) {
     const RepConst& rc = d.rc[b.rep];
     build_lists(d, rc, b.rep, li0, L, bm, d.bm_win);
@@ -1476,13 +1488,6 @@ __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_list
     w1 = list_words(nb, 8 * sub + 8 * kGroup);
   }
   step_list(d, b, c, li, cnt, me, w0, w1, L);
-  if (b.confined && sub == 0 && li < b.nmol) {
-    double f[3] = {0.0, 0.0, 0.0};
-    const double e = wall_site(d, d.rc[b.rep], qr, qr + 4, L, f);
-    double2* w = reinterpret_cast<double2*>(d.wallf + 4 * (long long)g);
-    w[0] = make_double2(f[0], f[1]);
-    w[1] = make_double2(f[2], e);
-  }
 }
 
 // FP32 form, second launch of a step: pair forces and A2M of kPart2Mol molecules per
