@@ -921,9 +921,10 @@ __device__ __forceinline__ void load_record(const DevPtrs& d, const PairConst& c
 }
 
 // The near pairs of a segment (SIMG), as a call: its image tests and their FP64
-// branch would otherwise hold registers through the far pairs' loop (with it
-// inlined the kernel spilled 200 bytes at 128 registers; it runs for a few percent
-// of the pairs of the boxes close to the minimum-image bound only).
+// branch would otherwise hold registers through the far pairs' loop (it runs for a few
+// percent of the pairs of the boxes close to the minimum-image bound only).  The call
+// costs its caller a frame: the kernel that makes it holds the sums whose address it
+// takes and spills 144-164 bytes at 128 registers; inlined, it spilled 200.
 template <int S, int C0>
 __device__ __noinline__ void near_pairs_f32(const DevPtrs& d, const PairConst& c, const F32Const& k32, int li,
                                             const uint16_t* row, int n, F32Sums<S>* out) {
@@ -1491,13 +1492,14 @@ __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_list
 }
 
 // FP32 form, second launch of a step: pair forces and A2M of kPart2Mol molecules per
-// block, and their partial sums.  Bound by the issue of FP32 instructions: 67 % of the
-// issue slots and 47 % of the FMA pipe at four warps per scheduler (256 replicas,
-// 111 432 molecules: 228 us, 166 M warp instructions; with two threads per molecule
-// 267 us at 62 %), then by the latency of a warp's other phases (lists and constants
-// 6 000, exchange and A2M 4 200 of 37 000 cycles).  16 TIP5P replicas of 1728
-// molecules: 148 -> 142 us of pairs, 8 TIP4P replicas of 512: 47 -> 18 us.  128
-// registers for all models: 168 measured 2-4 % slower and 96 spills.
+// block, and their partial sums.  Bound by the issue of FP32 instructions at four warps
+// per scheduler, then by the latency of a warp's other phases (lists and constants,
+// exchange and A2M).  The kernel parameter is a grid constant: near_pairs_f32 takes its
+// address, and every thread would copy its 350 bytes into local memory first (256
+// replicas, 111 432 molecules: 236 us a launch with that copy, 218 without; 64 tubes of
+// 700 TIP4P molecules 58 -> 47, 8 of 4096 48 -> 39, 64 slits of 512 57 -> 51; with two
+// threads per molecule instead of eight 272, 54, 55 and 78).  128 registers for all
+// models: 168 measured 2-4 % slower, 96 slower still.
 template <int S, int C0, bool STD>
 __device__ void force_block_f32(const DevPtrs& d, const PairBlk& b, const PairConst& c, const F32Const& k32, int nc,
                                 double q4, double wf, double (*wsum)[8]) {
@@ -1512,7 +1514,8 @@ __device__ void force_block_f32(const DevPtrs& d, const PairBlk& b, const PairCo
 // S: the sites of every replica of the launch (0: mixed models, chosen per
 // block); STD: every replica has the charge ratios of charge_ratio.
 template <int S, bool STD>
-__global__ void __launch_bounds__(32 * kPairWarps, kPairBlocks) k_force_pairs(DevPtrs d, const RepState* __restrict__ X) {
+__global__ void __launch_bounds__(32 * kPairWarps, kPairBlocks) k_force_pairs(const __grid_constant__ DevPtrs d,
+                                                                             const RepState* __restrict__ X) {
   step_kernel_entry();
   __shared__ PairConst c;
   __shared__ F32Const k32;
