@@ -222,17 +222,17 @@ static double neighbours(const RepConst& c) {
 }
 
 // Programmatic launch of the step kernels (launch_step_kernel) pays while a step's pair
-// kernels are short, up to about 4500 pairs per SM in all: the next kernel's blocks are
+// kernels are short, up to about 4000 pairs per SM in all: the next kernel's blocks are
 // scheduled early and wait on SMs that would idle.  Above, they hold slots that the
 // other chains' kernels would use.  Interval times with it / without: 16 replicas of 128
-// tube molecules (430 pairs per SM) 1087 / 1162 us, 4 x 2000 tube molecules (3200) 350 /
-// 378, 8 x 512 bulk molecules (3900) 389 / 402, 64 x 200 tube molecules (4300) 421 /
-// 431; 4096 bulk molecules (5200) 498 / 474, FP64 8 x 729 (5500) 566 / 549, 16 x 512 bulk
-// (7800) 496 / 487, 64 x 512 slit (19000) 1850 / 1636, 64 x 729 bulk (44000) 1580 / 1437.
+// tube molecules (430 pairs per SM) 1030 / 1081 us, 4 x 2000 tube molecules (3200) 322 /
+// 344, 8 x 512 bulk molecules (3900) 368 / 372; 64 x 200 tube molecules (4300) 391 / 385,
+// 4096 bulk molecules (5200) 483 / 454, FP64 8 x 729 (5500) 562 / 543, 16 x 512 bulk
+// (7800) 478 / 461, 64 x 512 slit (19000) 1760 / 1498, 64 x 729 bulk (44000) 1485 / 1330.
 static bool programmatic_steps(const remd_engine_s* h) {
   double pairs = 0.0;
   for (const RepConst& c : h->rc) pairs += c.nmol * neighbours(c);
-  return pairs <= 4500.0 * sm_count();
+  return pairs <= 4000.0 * sm_count();
 }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -359,14 +359,15 @@ static void layout(remd_engine_s* h, std::vector<size_t>& offs, size_t& total) {
     std::stable_sort(h->order.begin(), h->order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     h->pblk = force_blocks(h, h->order);
     split_chains(h, cost, std::min(kChains, h->nrep), h->chains[0]);
-    // A second graph of eight chains where they win 3 % or more, between 3 and 25 pair
-    // blocks per SM (interval times on four / eight chains: 16 x 512 bulk molecules 489 /
-    // 471 us, 64 x 512 slit 1636 / 1555, 8 x 4096 tube 766 / 723, 64 x 900 tube 1079 /
-    // 1039; below, 16 x 300 slit 342 / 333, 16 x 128 tube 1087 / 1084; above, 96 x 729
-    // bulk 2741 / 2706, 256-replica batches 3241 / 3225, 2142 / 2113, 3473 / 3474).
+    // A second graph of eight chains where they win, between 3 and 32 pair blocks per SM.
+    // Interval times on four / eight chains: 16 x 512 bulk molecules 461 / 441 us, 64 x 512
+    // slit 1498 / 1428, 8 x 4096 tube 627 / 596, 64 x 900 tube 879 / 844, 96 x 729 bulk
+    // 2542 / 2472, mixes of 256 replicas 1774 / 1685 and 997 / 979; below, 16 x 300 slit
+    // 329 / 326, 16 x 128 tube 1030 / 1033; above, mixes of 256 replicas 2004 / 1966, 3199 /
+    // 3174 and 3366 / 3337.
     const double per_sm = (double)npart2 / sm_count();
     h->chains[1] = Chains();
-    if (h->may_widen && !h->vscale && h->nrep > kChains && per_sm >= 3.0 && per_sm <= 25.0)
+    if (h->may_widen && !h->vscale && h->nrep > kChains && per_sm >= 3.0 && per_sm <= 32.0)
       split_chains(h, cost, std::min(kMaxChains, h->nrep), h->chains[1]);
   }
   const size_t N = h->N, nt = h->tiles.size(), nr = h->nrep;

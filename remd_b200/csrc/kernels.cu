@@ -2293,10 +2293,10 @@ static void launch_step_kernel(bool pdl, void (*k)(KArgs...), unsigned grid, uns
 void launch_integrate_prec(const DevPtrs& d, const RepState* X, RepState* Y, bool mid, int tile,
                            int prec, cudaStream_t s) {
   // the scalar chain's own warp where the blocks of all the handle's chains, which run
-  // side by side, are resident with it: 16 replicas of 128 molecules 1161 us a 50-step
-  // interval with it and 1208 without; 96 replicas of 729 molecules (2208 tiles) 2785 us
-  // a 10-step interval with it and 2741 without, 256 replicas (111 432 molecules) 3299
-  // and 3239
+  // side by side, are resident with it: 16 replicas of 128 molecules 1030 us a 50-step
+  // interval with it and 1085 without, 8 of 4096 627 a 10-step interval and 648; 96
+  // replicas of 729 molecules (2208 tiles) 2584 with it and 2542 without, 256 replicas
+  // (111 432 molecules) 3264 and 3194
   const bool chain = (long long)d.ntiles_h * (tile + 32) <= (long long)sm_count() * 3 * 160;
   void (*k)(DevPtrs, const RepState*, RepState*, int) =
       chain ? (mid ? k_integrate<true, true> : k_integrate<false, true>)
