@@ -37,15 +37,60 @@ def test_edges_of_groups_warps_and_blocks(nmol, prec):
     _check(e.spec, e.states[0], prec, "fp32 small" if prec == "fp32" else None)
 
 
+def _counts(spec, st):
+    """Per molecule: neighbours within rcut, and those of them that are near pairs
+    (their site vectors may cross half a box length)."""
+    d = st.r[:, None] - st.r[None]
+    d = (d - np.round(d)) * st.L
+    within = (d ** 2).sum(-1) <= spec.rcut ** 2
+    np.fill_diagonal(within, False)
+    reach = np.linalg.norm(spec.moltype.r, axis=1).max()
+    near = within & (np.abs(d) >= 0.5 * st.L - 2.0 * reach - 1e-3).any(-1)
+    return within.sum(1), near.sum(1)
+
+
+def _dense(model, nmol, scale, seed, moved=0.15):
+    """A bulk box denser than the liquid, the molecules moved a little off their lattice."""
+    e = S.make_ensemble("dense", model, 0, nmol, 0.0, 12.0, 10.0, 1, 1, 300, 300, 0.1e6, 0.1e6, seed)
+    st = e.states[0]
+    st.L = st.L * scale
+    rng = np.random.default_rng(seed)
+    st.r = (st.r + rng.normal(size=st.r.shape) * (moved / st.L)) % 1.0
+    return copy.deepcopy(e.spec), st
+
+
 @pytest.mark.parametrize("prec", ["fp32", "fp64"])
 @pytest.mark.parametrize("model", ["tip3p", "tip5p"])
 def test_more_pairs_than_one_partial_sum(model, prec):
     """A lane's FP32 sums, and the FP64 form's shared rows, close after 256 pairs of a
-    molecule: a bulk box at 1.2 times liquid density has about 290 within 12 A."""
-    e = S.make_ensemble("dense", model, 0, 1000, 0.0, 12.0, 10.0, 1, 1, 300, 300, 0.1e6, 0.1e6, 310)
-    st = e.states[0]
-    st.L = st.L * 0.94
-    _check(e.spec, st, prec)
+    molecule: a box where molecules of one warp lie on both sides of that."""
+    spec, st = _dense(model, 1000, 0.968, 310)
+    pairs, near = _counts(spec, st)
+    warps = pairs.reshape(-1, 4)
+    assert ((warps > 256).any(1) & (warps <= 256).any(1)).sum() > 20 and near.max() == 0
+    _check(spec, st, prec)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_near_pairs_beside_several_partial_sums(prec):
+    """A box little above 2 rcut: some near pairs beside more than 256 far ones."""
+    spec, st = _dense("tip3p", 729, 0.935, 312)
+    pairs, near = _counts(spec, st)
+    assert pairs.min() > 256 and 0 < near.mean() < 64
+    _check(spec, st, prec)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_more_near_pairs_than_one_partial_sum(prec):
+    """A weak charge far from its molecule's centre makes nearly every pair near.  The
+    energy gate needs terms that do not cancel: the FP32 form's Lennard-Jones and
+    Coulomb energies are good to some 8e-7 and 4e-7, which is 6e-7 of their sum here."""
+    spec, st = _dense("tip4p", 729, 0.935, 312, moved=0.05)
+    spec.moltype.r[1] *= 5.0
+    spec.moltype.charge[:] = (0.0, 1e-6, 1.04, -1.04)
+    pairs, near = _counts(spec, st)
+    assert near.min() > 256 and (pairs > near).all()
+    _check(spec, st, prec)
 
 
 @pytest.mark.parametrize("model", ["tip3p", "tip4p", "tip5p"])
@@ -79,17 +124,29 @@ def test_fp64_form_with_cell_lists():
     _check(e.spec, e.states[0], "fp64")
 
 
-def test_mixed_models_in_one_handle_equal_each_alone():
-    """More models than one kernel is compiled for share a launch (one chain): the
-    forces are those of the per-model kernels, bit for bit."""
+@pytest.mark.parametrize("prec,charges", [("fp32", "water"), ("fp64", "water"), ("fp32", "other")])
+def test_mixed_models_in_one_handle_equal_each_alone(prec, charges):
+    """The first forces of a handle come from one launch over all its models, for which
+    the kernels choose per block (alone, the kernel compiled for the model); then the
+    chains of the interval graph, one model each: both give the bits of each alone."""
     ens = [S.small_ensemble(m, 1, nmol=n, ntemp=1, npress=1, seed=340, interval=5)
            for m, n in (("tip3p", 70), ("tip4p", 65), ("tip5p", 80))]
-    both = E.REMDGPU(ens, precision="fp32")
-    both.execute_nsteps(5)
+    if charges == "other":
+        ens = copy.deepcopy(ens)
+        for e in ens:
+            q = e.spec.moltype.charge
+            q[int(np.nonzero(q)[0][0])] *= 0.9
+            q[-1] -= q.sum()
+    def run(e):
+        eng = E.REMDGPU(e, precision=prec)
+        first = [eng.ConvertVariablesToHost(k) for k in range(eng.nrep)]
+        eng.ExecuteSteps(eng.T, eng.P)
+        graph = [eng.ConvertVariablesToHost(k) for k in range(eng.nrep)]
+        eng.execute_nsteps(5)
+        last = [eng.ConvertVariablesToHost(k) for k in range(eng.nrep)]
+        eng.close()
+        return first, graph, last
+    both = run(ens)
     for k, e in enumerate(ens):
-        alone = E.REMDGPU([e], precision="fp32")
-        alone.execute_nsteps(5)
-        a, b = alone.ConvertVariablesToHost(0), both.ConvertVariablesToHost(k)
-        assert all(np.array_equal(a[x], b[x]) for x in ("r", "v", "q", "p", "f", "n"))
-        alone.close()
-    both.close()
+        for a, b in zip(run([e]), both):
+            assert all(np.array_equal(a[0][x], b[k][x]) for x in ("r", "v", "q", "p", "f", "n"))

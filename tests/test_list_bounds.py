@@ -1,4 +1,4 @@
-"""The FP32 form rebuilds its (rcut + skin) neighbour lists with a cheap test:
+"""Both forms rebuild their (rcut + skin) neighbour lists with a cheap test:
 FP32 arithmetic on the top 16 bits of each 32-bit fixed-point centre
 difference, against rcut + skin widened by sqrt(3) L_max 2^-16 and a relative
 1e-5 (kernels.cu, build_lists).  The lists only have to contain every pair
