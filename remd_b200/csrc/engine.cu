@@ -211,6 +211,16 @@ static remd_status check_desc(const remd_system_desc& s, std::string& why) {
   return REMD_OK;
 }
 
+// Measured best on a 256-replica mixed batch; remd_set_tuning / remd_autotune change it.
+static int default_tile(int prec) { return prec == kF32 ? 32 : 128; }
+
+// Neighbour list capacity: three times the liquid's density, at most every other molecule.
+static int list_capacity(double rc, double skin, int nmol) {
+  const double rl = rc + skin;
+  const double cap = 0.1 * 4.0 / 3.0 * M_PI * rl * rl * rl;
+  return std::max(1, std::min(nmol - 1, ((int)std::ceil(cap) + 7) / 8 * 8));
+}
+
 // Estimated neighbours of a molecule within rcut at liquid density: a sphere, in a tube
 // or a slit no more than the tube's or slit's part within rcut along it.
 static double neighbours(const RepConst& c) {
@@ -719,6 +729,22 @@ remd_status engine_get_exchange(remd_handle h, long long* steps, int* index) {
 
 size_t engine_bytes(remd_handle h) { return h ? h->bytes : 0; }
 
+// The sums that layout() makes, with the longest record (a batch's records are as long
+// as its longest) and a full set of alignment gaps.  The job is not checked yet.
+size_t engine_job_bytes(const remd_system_desc& s, int nrep, remd_precision prec) {
+  const remd_engine_s fresh;
+  const bool f32 = prec != REMD_PREC_FP64;
+  const size_t n = (size_t)s.nmol, T = default_tile(f32 ? kF32 : kF64);
+  const size_t row = ((size_t)list_capacity(s.rcut, fresh.skin, s.nmol) + 7) / 8 * 8;
+  const size_t mol = 21 * 8 + (f32 ? 4 * pack_stride(kMaxSites, kF32) : 8 * pack_stride(kMaxSites, kF64)) +
+                     2 * sizeof(int4) + 4 + (f32 ? 4 + 32 : sizeof(int4)) + (f32 ? 4 : 2) * row;
+  const size_t rep = (n + T - 1) / T * (sizeof(Tile) + 3 * 8 + 2 * 4) + (n + 31) / 32 * sizeof(Part1) +
+                     (n + kPart2Mol - 1) / kPart2Mol * (sizeof(Part2) + 2 * sizeof(PairBlk)) + sizeof(RepConst) +
+                     sizeof(PairConst) + 2 * sizeof(RepState) + (kNumAvg + 2) * 8 + sizeof(CellGrid) +
+                     4 * (kMaxCells + 1) + sizeof(int2) + 4 * 4;
+  return (mol * n + rep) * (size_t)nrep + 16 * (size_t)std::max(s.nfwall, 1) + 50 * 256 + 2 * kListPad + 128;
+}
+
 void engine_prepare_wall(const remd_system_desc& s) {
   std::string why;
   try {
@@ -849,7 +875,7 @@ static remd_status create_impl(const remd_system_desc* systems, int nens, const 
   auto* h = new remd_engine_s;
   h->device = device;
   h->prec = (prec == REMD_PREC_FP64) ? kF64 : kF32;
-  h->tile = (h->prec == kF32) ? 32 : 128;   // measured best on a 256-replica mixed batch; remd_set_tuning / remd_autotune change it
+  h->tile = default_tile(h->prec);
   h->nens = nens;
   h->interval = systems[0].interval;
   h->sys.assign(systems, systems + nens);
@@ -978,10 +1004,7 @@ static remd_status create_impl(const remd_system_desc* systems, int nens, const 
       c.sgm2 = sg * sg;
       const double eo = s.site_eps[0] * (1e+03 / 6.0221367e+23 / unit_energy());
       c.eps = std::sqrt(eo * eo);
-      const double rl = s.rcut + h->skin;
-      const double cap = 0.1 * 4.0 / 3.0 * M_PI * rl * rl * rl;
-      c.nbr_cap = std::min(s.nmol - 1, ((int)std::ceil(cap) + 7) / 8 * 8);
-      if (c.nbr_cap < 1) c.nbr_cap = 1;
+      c.nbr_cap = list_capacity(s.rcut, h->skin, s.nmol);
       h->rc.push_back(c);
       h->rep_ens.push_back(e);
       RepState rs;
@@ -1159,9 +1182,7 @@ static remd_status relayout(remd_engine_s* h, int tile, double skin, const Saved
   h->skin = skin;
   for (auto& c : h->rc) {
     c.skin = skin;
-    const double rl = c.rc + skin;
-    const double cap = 0.1 * 4.0 / 3.0 * M_PI * rl * rl * rl;
-    c.nbr_cap = std::max(1, std::min(c.nmol - 1, ((int)std::ceil(cap) + 7) / 8 * 8));
+    c.nbr_cap = list_capacity(c.rc, skin, c.nmol);
   }
   if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
   remd_status s = allocate(h);

@@ -37,6 +37,8 @@
 namespace remd {
 remd_status engine_get_exchange(remd_handle h, long long* steps, int* index);
 size_t engine_bytes(remd_handle h);
+// Device bytes that the replicas of a job take in a batch handle (its own layout).
+size_t engine_job_bytes(const remd_system_desc& s, int nrep, remd_precision prec);
 void engine_prepare_wall(const remd_system_desc& s);
 double engine_last_graph_ms(remd_handle h);
 remd_status engine_create_carry(remd_handle from, const remd_system_desc* systems, int nens,
@@ -80,18 +82,6 @@ struct Job {
 double now_s() {
   using namespace std::chrono;
   return duration<double>(steady_clock::now().time_since_epoch()).count();
-}
-
-// Device footprint of a job, with the engine's own layout formula.
-size_t estimate_bytes(const remd_system_desc& s, int nrep) {
-  const double rl = s.rcut + 1.0;
-  int cap = ((int)std::ceil(0.1 * 4.0 / 3.0 * M_PI * rl * rl * rl) + 7) / 8 * 8;
-  cap = std::min(cap, s.nmol - 1);
-  const size_t ntile = (s.nmol + 127) / 128;
-  // skin list + FP32 per-step list: 2 x 2 bytes per slot
-  const size_t per_rep = (size_t)s.nmol * (176 + 80 + 16 + 4) + ntile * (size_t)cap * 128 * 4 +
-                         ntile * (3 * 8 + 64 + 64 + 16) + 1024;
-  return per_rep * nrep + (size_t)std::max(s.nfwall, 0) * 16 + 4096;
 }
 
 double pct(std::vector<double> v, double q) {
@@ -305,7 +295,7 @@ remd_status remd_job_submit(remd_server S, const remd_job_desc* jd, remd_job_id*
     j->reps.push_back(R);
     j->index.push_back(k);
   }
-  j->bytes = estimate_bytes(j->sys, j->nrep());
+  j->bytes = engine_job_bytes(j->sys, j->nrep(), S->prec);
   std::lock_guard<std::mutex> lk(S->mu);
   if (j->bytes > S->budget) {
     delete j;
@@ -558,7 +548,7 @@ remd_status remd_server_step(remd_server S, int* pending) {
 
 remd_status remd_job_bytes(const remd_job_desc* jd, size_t* out) {
   if (!jd || !out || jd->ntemp < 1 || jd->npress < 1 || jd->system.nmol < 2) return REMD_ERR_INVALID;
-  *out = estimate_bytes(jd->system, jd->ntemp * jd->npress);
+  *out = engine_job_bytes(jd->system, jd->ntemp * jd->npress, REMD_PREC_FP32);
   return REMD_OK;
 }
 

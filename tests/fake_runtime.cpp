@@ -32,7 +32,7 @@ std::map<const void*, std::string> names;
 std::vector<Launch> launches, captured;   // run so far; nodes of the graph being captured
 std::set<cudaStream_t> streams;
 bool capture = false;
-long host_allocs, streams_made, instantiated, updated, nodes;
+long host_allocs, streams_made, instantiated, updated, nodes, device_bytes;
 
 cudaError_t fail(cudaError_t e) { last = e; return e; }
 
@@ -56,12 +56,12 @@ extern "C" {
 // ---- the record, read by the tests
 void fake_reset() {
   launches.clear();
-  host_allocs = streams_made = instantiated = updated = nodes = 0;
+  host_allocs = streams_made = instantiated = updated = nodes = device_bytes = 0;
 }
 long fake_count(const char* what) {
   const std::string w = what;
   return w == "host_allocs" ? host_allocs : w == "streams_made" ? streams_made : w == "instantiated" ? instantiated
-         : w == "updated" ? updated : w == "nodes" ? nodes : w == "launches" ? (long)launches.size() : -1;
+         : w == "updated" ? updated : w == "nodes" ? nodes : w == "device_bytes" ? device_bytes : w == "launches" ? (long)launches.size() : -1;
 }
 const char* fake_launch(int i, int* grid, int* block, int* programmatic, int* stream) {
   const Launch& l = launches[i];
@@ -111,14 +111,14 @@ cudaError_t cudaGetLastError() { const cudaError_t e = last; last = cudaSuccess;
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorInvalidResourceHandle ? "invalid resource handle" : "error"; }
 
 // ---- memory
-cudaError_t cudaMalloc(void** p, size_t n) { *p = std::calloc(1, n); return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { *p = std::calloc(1, n); device_bytes += (long)n; return cudaSuccess; }
 cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return cudaFree(p); }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) { *p = nullptr; return cudaSuccess; }
 cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { host_allocs++; return cudaMalloc(p, n); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::calloc(1, n); host_allocs++; return cudaSuccess; }
 cudaError_t cudaMallocHost(void** p, size_t n) { return cudaHostAlloc(p, n, 0); }
 cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }

@@ -164,3 +164,19 @@ def test_serving_loop_updates_its_graph_in_place(fake):
     assert fake.fake_count(b"instantiated") == 0 and fake.fake_count(b"updated") == 1
     assert _chains(_launches(fake)) == 4
     srv.close()
+
+
+@pytest.mark.parametrize("model", ["tip3p", "tip5p"])
+@pytest.mark.parametrize("nmol,nrep", [(2, 1), (64, 16), (100, 64), (128, 16), (129, 4), (900, 3)])
+def test_job_bytes_cover_what_the_batch_allocates(fake, model, nmol, nrep):
+    """The serving loop admits jobs by these bytes: they are no less than the device
+    memory that the job's batch takes, and not far above it."""
+    e = _grid(nmol, nrep, model)
+    said = E.Server.job_bytes(e)
+    srv = E.Server(budget_bytes=said)   # and exactly that budget admits it
+    srv.submit(e, 2)
+    fake.fake_reset()
+    srv.step()
+    used = fake.fake_count(b"device_bytes")
+    assert used <= said <= 1.25 * used + 20000
+    srv.close()
