@@ -17,7 +17,8 @@ namespace remd {
 
 constexpr int kRepThreads = 256;   // threads of the per-replica kernels
 constexpr int kBitmapMaxWords = 64; // list-rebuild bitmap window: 2048 molecules per pass
-constexpr int kCellMinPrune = 4;    // cut a replica into cells when they prune at least 4x
+constexpr int kCellMinPrune = 4;    // cut a replica into cells when they prune at least 4x,
+constexpr int kCellMinMol = 512;    // and it is no smaller than this (cell_grid)
 constexpr int kGroup = 8;           // FP32 form: lanes per molecule in the list and pair kernels
 constexpr int kWarpMol = 32 / kGroup;   // molecules of a warp there
 constexpr int kPairWarps = kPart2Mol / kWarpMol;   // warps of a list or pair block (kPart2Mol molecules)
@@ -351,9 +352,9 @@ __device__ __forceinline__ int cell_coord(int x, int n) {
   return (int)(((unsigned long long)u * (unsigned)n) >> 32);
 }
 
-// Radius the list build tests (FP32 form): rcut + skin widened by the
-// truncation error of its FP32 test, sqrt(3) L_max 2^-16, and a relative 1e-5.
-// The FP64 form's test radius, rcut + skin, is below it.
+// Radius the list build tests: rcut + skin widened by the
+// truncation error of its FP32 test (both forms'), sqrt(3) L_max 2^-16, and a
+// relative 1e-5.
 __device__ inline double list_test_radius(const RepConst& c, const double* L) {
   const double lmax = fmax(fmax(L[0], L[1]), L[2]);
   return (c.rc + c.skin + 1.7320508075688772 * lmax * (1.0 / 65536.0)) * (1.0 + 1e-5);
@@ -378,11 +379,15 @@ __device__ inline CellGrid cell_grid(const RepConst& c, const double* L) {
     const int m = (n[0] >= n[1] && n[0] >= n[2]) ? 0 : (n[1] >= n[2] ? 1 : 2);
     n[m] = (n[m] - 1 >= 3) ? n[m] - 1 : 1;
   }
-  // a candidate from the cells costs several times one of the all-molecule scan
-  // (gathered, per lane, versus a shared-memory broadcast): cut the box only
-  // where the neighbouring cells hold at most 1/kCellMinPrune of the replica
+  // A candidate from the cells (gathered, a bitmap bit set) costs several times one of
+  // the all-molecule scan (one load tested against four molecules), and the stencil's
+  // loops cost a small replica more than its scan.  The lists are the same either way.
+  // Lists launches with a quarter of the replicas rebuilt, cut / uncut: 64 tubes of 200
+  // molecules (pruned 4x) 23.4 / 14.9 us, of 300 (3x) 24.9 / 20.1, of 450 (6x) 29.2 /
+  // 28.4; 16 slits of 1000 (3.6x) 34.9 / 33.4, 8 of 2000 (7x) 34.8 / 51.4, 4 bulk boxes
+  // of 4096 (2.4x) 59.5 / 64.7 with 3 us more in the head, of 6000 (4.6x) 111 / 119.
   const int stencil = (n[0] > 1 ? 3 : 1) * (n[1] > 1 ? 3 : 1) * (n[2] > 1 ? 3 : 1);
-  if ((long long)stencil * kCellMinPrune > (long long)n[0] * n[1] * n[2]) n[0] = n[1] = n[2] = 1;
+  if (c.nmol < kCellMinMol || (long long)stencil * kCellMinPrune > (long long)n[0] * n[1] * n[2]) n[0] = n[1] = n[2] = 1;
   CellGrid g;
   g.nx = n[0]; g.ny = n[1]; g.nz = n[2];
   g.rebuild = 1;

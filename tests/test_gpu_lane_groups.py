@@ -117,11 +117,15 @@ def test_charges_far_apart(model, charges):
     _check(spec, e.states[0], "fp32")
 
 
-def test_fp64_form_with_cell_lists():
-    """A tube long enough to be cut into cells: the FP64 form takes the list rebuild
-    of the FP32 form and tests its entries in FP64."""
-    e = S.make_ensemble("cells", "tip4p", 1, 1500, 7.0, 9.0, 8.0, 1, 1, 300, 300, 0.1e6, 0.1e6, 330)
-    _check(e.spec, e.states[0], "fp64")
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("nmol", [511, 512, 1500, 2100])
+def test_cell_lists_and_their_smallest_replica(nmol, prec):
+    """A tube long enough to be cut into cells, from 512 molecules on; 2100 take two
+    windows of the rebuild's bitmap.  Both forms share the rebuild, and the FP64 form
+    tests its entries in FP64.  (A cutoff off the lattice: at 9.0 A every molecule has
+    a neighbour exactly at it.)"""
+    e = S.make_ensemble("cells", "tip4p", 1, nmol, 7.0, 9.1, 8.1, 1, 1, 300, 300, 0.1e6, 0.1e6, 330)
+    _check(e.spec, e.states[0], prec, "fp32 small" if prec == "fp32" else None)
 
 
 @pytest.mark.parametrize("prec,charges", [("fp32", "water"), ("fp64", "water"), ("fp32", "other")])
