@@ -210,18 +210,18 @@ remd_status remd_measure_atomics(int device, double *rates);
 /* Per-replica health word of the last interval: 0 ok, else a remd_status. */
 remd_status remd_replica_status(remd_handle h, int rep, int *status);
 
-/* Tuning: molecules of one force tile (multiple of 32: 32..64 for FP32 handles,
- * 32..128 for FP64; defaults 32 / 128) and the neighbour
+/* Tuning: molecules of one tile, a block of the integration kernel (multiple of 32:
+ * 32..64 for FP32 handles, 32..128 for FP64; defaults 32 / 128), and the neighbour
  * skin (A).  Takes effect on the next call. */
 remd_status remd_set_tuning(remd_handle h, int tile, double skin);
 
 /* Autotuner (no counterpart in the reference): times every (tile, skin) of
- * {32, 64, 96, 128} x {0.6, 0.8, 1.0, 1.4} A that the handle's precision
+ * {32, 64, 96, 128} x {0.2, 0.4, 0.6, 0.8, 1.0, 1.4} A that the handle's precision
  * allows (remd_set_tuning) over `nsteps` MD steps of this
  * batch (integrate + force per step, CUDA events), restores the state after
  * each trial and keeps the fastest.  The trajectory does not depend on the
- * choice: forces are a function of positions only and every partial sum is
- * per 32 molecules.  Outputs (any may be NULL): the chosen tile, skin and its
+ * choice: forces are a function of positions only, and partial sums are per 32
+ * molecules (integration) or 16 (forces) whatever the tile.  Outputs (any may be NULL): the chosen tile, skin and its
  * ms per MD step.  Synchronous; call it before stream capture. */
 remd_status remd_autotune(remd_handle h, int nsteps, int *tile, double *skin, double *ms_per_step);
 

@@ -79,7 +79,7 @@ struct remd_engine_s {
   std::vector<int> rep_ens, ens_rep_off, ens_nrep;
   std::vector<RepConst> rc;
   std::vector<Tile> tiles;
-  std::vector<int> order;          // force blocks -> tiles, costliest first
+  std::vector<int> order;          // tiles, costliest first
   std::vector<PairBlk> pblk;       // list and pair blocks in that order
   Chains chains[2];                // of the interval graph: the first one's, and the second one's
   bool may_widen = true;           // a second one may be made (not in the serving loop)
@@ -1175,8 +1175,9 @@ static remd_status save_state(remd_engine_s* h, SavedState& sv) {
 }
 
 // Re-lay out the arrays for (tile, skin) and restore `sv`.  Forces are a pure
-// function of the positions and every partial sum is per 32 molecules, so the
-// trajectory that follows does not depend on the tile or the skin.
+// function of the positions and partial sums are per 32 (integrate) or 16 (forces)
+// molecules whatever the tile, so the trajectory that follows does not depend on the
+// tile or the skin.
 static remd_status relayout(remd_engine_s* h, int tile, double skin, const SavedState& sv) {
   h->tile = tile;
   h->skin = skin;
@@ -1207,7 +1208,7 @@ static remd_status relayout(remd_engine_s* h, int tile, double skin, const Saved
 }
 
 remd_status remd_set_tuning(remd_handle h, int tile, double skin) {
-  if (!h || tile < 32 || tile > max_force_tile(h->prec) || tile % 32 || !(skin > 0.0)) {
+  if (!h || tile < 32 || tile > max_tile(h->prec) || tile % 32 || !(skin > 0.0)) {
     set_error("remd_set_tuning: tile must be a multiple of 32 in 32..64 (FP32) or 32..128 (FP64), skin > 0");
     return REMD_ERR_INVALID;
   }
@@ -1230,7 +1231,7 @@ remd_status remd_autotune(remd_handle h, int nsteps, int* tile_out, double* skin
   double best_skin = h->skin, best_ms = 1e300;
   for (int t : tiles)
     for (double k : skins) {
-      if (t > max_force_tile(h->prec)) continue;
+      if (t > max_tile(h->prec)) continue;
       if ((s = relayout(h, t, k, sv)) != REMD_OK) return s;
       double ms[2];
       if ((s = remd_profile_steps(h, nsteps, ms)) != REMD_OK) return s;

@@ -126,7 +126,7 @@ __device__ inline P2Sum reduce_part2(const DevPtrs& d, int part2_off, int npart2
 }
 
 // Programmatic dependent launch of the MD-step kernels (launch_integrate_prec,
-// launch_force): where a step's tile grid is smaller than the GPU, each is
+// launch_force): where a step's pair work is small (DevPtrs::pdl), each is
 // launched allowed to start while the kernel before it on its stream is still
 // running.  Its blocks first wait for that kernel's completion and memory
 // (griddepcontrol.wait, which returns at once when there is no such kernel or
@@ -230,9 +230,9 @@ struct StepCoef {
 // One MD step's integration.  It is bound by latency, not by throughput (a block's
 // FP64 scalar chain, then each molecule's): what a block needs -- the replica's
 // constants and scalars, the force partials -- is requested at once from the tile's
-// descriptor (14.5 -> 11.8 us a launch at 64 molecules).  CHAIN: one more warp runs the scalar chain while the molecules' warps
-// load their state, into registers; for grids that leave room for the extra warp
-// (launch_integrate_prec).
+// descriptor (14.5 -> 11.8 us a launch at 64 molecules).  CHAIN: one more warp runs the
+// scalar chain while the molecules' warps load their state, into registers; for grids
+// that leave room for the extra warp (launch_integrate_prec).
 template <bool MID, bool CHAIN>
 __global__ void __launch_bounds__(CHAIN ? 160 : 128, CHAIN ? 3 : 7)
     k_integrate(DevPtrs d, const RepState* __restrict__ X, RepState* __restrict__ Y, int prec) {
@@ -352,9 +352,8 @@ __device__ __forceinline__ int cell_coord(int x, int n) {
   return (int)(((unsigned long long)u * (unsigned)n) >> 32);
 }
 
-// Radius the list build tests: rcut + skin widened by the
-// truncation error of its FP32 test (both forms'), sqrt(3) L_max 2^-16, and a
-// relative 1e-5.
+// Radius the list build tests: rcut + skin widened by the truncation error of its FP32
+// test (both forms'), sqrt(3) L_max 2^-16, and a relative 1e-5.
 __device__ inline double list_test_radius(const RepConst& c, const double* L) {
   const double lmax = fmax(fmax(L[0], L[1]), L[2]);
   return (c.rc + c.skin + 1.7320508075688772 * lmax * (1.0 / 65536.0)) * (1.0 + 1e-5);
@@ -1445,8 +1444,8 @@ __device__ __forceinline__ void step_list(const DevPtrs& d, const PairBlk& b, co
 // 111 432 molecules).  It is bound by the latency of its loads, so all that need only
 // the block's descriptor are issued together, and the wall's FP64 chain runs under
 // them, a molecule per thread of the first warp (one lane in eight of every warp,
-// after the lists: 88.6 us there, now 83.4, of which 25 the rebuild of 14 replicas;
-// 256 tubes of 128 .. 420 molecules 41.0 -> 36.0).  Two and four lanes per molecule
+// after the lists: 88.6 us there, now 83.4; 256 tubes of 128 .. 420 molecules 41.0 ->
+// 36.0).  Two and four lanes per molecule
 // measured slower at every length of the lists (158 and 112 us; on the tubes 64 and 45).
 __global__ void __launch_bounds__(32 * kPairWarps, 128 / kPart2Mol) k_force_lists(DevPtrs d, const RepState* __restrict__ X) {
   step_kernel_entry();
@@ -2308,7 +2307,7 @@ void launch_integrate_prec(const DevPtrs& d, const RepState* X, RepState* Y, boo
             : (mid ? k_integrate<true, false> : k_integrate<false, false>);
   launch_step_kernel(d.pdl, k, d.ntiles, tile + (chain ? 32 : 0), 0, s, d, X, Y, prec);
 }
-int max_force_tile(int prec) { return prec == kF32 ? 64 : 128; }
+int max_tile(int prec) { return prec == kF32 ? 64 : 128; }
 
 // Bitmap of the list rebuild: one row of (win | 1) words per molecule of a block.
 size_t bitmap_smem_bytes(int mols, int win) { return (size_t)mols * (size_t)(win | 1) * sizeof(uint32_t); }

@@ -2,7 +2,7 @@
 //
 // One MD step of every replica of every ensemble is a short chain of launches
 // (a tile = 32 or 64 consecutive molecules of one replica, up to 128 in the
-// FP64 form, a block of k_integrate):
+// FP64 form, is a block of k_integrate; the force kernels' blocks are 16 molecules):
 //
 //   k_integrate     [end of the previous step: D5 kick, D5/D6 scalars]
 //                   D6, D5, D4, D3 D2 D1 D2 D3 (src/integrator.cxx:646-673),
@@ -30,8 +30,8 @@ enum Prec : int { kF32 = 0, kF64 = 1 };
 void launch_pack(const DevPtrs& d, int prec, int tile, cudaStream_t s);
 void launch_integrate_prec(const DevPtrs& d, const RepState* X, RepState* Y, bool mid, int tile,
                            int prec, cudaStream_t s);
-// Largest tile (molecules per integrate block; FP64 form: per force block) of a precision.
-int max_force_tile(int prec);
+// Largest tile (molecules per integrate block) of a precision.
+int max_tile(int prec);
 // Words per row of the list-rebuild bitmap for replicas of up to max_nmol molecules (DevPtrs::bm_win).
 int bitmap_window(int max_nmol);
 void launch_force(const DevPtrs& d, const RepState* Yin, RepState* Xout, int prec, bool force_only,

@@ -75,8 +75,8 @@ def test_noalloc_snapshot_equals_regular_snapshot_on_consecutive_calls():
         g, pairs = expected[k]
         assert out[7] == 0.0
         assert np.array_equal(f, g["f"]) and np.array_equal(n, g["n"])
-        # energies and virial: the same per-32-molecule partial sums, added up in
-        # another order (a warp butterfly here, a host loop in remd_get_state)
+        # energies and virial: the same partial sums per 16 molecules, added up by the
+        # same butterfly
         for a, b in [(out[0], g["lj"]), (out[1], g["clmb"]), (out[2], g["wall"])]:
             assert a == pytest.approx(b, rel=1e-13, abs=1e-13)
         assert np.allclose(out[3:6], g["vir"], rtol=1e-13, atol=1e-13)
