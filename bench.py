@@ -832,8 +832,8 @@ def engine_arm(args, rank, world, local):
     achieved = flops / (force_ms * 1e-3) / 1e12
     roof = {"bound": "fp32",
             "kernel": "force step: k_replica_head (PsPv + D4, list decision, cell sort) + "
-                      "k_force_lists (list rebuild, pairs within rcut) + "
-                      "k_force_pairs (pair forces, wall, A2M)",
+                      "k_force_lists (wall terms, list rebuild, pairs within rcut) + "
+                      "k_force_pairs (pair forces, A2M)",
             "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
             "frac": achieved / peak.value,
             "peak_source": "measured: register-resident FP32 FMA chains on all SMs "
