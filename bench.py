@@ -280,10 +280,13 @@ def cpu_threads():
 def reference_arm(args, rank, world):
     if rank != 0:
         return
-    ens = workload(args.config, args.seed, args.interval)
     from oracle import oracle as O
+    if not O.reference_available("generic"):   # nothing of ours may stand in for it
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's own CPU objects (oracle/_ref) are not "
+                          "built: its sources are not on this machine"}), flush=True)
+        return
+    ens = workload(args.config, args.seed, args.interval)
     nth = cpu_threads()
-    total = sum(e.spec.nmol for e in ens for _ in e.states)
     # warm-up then K timed steps, each one MD step of every replica
     b = cpu_baseline(ens, max(args.warmup, 1), nth) if args.warmup > 0 else None
     res = cpu_baseline(ens, args.steps, nth)

@@ -85,3 +85,16 @@ def test_cpu_model_names_the_host():
     import bench
     s = bench.cpu_model()
     assert s.endswith("logical CPUs") and str(os.cpu_count()) in s
+
+
+def test_reference_arm_says_so_when_the_reference_is_not_there(monkeypatch, capsys):
+    """The arm runs the reference's own code or prints why it cannot; the repository's
+    restatement does not stand in for it."""
+    import json
+
+    import bench
+    from oracle import oracle as O
+    monkeypatch.setattr(O, "reference_available", lambda variant="generic": False)
+    bench.reference_arm(bench.parse_args(["--impl", "reference", "--steps", "1", "--warmup", "0"]), 0, 1)
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
