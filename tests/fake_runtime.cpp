@@ -32,6 +32,7 @@ std::map<const void*, std::string> names;
 std::vector<Launch> launches, captured;   // run so far; nodes of the graph being captured
 std::set<cudaStream_t> streams;
 bool capture = false;
+int fail_instantiations = 0;
 long host_allocs, streams_made, instantiated, updated, nodes, device_bytes;
 
 cudaError_t fail(cudaError_t e) { last = e; return e; }
@@ -54,6 +55,7 @@ std::vector<int> topology(const std::vector<Launch>& v) {
 
 extern "C" {
 // ---- the record, read by the tests
+void fake_fail_instantiations(int n) { fail_instantiations = n; }
 void fake_reset() {
   launches.clear();
   host_allocs = streams_made = instantiated = updated = nodes = device_bytes = 0;
@@ -177,6 +179,10 @@ cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
 }
 cudaError_t cudaGraphDestroy(cudaGraph_t g) { delete g; return cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t g, unsigned long long) {
+  if (fail_instantiations > 0) {
+    fail_instantiations--;
+    return fail(cudaErrorMemoryAllocation);
+  }
   *x = new CUgraphExec_st{g->nodes};
   instantiated++;
   return cudaSuccess;

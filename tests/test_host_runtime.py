@@ -150,6 +150,19 @@ def test_eight_chains_come_once_they_pay(fake, nmol, nrep, later):
     eng.close()
 
 
+def test_no_room_for_the_second_graph(fake):
+    """Where the second graph cannot be made the handle goes on with the first one, and
+    does not try again every interval."""
+    eng = E.REMDGPU([_grid(512, 64)])
+    for _ in range(32):
+        _interval(fake, eng)
+    fake.fake_fail_instantiations(1)
+    assert _chains(_interval(fake, eng)) == 4 and fake.fake_count(b"instantiated") == 1
+    assert _chains(_interval(fake, eng)) == 4 and fake.fake_count(b"instantiated") == 0
+    fake.fake_fail_instantiations(0)
+    eng.close()
+
+
 def test_serving_loop_updates_its_graph_in_place(fake):
     """A batch that grows and shrinks keeps one graph topology, so the executable graph
     is updated and not made anew, also after many rounds."""
