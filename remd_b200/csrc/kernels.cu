@@ -696,7 +696,7 @@ __device__ __forceinline__ double wall_site(const DevPtrs& d, const RepConst& c,
 //    the others ("near") from the back;
 //  * k_force_pairs computes exactly those pairs, lane sub entries sub, sub + 8, ...
 //    (first the near, then the far ones), with no cutoff branch.  A lane's sums are
-//    FP32 in registers over at most 32 + 1 pairs; then the group's lanes are added
+//    FP32 in registers over at most 32 pairs; then the group's lanes are added
 //    in FP64 by a fixed exchange tree that leaves three of the molecule's 24 sums
 //    with each lane, and finish_group forms force and torque (A2M).
 // Which pairs a lane sums, and in what order, depends on the positions only:
@@ -985,8 +985,10 @@ __device__ __forceinline__ int force_warp_f32(const DevPtrs& d, const PairBlk& b
   const int lic = min(li0 + grp, b.nmol - 1);
   const int nfar = nc & 0xffff, nnear = nc >> 16;
   const uint16_t* row = d.nbt + b.nbr_off + (long long)lic * b.nbr_stride + sub;
-  // FP32 sums close every 32 pairs of a lane
-  const bool segments = __any_sync(kAll, nfar + nnear > kSegPairs);
+  // FP32 sums close every 32 pairs of a lane: where its near and far pairs together
+  // are no more, one segment holds both
+  const bool segments = __any_sync(kAll, (nfar + kGroup - 1) / kGroup + (nnear + kGroup - 1) / kGroup >
+                                             kSegPairs / kGroup);
   F32Sums<S> a;
   a.zero();
   for (int p0 = 0; __any_sync(kAll, p0 < nnear); p0 += kSegPairs) {
